@@ -267,4 +267,156 @@ static __device__ __forceinline__ float cell_slow(float diag, float up, float le
     return pick(d, u, l, from);
 }
 
+// ---------------------------------------------------------------- candidates on a grid
+// A candidate is RN32(X), X = RN64(RN64(a + B) + em), of a score a, a transition
+// B and an emission em.  Let T = B + em.  Once the band's scores are all below
+// -2^m (m >= kGridMin), everything but one FP32 add can be done ahead of the band,
+// from T alone, for all scores in [-60 * 2^m, -2^m):
+//
+//  Let g = 2^(m-25).  Floats of magnitude 2^m or more are multiples of 4g or more,
+//  so a is a multiple of 2g and every rounding breakpoint (a midpoint of two
+//  neighbouring floats) of that range is one too.  Take x = the midpoint of the
+//  cell (2g j, 2g (j + 1)) that holds T (round-to-odd of T on the grid g: Boldo
+//  and Melquiond, IEEE Trans. Comput. 57, 2008).  a + T and a + x lie strictly in
+//  the same cell, no breakpoint lies inside a cell, so RN32(a + T) = RN32(a + x),
+//  and X does too if T is further than |X - (a + T)| from both ends of its cell:
+//  |X - (a + T)| <= 2^-52 (|a| + |T| + ulps) < 2^-52 * 2^(m+6) = 2^-21 g.  The
+//  error of T's position in its cell as computed below is under 2^-22 g, and the
+//  margin asked for is eps = 2^-20 g.  x is a float when |T| < 2^(m-1) (an odd
+//  multiple of g below 2^24 g), and __fadd_rn(a, x) is the candidate.  The result
+//  must be checked to be < -2^m (then a + x lies beyond -2^m, in the range above).
+//
+// The emission's side: fe = the multiple of 2g at or below em, by one add rounded
+// down to c = -(2^(m-1) + 64), whose binade has ulp 2g (em in (-(2^(m-1) - 64), 64]);
+// re = em - fe in [0, 2g).  The constant's side, once per grid: B = f + rs likewise.
+// T = fe + f + (re + rs), so T's cell is f's, or the next one when z = re + rs - 2g
+// is not negative, and |z| > eps is the margin asked for (rs itself is kept 2 eps
+// away from the ends: GridStep::ok).
+//
+// Emissions below the range (an event many deviations from its k-mer): on the
+// grids below kGridWide x is then only an upper bound of T (kGridOpt), so that the
+// add gives an upper bound of the candidate; it is recognised by x < -lim, and must
+// not win its cell.  On the others, whose range seldom falls short, x is NaN.
+// x < 0 (grid_kmer_ok): no score exceeds the largest one it derives from.
+constexpr int kGridMin = 11, kGridWide = 13, kGridMax = 22;
+constexpr float kGridOpt = 1.0f - 1.0f / 65536.0f;     // 1 - 2^-16
+constexpr float kGridLimLo = 1.0f - 1.0f / 32768.0f;   // 1 - 2^-15
+
+struct GridStep {
+    float z, o0, o1;  // rs - 2g; the cell midpoint's part f + g, and the next cell's
+};
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
+
+__device__ __forceinline__ GridStep grid_step(float bh, float bl, int m, bool& ok) {
+    const float c = -(pow2f(m - 1) + 64.0f), g2 = pow2f(m - 24), eps = pow2f(m - 45);
+    float f = __fsub_rn(__fadd_rd(c, bh), c);
+    float t = __fadd_rn(__fsub_rn(bh, f), bl);
+    if (t < 0.0f) {
+        f = __fsub_rn(f, g2);
+        t = __fadd_rn(t, g2);
+    }
+    if (t >= g2) {
+        f = __fadd_rn(f, g2);
+        t = __fsub_rn(t, g2);
+    }
+    ok = t > 2.0f * eps && t < g2 - 2.0f * eps && fabsf(bh) < 30.0f;
+    GridStep s;
+    s.z = __fsub_rn(t, g2);
+    s.o0 = __fadd_rn(f, 0.5f * g2);
+    s.o1 = __fadd_rn(s.o0, g2);
+    return s;
+}
+
+// The grids (bit m) on which the read's three constants keep their margin.
+__device__ __forceinline__ uint32_t grid_modes(const CellConsts& c) {
+    uint32_t r = 0;
+#pragma unroll 1
+    for (int m = kGridMin; m <= kGridMax; ++m) {
+        bool a, b, d;
+        grid_step(c.step_h, c.step_l, m, a);
+        grid_step(c.stay_h, c.stay_l, m, b);
+        grid_step(c.skip_h, c.skip_l, m, d);
+        if (a && b && d) r |= 1u << m;
+    }
+    return r;
+}
+
+// Emission-side constants of grid m.
+struct Grid {
+    float c, eps, lim;
+    float skip;  // the skip's part
+    GridStep step, stay;
+};
+__device__ __forceinline__ Grid make_grid(const CellConsts& cc, int m) {
+    bool ok;
+    Grid G;
+    G.c = -(pow2f(m - 1) + 64.0f);
+    G.eps = pow2f(m - 45);
+    G.lim = -(pow2f(m - 1) - 128.0f);
+    G.skip = grid_step(cc.skip_h, cc.skip_l, m, ok).o0;
+    G.step = grid_step(cc.step_h, cc.step_l, m, ok);
+    G.stay = grid_step(cc.stay_h, cc.stay_l, m, ok);
+    return G;
+}
+
+// What grid_pair asks of a k-mer's parameters: no under- or overflow in the
+// division of any emission that matters (quotients of 2^-40 and more have their
+// remainder in range, and the square of a smaller one vanishes against k1), and
+// emissions (at most k1) whose T is negative.
+__device__ __forceinline__ float grid_k1_max(float step_h, float stay_h) {
+    return fminf(-fmaxf(step_h, stay_h), 60.0f) - 0.125f;
+}
+__device__ __forceinline__ bool grid_kmer_ok(float sd, float k1, float k1_max) {
+    return sd >= 9.094947e-13f && sd <= 1.0995116e12f && k1 <= k1_max && fabsf(k1) >= 9.094947e-13f;
+}
+
+// {x of the step (diagonal), x of the stay (up)} of one emission; NaN when not proven.
+// kLow: a grid below kGridWide.
+template <bool kLow>
+__device__ __forceinline__ float2 grid_pair(float x, float gm, float sd, float rsd, float k1, const Grid& G) {
+    // the emission, as emission_fast (the bracket proves the division)
+    const float n = __fsub_rn(x, gm);
+    const float q0 = __fmul_rn(n, rsd);
+    const float r = __fmaf_rn(-q0, sd, n);
+    const float dq = __fmul_rn(r, rsd);
+    const float hp = __fmaf_rn(dq, kDivHi, q0);
+    const float hm = __fmaf_rn(dq, kDivLo, q0);
+    const float em = __fadd_rn(k1, __fmul_rn(__fmul_rn(-0.5f, hp), hp));
+    float fe = __fsub_rn(__fadd_rd(G.c, em), G.c);
+    const float re = __fsub_rn(em, fe);
+    const float zd = __fadd_rn(re, G.step.z), zu = __fadd_rn(re, G.stay.z);
+    const bool ok = hp == hm && fabsf(zd) > G.eps && fabsf(zu) > G.eps && (kLow || em >= G.lim);
+    fe = ok ? fe : __int_as_float(0x7fc00000);
+    float xd = __fadd_rn(fe, zd >= 0.0f ? G.step.o1 : G.step.o0);
+    float xu = __fadd_rn(fe, zu >= 0.0f ? G.stay.o1 : G.stay.o0);
+    if (kLow) {
+        const float k = xu < G.lim ? kGridOpt : 1.0f;
+        xd = __fmul_rn(xd, k);
+        xu = __fmul_rn(xu, k);
+    }
+    return make_float2(xd, xu);
+}
+
+// max of three and of two, NaN if any is NaN.
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float a) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ float warp_min(float a) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(a));
+    return r;
+}
+
 }  // namespace abea

@@ -97,7 +97,6 @@ struct abea_batch {
     std::vector<int32_t> dev_order;       // the batched form's order: wide reads, then the rest longest first
     std::vector<int32_t> dev_order_sent;  // the order last copied to the device
     int32_t n_wide = 0;          // leading reads of `order` run on the wide shape
-    int32_t n_mid = 0;           // the reads after them run on the medium shape
     // sizes
     int64_t seq_bytes = 0, n_events_total = 0, ev_pad_total = 0, km_pad_total = 0,
             band_pad_total = 0, pair_cap = 0, band_cells = 0;
@@ -113,6 +112,7 @@ struct abea_batch {
     abea_model_t* d_model = nullptr;
     float *d_ev_mean = nullptr, *d_km_gm = nullptr, *d_km_sd = nullptr, *d_km_rsd = nullptr,
           *d_km_k1 = nullptr, *d_last_col = nullptr;
+    float4* d_km4 = nullptr;
     uint8_t* d_trace = nullptr;
     float* d_scores = nullptr;
     float* d_ck = nullptr;           // checkpoint records
@@ -148,7 +148,7 @@ struct abea_ctx {
     int64_t store_scores = 0;
     int64_t use_graph = 1;
     int64_t long_read_bands = 0;
-    int64_t mid_read_bands = 0;  // medium-shape threshold (0 = the autotuned value, else none)
+    int64_t mid_read_bands = 0;  // a second wide-shape threshold (ABEA_OPT_MEDIUM_READ_BANDS; 0 = the autotuned value, else none)
     int64_t spin_limit = 1 << 22;
     int64_t var_aware = 0;
     int64_t trace_budget = 0;  // bytes of trace a read may keep (0 = every trace)
@@ -483,8 +483,8 @@ static abea_status_t ensure_device(abea_batch* b, bool scores, size_t reserve = 
         (size_t)kCkBands * kSlots * (size_t)std::max<int32_t>(b->n_ck, 0),  // recompute scratch
         sizeof(int32_t) * kSpecRound * kSpecBands * (size_t)b->n_spec,      // traceback cell maps
         kAuxBytes,  // landed counter and output mirror
-        0};
-    const int n_bufs = 32;
+        sizeof(float4) * (size_t)std::max<int64_t>(b->km_pad_total, 16)};  // km4
+    const int n_bufs = 33;
     size_t total = 0;
     for (int i = 0; i < n_bufs; ++i) total += align256(sizes[i]);
     if (total > b->slab.bytes) {
@@ -538,6 +538,7 @@ static abea_status_t ensure_device(abea_batch* b, bool scores, size_t reserve = 
     b->d_ck_scratch = (uint8_t*)ptrs[29];
     b->d_spec = (int32_t*)ptrs[30];
     b->d_aux = (char*)ptrs[31];
+    b->d_km4 = (float4*)ptrs[32];
     b->scores_kept = scores;
     b->carve.assign(1, (uint64_t)(uintptr_t)b->slab.base);
     for (int i = 0; i < n_bufs; ++i) b->carve.push_back((uint64_t)sizes[i]);
@@ -658,33 +659,29 @@ static int64_t heuristic_threshold(const abea_batch* b, int blocks) {
     return best_n > 0 ? wide_ok[(size_t)best_n - 1] : INT64_MAX;
 }
 
-// Reads of the batched form that run on the wide and the medium shapes: the
-// longest reads over the wide threshold (the option, the autotuned value, or the
-// heuristic above; the blocks take them longest first, one at a time, as many
-// each as the queue holds; with the cluster pair at most one per cluster), then
-// the longest remaining reads over the medium threshold (none without one; never
-// with the cluster pair); never a checkpointed read.  Fills b->dev_order with the wide reads, the
-// medium reads, then the rest, each longest first, and sets n_wide and n_mid.
+// Reads of the batched form that run on the wide shape: those over the wide
+// threshold (the option, the autotuned value, or the heuristic above) or over the
+// medium one, when there is one (its own shape, two reads per block, is no longer
+// faster than one wide read after another); never a checkpointed read.  The blocks
+// take them longest first, one at a time, as many each as the queue holds; with the
+// cluster pair at most one per cluster, and no medium threshold.  Fills
+// b->dev_order with the wide reads, then the rest, each longest first, and sets n_wide.
 static void choose_shape_reads(abea_batch* b, int sm_count, int64_t threshold, int64_t mid_threshold, bool scores,
                                bool cluster) {
     const int blocks = cluster ? sm_count / 2 : batched_blocks_per_sm(scores) * sm_count;
     if (threshold <= 0) threshold = heuristic_threshold(b, blocks);
-    if (mid_threshold <= 0 || cluster) mid_threshold = INT64_MAX;
-    std::vector<int32_t> wide, mid, rest;
+    if (mid_threshold > 0 && !cluster) threshold = std::min(threshold, mid_threshold);
+    std::vector<int32_t> wide, rest;
     for (int32_t i : b->order) {
         const ReadDesc& r = b->reads[(size_t)i];
         if ((!cluster || (int)wide.size() < blocks) && !r.ck && r.n_bands >= threshold)
             wide.push_back(i);
-        else if (!r.ck && r.n_bands >= mid_threshold)
-            mid.push_back(i);
         else
             rest.push_back(i);
     }
     b->dev_order = wide;
-    b->dev_order.insert(b->dev_order.end(), mid.begin(), mid.end());
     b->dev_order.insert(b->dev_order.end(), rest.begin(), rest.end());
     b->n_wide = (int32_t)wide.size();
-    b->n_mid = (int32_t)mid.size();
 }
 
 // Queues pre, core and post for a batch on the context's stream.
@@ -692,12 +689,12 @@ static abea_status_t launch_all(abea_ctx* c, abea_batch* b, int* launches, bool 
     LaunchArgs la;
     const GlobalConsts g = global_consts(b->var_aware);
     la.pre = PreArgs{b->d_reads, b->n_reads, g, b->d_seq, b->d_ev, b->d_model, b->d_ev_mean, b->d_km_gm,
-                     b->d_km_sd, b->d_km_rsd, b->d_km_k1, b->d_last_col, (const InMirror*)b->d_aux};
+                     b->d_km_sd, b->d_km_rsd, b->d_km_k1, b->d_last_col, (const InMirror*)b->d_aux, b->d_km4};
     la.core = CoreArgs{b->d_reads, b->n_reads, g, b->d_ev_mean, b->d_km_gm, b->d_km_sd, b->d_km_rsd, b->d_km_k1,
                        b->d_last_col, b->d_trace, b->scores_kept ? b->d_scores : nullptr, b->d_band_k0,
                        b->d_slow, b->d_order, b->d_queue, b->n_wide, b->d_ck, b->d_ck_scratch, b->d_spec,
                        b->n_spec,
-                       (long long)c->spin_limit, b->n_mid};
+                       (long long)c->spin_limit, b->d_km4};
     la.post = PostArgs{b->d_reads, b->n_reads, g, b->d_ev_mean, b->d_km_gm, b->d_km_sd, b->d_km_k1, b->d_km_rsd,
                        b->d_last_col, b->d_trace, b->d_band_k0, b->d_pairs, b->d_n_pairs, b->d_best,
                        b->d_status, b->d_path_len, b->d_path_flags, b->d_best_event,
@@ -738,7 +735,6 @@ static abea_status_t queue_work(abea_ctx* c, abea_batch* b, int* launches, bool 
 // (threshold from the option, else the autotuned value, else none), then the rest.
 static void prepare_order(abea_ctx* c, abea_batch* b) {
     b->n_wide = 0;
-    b->n_mid = 0;
     if (c->mode != ABEA_MODE_BATCHED) return;
     const uint64_t sig = workload_signature(b);
     int64_t thr = c->long_read_bands, mid = c->mid_read_bands;
@@ -779,7 +775,6 @@ static abea_status_t run_batch(abea_ctx* c, abea_batch* b) {
         std::vector<uint64_t> key = b->carve;
         key.push_back((uint64_t)b->n_reads);
         key.push_back((uint64_t)b->n_wide);
-        key.push_back((uint64_t)b->n_mid);
         key.push_back((uint64_t)(b->scores_kept ? 1 : 0) | ((uint64_t)b->var_aware << 1) |
                       ((uint64_t)(c->wide_cluster != 0) << 2));
         if (!b->graph || key != b->graph_key) {
@@ -832,8 +827,8 @@ extern "C" abea_status_t abea_autotune(abea_ctx_t* c, abea_batch_t* b, int64_t* 
     const abea_mode_t mode0 = c->mode;
     const int64_t thr0 = c->long_read_bands, mid0 = c->mid_read_bands;
     c->mode = ABEA_MODE_BATCHED;
-    // the wide stage runs without medium reads: neither the option nor a medium
-    // threshold tuned earlier for this signature may shape its timings
+    // without a medium threshold: neither the option's nor one from a cache file may
+    // shape the timings
     c->mid_read_bands = INT64_MAX;
     const int blocks = batched_blocks_per_sm(b->scores_kept) * c->sm_count;
     int64_t longest = 0;
@@ -873,56 +868,12 @@ extern "C" abea_status_t abea_autotune(abea_ctx_t* c, abea_batch_t* b, int64_t* 
             best = cand;
         }
     }
-    // then the medium shape with that wide threshold: none, or the band count of
-    // the reads that leave k of the remaining reads for it (k from a quarter of the
-    // block halves to four per half) or at fractions of the longest remaining read
-    int64_t best_mid = INT64_MAX;
-    if (!st && c->wide_cluster == 0) {
-        c->long_read_bands = best;
-        std::vector<int64_t> rest;  // band counts of the reads left after the wide ones, longest first
-        int n_wide_best = 0;
-        for (int32_t i : b->order) {
-            const ReadDesc& r = b->reads[(size_t)i];
-            if (n_wide_best < blocks && !r.ck && r.n_bands >= best) {
-                ++n_wide_best;
-                continue;
-            }
-            if (!r.ck) rest.push_back(r.n_bands);
-        }
-        std::vector<int64_t> mids;
-        for (int num : {1, 2, 4, 8, 16}) {  // num/2 medium reads per block half
-            const size_t k = (size_t)std::max(1, blocks * 2 * num / 4);
-            if (k <= rest.size()) {
-                const int64_t v = std::max<int64_t>(1, rest[k - 1]);
-                if (std::find(mids.begin(), mids.end(), v) == mids.end()) mids.push_back(v);
-            }
-        }
-        if (!rest.empty())
-            for (int pct : {25, 50, 75}) {
-                const int64_t v = std::max<int64_t>(1, rest[0] * pct / 100);
-                if (std::find(mids.begin(), mids.end(), v) == mids.end()) mids.push_back(v);
-            }
-        for (int64_t cand : mids) {
-            c->mid_read_bands = cand;
-            float t_min = 1e30f;
-            for (int rep = 0; rep < 3 && !st; ++rep) {
-                if ((st = run_batch(c, b))) break;
-                if ((st = collect_timing(c, b))) break;
-                if (rep > 0) t_min = std::min(t_min, b->timing.total_ms);
-            }
-            if (st) break;
-            if (t_min < best_t * 0.98f) {  // the medium shape must buy 2%
-                best_t = t_min;
-                best_mid = cand;
-            }
-        }
-    }
     c->mode = mode0;
     c->long_read_bands = thr0;
     c->mid_read_bands = mid0;
     if (st) return st;
     c->tuned[workload_signature(b)] = best;
-    c->tuned_mid[workload_signature(b)] = best_mid;
+    c->tuned_mid.erase(workload_signature(b));  // of an older cache file
     if (best_threshold) *best_threshold = best;
     if (best_ms) *best_ms = best_t;
     return ABEA_OK;
@@ -1702,7 +1653,7 @@ static int64_t read_device_bytes(int32_t len, int32_t ne, int64_t trace_budget, 
                     8 * (int64_t)sizeof(int32_t) + 9 * (int64_t)sizeof(double);
     if (nk > 0 && ne > 0) {
         const int64_t nb = ne + nk + 2, nb4 = round_up(nb, 4);
-        bytes += 2 * 4 * round_up(ne, kChunk) + 4 * 4 * round_up(nk, kChunk) + 4 * nb4;
+        bytes += 2 * 4 * round_up(ne, kChunk) + 8 * 4 * round_up(nk, kChunk) + 4 * nb4;
         const int64_t trace = nb4 * kSlots;
         if (trace_budget > 0 && trace > trace_budget)
             bytes += 4 * (nb / kCkBands + 1) * kCkStride + (int64_t)kCkBands * kSlots;
@@ -1715,7 +1666,7 @@ static int64_t read_device_bytes(int32_t len, int32_t ne, int64_t trace_budget, 
 
 static int64_t slab_fixed_bytes() {
     return (int64_t)sizeof(abea_model_t) * ABEA_NUM_KMER + 2 * (int64_t)sizeof(double) * ABEA_NUM_KMER +
-           32 * 256 + 16 * 1024;
+           33 * 256 + 16 * 1024;
 }
 
 // Traceback cell maps of a batch holding n reads of at least kSpecMinBands bands.

@@ -9,6 +9,8 @@
 //   km_gm/km_sd/km_rsd/km_k1  f32 [per read: round_up(n_kmers,16)]  scaled level mean,
 //                       level stdv, RN(1/stdv), (log_inv_sqrt_2pi - log stdv) per
 //                       k-mer position (pre)
+//   km4                 float4 [as km_gm]  the same four side by side, for the wide shape's
+//                       emissions (one load per k-mer)
 //   last_col            f32 [per read: round_up(n_events,16)]   scores of the last
 //                       k-mer column, -inf where the cell was not computed (core)
 //   trace               u8  [per read: round_up(n_bands,4) * 128]  backpointers in

@@ -12,23 +12,20 @@
 //   warp   — one warp per read, lane l holds k-mer slots 4l..4l+3.  Neighbour
 //            scores move by one shuffle per band, the band move is decided from two
 //            shuffled end cells; no block barrier.  Most reads per SM.
-//   wide   — twelve warps of a 512-thread block per read (fill_chain): four run
-//            the band-to-band chain (one slot per thread, one barrier per band, cells
-//            exchanged in shared memory), eight compute the emissions and their exact
-//            splits up to 16 bands ahead into a ring.  Shortest band latency.
-//   medium — the same chain and producer with four producer warps, two reads per
-//            block (off unless tuned).
+//   wide   — one read per 512-thread block (fill_chain): a few warps run the band-to-band
+//            chain, cells exchanged in shared memory, the others compute the emissions
+//            ahead of it.  Shortest band latency.
 // Forms:
 //   plain   — pre, core (warp shape, one block per read), post (one block per
 //             read): the reference's three launches.
 //   batched — one persistent kernel of one block per SM (each read's pre runs
 //             in the block or warp that fills it): the blocks take the wide reads
 //             from a queue, longest first, one after another, each walking its
-//             read's traceback with the whole block (post_wide_block); then the
-//             medium reads; the blocks without a wide read take the first wave of the
-//             other reads round-robin, one per warp, and then every warp pulls the
-//             rest longest-first from a device queue; a warp-shape read's post runs
-//             in the warp that filled it, right after its fill (trace still in L2).
+//             read's traceback with the whole block (post_wide_block); the blocks
+//             without a wide read take the first wave of the other reads
+//             round-robin, one per warp, and then every warp pulls the rest
+//             longest-first from a device queue; a warp-shape read's post runs in the
+//             warp that filled it, right after its fill (trace still in L2).
 //   The wide shape on a cluster of two blocks (emissions on the second SM) is an
 //   option, measured slower.
 #include <cooperative_groups.h>
@@ -104,9 +101,12 @@ __device__ __forceinline__ CellConsts make_consts(const ReadDesc& r, const Globa
 // to host memory are in flight at once: a warp-shape read's pre stage is latency-
 // bound on them (a k-mer's six bases share the cache lines of its neighbours').
 constexpr int kPreUnroll = 4, kEvUnroll = 16;
-__device__ __forceinline__ void pre_read(const PreArgs& a, int i, int t, int nt) {
+// Returns whether some k-mer of this thread's is none for a grid (grid_kmer_ok).
+__device__ __forceinline__ bool pre_read(const PreArgs& a, int i, int t, int nt) {
     const ReadDesc r = a.reads[i];
-    if (r.skip) return;
+    if (r.skip) return false;
+    const float k1_max = grid_k1_max(r.step_h, r.stay_h);
+    bool odd = false;
     const InMirror* m = r.in_hbm ? nullptr : a.inm;
     const char* seq = a.seq;
     const abea_event_t* ev_in = a.ev_in;
@@ -146,11 +146,13 @@ __device__ __forceinline__ void pre_read(const PreArgs& a, int i, int t, int nt)
                 }
                 rsd = __frcp_rn(sd);
                 k1 = __fsub_rn(kLogInvSqrt2Pi, lsd);
+                odd |= !grid_kmer_ok(sd, k1, k1_max);
             }
             a.km_gm[r.km_off + k] = gm;
             a.km_sd[r.km_off + k] = sd;
             a.km_rsd[r.km_off + k] = rsd;
             a.km_k1[r.km_off + k] = k1;
+            if (a.km4) a.km4[r.km_off + k] = make_float4(gm, sd, rsd, k1);
         }
     }
     const int ne = r.n_events, ne_pad = round_up_dev(ne);
@@ -167,6 +169,7 @@ __device__ __forceinline__ void pre_read(const PreArgs& a, int i, int t, int nt)
             a.last_col[r.ev_off + e] = -INFINITY;
         }
     }
+    return odd;
 }
 
 __global__ void __launch_bounds__(128) abea_pre_kernel(PreArgs a) {
@@ -572,58 +575,86 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
 }
 
 // ---------------------------------------------------------------- wide shape
-// Twelve warps per read (the block's other warps wait at its next barrier):
-//   B (warps 0-3)   the band-to-band chain, one k-mer slot per thread.  Per band:
-//                   the end cells and the left neighbour of band b-1 from shared
-//                   memory, the placement, the in-band test, the exact up and
-//                   diagonal candidates (both from registers), the exact skip
-//                   candidate, the comparison, and the
-//                   bookkeeping (backpointers packed four bands to a word and
-//                   stored once per tile, band origins packed one per lane,
-//                   last k-mer column).  One 128-thread named barrier per band.
-//   E (warps 4-11)  the emissions and their exact splits, kWideChunk bands at a
-//                   time for the thread's slot (a slot keeps its k-mer while its
-//                   event advances by one per band: one load of its pore-model
-//                   parameters per chunk), up to kWideRing chunks ahead of B, into a
-//                   ring in shared memory; warps 4-7 take the even chunks, warps
-//                   8-11 the odd ones.
-// A band's cells lie on one anti-diagonal, so the placement of any band p with
-// bn - p <= 28 gives a window [k0(p), k0(p) + 128) that holds band bn's k-mers
-// (each band moves k0 by at most one): E computes a chunk from the placement B
-// published when it released the ring slot, kWideChunk * kWideRing + 1 = 17
-// bands before the chunk's last band.  B and E hand the ring slots over with
-// named barriers, FULL[s] (E arrives, B waits) and EMPTY[s] (B arrives, E waits);
-// every use of a barrier completes before its next, so arrivals never pile up.
+// A read's fill by one block of 16 warps, in chunks of four bands (a tile of
+// backpointers), by two engines over one ring of band scores in shared memory:
 //
-// The medium shape is the same chain and producer with one E group (warps 4-7)
-// and a ring of kMidRing chunks: eight warps per read, two reads per block (warps
-// 0-7 and 8-15), each half on its own named barriers.
+//   exact (chain_exact): any band.  B, warps 0-3, one k-mer slot per thread, runs the
+//     band-to-band chain with the exact sums and their proofs (abea_cell.cuh), E, warps
+//     4-11, the emissions and their splits up to 16 bands ahead.  Bound by the chain's own
+//     dependent instructions, ~330 cycles per band.
+//   grid (chain_grid): bands inside the read whose scores are all below -2^11.  A
+//     candidate is then one add of a part that E makes and proves ahead ("candidates on
+//     a grid"), the chain's bound its exchange through shared memory (94 cycles per band on
+//     a bare one), and E does the backpointers.  Measured ~150 cycles per band, E's issue
+//     slots the bound now: align() of a 20 kb read 8.10 -> 5.21 ms, the 1.3 Mbase batch of
+//     f5c's lengths 7.97 -> 5.14 ms, 1,024 reads of 1-10 kb 17.3 -> 12.7 ms.
+//
+// A band's cells lie on one anti-diagonal (event + k-mer = band - 2) and each band moves
+// k0 by at most one, so the placement of band p gives a window [k0, k0 + 128) that holds
+// the k-mers of every band up to p + 28: E works up to 28 bands ahead of B from the
+// placements that B leaves in the ring.
 constexpr int kWideThreads = 512;   // block size of the batched kernel
-constexpr int kWideChunk = 4;       // bands per emission chunk
-constexpr int kWideRing = 4;        // chunks in the wide shape's ring (kWideChunk * ring + 1 <= 28)
-constexpr int kMidRing = 2;         // chunks in the medium shape's ring
-constexpr int kMidThreads = 256;    // threads per medium read
-// Named barriers of one read (IDs from a base): base = B's per-band barrier,
-// base + 1 + s = FULL[s], base + 1 + ring + s = EMPTY[s]; the medium shape adds
-// base + 1 + 2 * ring, the half-block barrier between its reads.
-constexpr int kMidBars = 2 + 2 * kMidRing;
-static_assert(kWideChunk * kWideRing + 1 <= 28, "E's k-mer window must hold the chunk's bands");
-static_assert(kWideRing % 2 == 0, "each ring slot, and its two barriers, belongs to one of the two E groups");
-static_assert(1 + 1 + 2 * kWideRing <= 16 && 1 + 2 * kMidBars <= 16, "named barriers 0-15");
+constexpr int kWideChunk = 4;       // bands per chunk
+constexpr int kScoreRing = 32;      // bands of scores and placements in shared memory
+constexpr int kHeadRing = 16;       // chunk headers of the grid engine
+static_assert(kWideChunk == 4, "a chunk is a tile of backpointers, one word per slot");
 
-template <int kRing>
-struct alignas(16) ChainSmem {
-    // band kWideChunk*j + 2 + q of chunk j in slot j % kRing, entry [q]:
-    // {p_step, p_stay, w_step, w_stay} and {|em| + |step_h|, |em| + |stay_h|} (NaN
-    // when the emission's division was not proven)
-    float4 ems[kRing][kWideChunk][kSlots];
-    float2 emm[kRing][kWideChunk][kSlots];
-    float sc[2][kSlots];                  // band scores, buffer b & 1
-    float trim[kRing][kWideChunk];        // the trim cell's value of each band (-inf: past the read's events)
-    int32_t k0h[64];                      // placement of band b at [b & 63] (b a multiple of 4), for E
+// Exact engine.  Named barriers: 1 = B's per-band barrier, 2 + s = FULL[s] (E arrives, B
+// waits; it is also B's barrier before a chunk's first band), 6 + s = EMPTY[s].
+constexpr int kExactRing = 4, kExactGroups = 2;
+constexpr int kBarChain = 1, kBarFull = 2, kBarExEmpty = 2 + kExactRing;
+static_assert(kExactRing % kExactGroups == 0, "each ring slot, and its two barriers, belongs to one E group");
+
+// Grid engine.  B = warps 0 and 1, two slots per thread, E = five groups of two warps:
+// the warps w with w & 2, and warps 4 and 5.  A warp runs on scheduler (w & 3) of the SM,
+// so B shares its two with one group only.  Measured on a bare chain, cycles per band: 87
+// with four B warps alone and 134 with E's load on every scheduler; 94 with two, whatever
+// runs on the other two schedulers; 141 with one warp of four slots per lane.
+//   Named barriers: 1 = B's per-band barrier, 2 + g = E group g's own, 7 + s = EMPTY[s]: B
+// has released the chunk of ring slot s (B arrives, the group of the slot's next chunk
+// waits; fewer groups than slots, so no two wait on one).  The other way round a header
+// in shared memory tells B that a chunk is made: a barrier there costs the chain 68 cycles
+// per chunk, a reduction of the failed checks (bar.red) 78; a header read a chunk ahead
+// and a flag word next to nothing.
+constexpr int kGridRing = 7;        // chunks in the ring
+constexpr int kGridGroups = 5;
+constexpr int kPerLane = 2;         // slots per thread of B and of E
+constexpr int kTeam = kSlots / kPerLane;  // threads of B, and of an E group
+constexpr int kPair = 2 * kTeam;          // B and one E group on EMPTY
+constexpr int kBarGroup = 2, kBarEmpty = 2 + kGridGroups;
+constexpr int kReadyPolls = 1 << 22;      // B's polls of a header before it gives up
+static_assert(kWideChunk * kGridRing <= kSlots - kBand && kWideChunk * kExactRing <= kSlots - kBand,
+              "E's k-mer window must hold the chunk's bands");
+static_assert(kBarEmpty + kGridRing <= 16 && kBarExEmpty + kExactRing <= 16, "named barriers 0-15");
+static_assert(kGridGroups < kGridRing, "two groups never wait on one EMPTY barrier");
+static_assert(kWideChunk * kGridRing + 2 <= kScoreRing, "bands in use: two before the chunk E closes, to B's");
+static_assert(2 * kGridRing <= kHeadRing, "headers in use");
+
+// How long the exact engine runs (chunks) before the grid engine is tried: at the start,
+// again, and after failures.  A read's scores pass -2^11 after some 950 bands.
+constexpr int kFirstExact = 200, kNextExact = 32;
+
+struct alignas(16) WideSmem {
+    union {
+        struct {  // exact: band 4j + q of chunk j in slot (j - j0) % kExactRing, entry [q]
+            // {p_step, p_stay, w_step, w_stay} and {|em| + |step_h|, |em| + |stay_h|}
+            // (NaN when the emission's division was not proven)
+            float4 ems[kExactRing][kWideChunk][kSlots];
+            float2 emm[kExactRing][kWideChunk][kSlots];
+            float trim[kExactRing][kWideChunk];  // the trim cell's value (-inf: past the read's events)
+        };
+        float2 x[kGridRing][kWideChunk][kSlots];  // grid: {x_step, x_stay} (grid_pair), slot (j - j0) % kGridRing
+    };
+    float sc[kScoreRing][kSlots];   // scores of band b at [b & 31]
+    int32_t kb[kScoreRing];         // 4 * placement of band b at [b & 31]
+    // grid engine, of chunk j at [j & 15]
+    int32_t head[kHeadRing];        // made: chunk_head(j, its grid or 0 for none)
+    float2 skip[kHeadRing];         // {the grid's skip part, 1: B has stored its backpointers and origins}
+    int32_t flag;                   // a failed check
+    int32_t exit, failing;          // the first chunk not done; failures made it leave
 };
-using WideSmem = ChainSmem<kWideRing>;
-using MidSmem = ChainSmem<kMidRing>;
+__device__ __forceinline__ int chunk_head(int j, int mode) { return (j + 1) << 5 | mode; }  // never 0
+static_assert(kGridMax < 32, "five bits of mode");
 
 __device__ __forceinline__ void named_bar_sync(int id, int n) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory");
@@ -647,43 +678,6 @@ __device__ __forceinline__ bool band_moves_right(float ll, float ur, int b) {
     return (ll == -INFINITY && ur == -INFINITY) ? (bool)(b & 1) : (ll < ur);
 }
 
-// E: chunk j's emissions for slot t, from the placement kp of an earlier band.
-template <int kRing>
-__device__ __forceinline__ void wide_chunk(ChainSmem<kRing>& ws, const CoreArgs& a, const ReadDesc& r,
-                                           const CellConsts& cc, int t, int j, int kp) {
-    const int s = j % kRing, bb = 2 + kWideChunk * j;
-    const int kk = kp + ((t - kp) & (kSlots - 1));  // slot t's k-mer in the window
-    const bool kin = kk >= 0 && kk < r.n_kmers;
-    const int64_t ko = r.km_off + (kin ? kk : 0);
-    const float gm = a.km_gm[ko], sd = a.km_sd[ko], rsd = a.km_rsd[ko], k1 = a.km_k1[ko];
-    const float* ev = a.ev_mean + r.ev_off;
-    const int e_first = bb - 2 - kk;
-    float x[kWideChunk];
-#pragma unroll
-    for (int q = 0; q < kWideChunk; ++q) {
-        // cells outside the read get a finite stand-in; B's in-band test keeps them out
-        const int e = e_first + q;
-        x[q] = (kin && e >= 0 && e < r.n_events) ? ev[e] : gm;
-    }
-#pragma unroll
-    for (int q = 0; q < kWideChunk; ++q) {
-        bool ok;
-        const float em = emission_fast(x[q], gm, sd, rsd, k1, ok);
-        const EmSplit s1 = em_split(em, cc.step_h, cc.step_l);
-        const EmSplit s2 = em_split(em, cc.stay_h, cc.stay_l);
-        const float nan = __int_as_float(0x7fc00000);
-        ws.ems[s][q][t] = make_float4(s1.p, s2.p, s1.w, s2.w);
-        ws.emm[s][q][t] = ok ? make_float2(__fadd_rn(fabsf(em), fabsf(cc.step_h)), __fadd_rn(fabsf(em), fabsf(cc.stay_h)))
-                             : make_float2(nan, nan);
-    }
-    if (t < kWideChunk) {
-        // the trim cell (k = -1) of band bb + t: event bb + t - 1, (float)(lp_trim * (e + 1))
-        // (GPU/align_cuda.cl:431-443); B uses it while the band reaches below k-mer 0
-        const int e_t = bb + t - 1;
-        ws.trim[s][t] = e_t < r.n_events ? __double2float_rn(__dmul_rn(a.g.lp_trim, (double)(e_t + 1))) : -INFINITY;
-    }
-}
-
 // The reference's arithmetic for one cell whose exactness proof failed, as a
 // call: its division routine and FP64 code stay out of the band loop's body.
 struct SlowCell {
@@ -701,145 +695,147 @@ __device__ __noinline__ SlowCell slow_cell_call(float diag, float up, float left
     return o;
 }
 
-// One read's fill by warps 0 .. 4 + 4 * kGroups - 1 of the calling threads
-// (tid = index among them; others return at once): B = warps 0-3, E = the
-// kGroups groups of four warps after them, group g taking chunks g, g + kGroups,
-// ...  bar0 = the read's first named barrier.  The wide shape is kGroups = 2 with
-// kWideRing chunks, the medium shape kGroups = 1 with kMidRing.
-template <bool kScores, int kGroups, int kRing>
-__device__ void fill_chain(const CoreArgs& a, const ReadDesc& r, ChainSmem<kRing>& ws, int tid, int bar0) {
-    static_assert(kGroups == 1 || kRing % kGroups == 0, "each ring slot belongs to one E group");
-    const int warp = tid >> 5;
-    if (warp >= 4 + 4 * kGroups) return;
-    const CellConsts cc = make_consts(r, a.g);
-    const int n_events = r.n_events, n_kmers = r.n_kmers, n_bands = r.n_bands;
-    const int n_chunks = (n_bands - 2 + kWideChunk - 1) / kWideChunk;
-    const int t = tid & (kSlots - 1);
-    constexpr int kPair = 2 * kSlots;  // B and E threads on FULL / EMPTY
-    const int kBarChain = bar0, kBarFull = bar0 + 1, kBarEmpty = bar0 + 1 + kRing;
+// A read as the two engines see it.
+struct WideRead {
+    const CoreArgs& a;
+    const ReadDesc& r;
+    WideSmem& ws;
+    CellConsts cc;
+    int n_events, n_kmers, n_bands, n_chunks;
+    uint8_t* trace;
+    int32_t* bk0;
+    float* scores;
 
+    // the origins of chunk j's bands, by threads 0-3
+    __device__ __forceinline__ void store_origins(int j, int t) const {
+        const int band = kWideChunk * j + t;
+        if (t < kWideChunk && band < n_bands && in_bounds(band, n_bands, a.counters))
+            bk0[band] = ws.kb[band & (kScoreRing - 1)] >> 2;
+    }
+    __device__ __forceinline__ bool tile_in(int j) const { return in_bounds(j, (n_bands + 3) / 4, a.counters); }
+    // the end cells of band b-1 (its row of the ring) and the left neighbour of a slot
+    __device__ __forceinline__ void ends(int row, int k0, float& ll, float& ur) const {
+        ll = ws.sc[row][k0 & (kSlots - 1)];
+        ur = ws.sc[row][(k0 + kBand - 1) & (kSlots - 1)];
+    }
+};
+
+// ---- exact engine
+// E: chunk j's emissions for slot t into ring slot s, from the placement kp of an earlier
+// band.
+__device__ __forceinline__ void exact_chunk(const WideRead& w, int t, int s, int j, int kp) {
+    const ReadDesc& r = w.r;
+    const int kk = kp + ((t - kp) & (kSlots - 1));  // slot t's k-mer in the window
+    const bool kin = kk >= 0 && kk < w.n_kmers;
+    const float4 km = w.a.km4[r.km_off + (kin ? kk : 0)];
+    const float gm = km.x, sd = km.y, rsd = km.z, k1 = km.w;
+    const float* ev = w.a.ev_mean + r.ev_off;
+    const int b0 = kWideChunk * j, e_first = b0 - 2 - kk;
+    float x[kWideChunk];
+#pragma unroll
+    for (int q = 0; q < kWideChunk; ++q) {
+        // cells outside the read get a finite stand-in; B's in-band test keeps them out
+        const int e = e_first + q;
+        x[q] = (kin && e >= 0 && e < w.n_events) ? ev[e] : gm;
+    }
+#pragma unroll
+    for (int q = 0; q < kWideChunk; ++q) {
+        bool ok;
+        const float em = emission_fast(x[q], gm, sd, rsd, k1, ok);
+        const EmSplit s1 = em_split(em, w.cc.step_h, w.cc.step_l);
+        const EmSplit s2 = em_split(em, w.cc.stay_h, w.cc.stay_l);
+        const float nan = __int_as_float(0x7fc00000);
+        w.ws.ems[s][q][t] = make_float4(s1.p, s2.p, s1.w, s2.w);
+        w.ws.emm[s][q][t] = ok ? make_float2(__fadd_rn(fabsf(em), fabsf(w.cc.step_h)),
+                                             __fadd_rn(fabsf(em), fabsf(w.cc.stay_h)))
+                               : make_float2(nan, nan);
+    }
+    if (t < kWideChunk) {
+        // the trim cell (k = -1) of band b0 + t: event b0 + t - 1, (float)(lp_trim * (e + 1))
+        // (GPU/align_cuda.cl:431-443); B uses it while the band reaches below k-mer 0
+        const int e_t = b0 + t - 1;
+        w.ws.trim[s][t] = e_t < w.n_events ? __double2float_rn(__dmul_rn(w.a.g.lp_trim, (double)(e_t + 1))) : -INFINITY;
+    }
+}
+
+// Chunks j0 .. j1 - 1, from the bands before them in the score ring; every thread of the
+// block calls it.
+template <bool kScores>
+__device__ __forceinline__ void chain_exact(const WideRead& w, int tid, int j0, int j1) {
+    const int warp = tid >> 5;
+    if (warp >= 4 + 4 * kExactGroups) return;
+    WideSmem& ws = w.ws;
+    const ReadDesc& r = w.r;
+    const CoreArgs& a = w.a;
+    const int n_events = w.n_events, n_kmers = w.n_kmers, n_bands = w.n_bands;
+    const int t = tid & (kSlots - 1), tl = (t + kSlots - 1) & (kSlots - 1);
+    constexpr int kBoth = 2 * kSlots;  // B and one E group on FULL / EMPTY
+    const int before = (kWideChunk * j0 - 1) & (kScoreRing - 1);  // band 4 j0 - 1
+    const int k_start = ws.kb[before] >> 2;
     if (warp >= 4) {
-        // ------------------------------------------------ E: the emission chunks; with
-        // two groups each has two chunks of B's time for the loads and arithmetic of one
-        for (int j = (warp >> 2) - 1; j < n_chunks; j += kGroups) {
-            const int s = j % kRing;
-            int kp = -1 - kBand / 2;  // band 1's placement, for the first kRing chunks
-            if (j >= kRing) {
-                named_bar_sync(kBarEmpty + s, kPair);  // B released chunk j - kRing
-                kp = ws.k0h[(kWideChunk * (j - kRing) + kWideChunk) & 63];  // band bb(j - R) + C - 2
+        for (int j = j0 + (warp >> 2) - 1; j < j1; j += kExactGroups) {
+            const int s = (j - j0) & (kExactRing - 1), jr = j - kExactRing;
+            int kp = k_start;
+            if (jr >= j0) {
+                named_bar_sync(kBarExEmpty + s, kBoth);  // B released chunk jr
+                kp = ws.kb[(kWideChunk * jr + kWideChunk - 1) & (kScoreRing - 1)] >> 2;
             }
-            wide_chunk(ws, a, r, cc, t, j, kp);
-            named_bar_arrive(kBarFull + s, kPair);
+            exact_chunk(w, t, s, j, kp);
+            named_bar_arrive(kBarFull + s, kBoth);
         }
         return;
     }
-
-    // ------------------------------------------------ B: the chain
-    // One iteration per chunk, its kWideChunk bands unrolled: the chunk's barriers
-    // and the backpointer tile stores fall on fixed bands.  Band b-1's bookkeeping
-    // (backpointers, band origin, last k-mer column, scores) runs just after band
-    // b's barrier, beside the loads, so that nothing but the chain stands between
-    // a band's comparison and the next barrier.
-    const int lane = tid & 31;
-    uint8_t* trace = a.trace + r.trace_off * kSlots;
-    int32_t* bk0 = a.band_k0 + r.band_off;
+    // B.  band b's placement: lower-left k-mer k0, event e0 = b - 2 - k0, so only k0 is
+    // carried; s1 = band b-1's score of this slot, lp = band b's diagonal (band b-2's score
+    // of slot t-1).  Before band 2: bands 1 and 0.
+    int k0 = k_start;
+    float s1 = ws.sc[j0 ? before : 1][t], lp = ws.sc[j0 ? (before - 1) & (kScoreRing - 1) : 0][tl];
     float* lastc = a.last_col + r.ev_off;
-    float* scores = kScores ? a.scores + r.band_off * kSlots : nullptr;
     const int sl_last = (n_kmers - 1) & (kSlots - 1);
-
-    // band b's placement: lower-left k-mer k0, event e0 = b - 2 - k0 (a band's cells
-    // lie on one anti-diagonal), so only k0 is carried
-    int k0 = -1 - kBand / 2;                         // band 1 (band 0 is (49,-51), band 1 moved down)
-    float s1 = (t == 127) ? a.g.trim_f : -INFINITY;  // band b-1's score of this slot
-    float lp = (t == 0) ? 0.0f : -INFINITY;          // band b-2's score of slot t-1: band b's diagonal
-    ws.sc[1][t] = s1;
-    if (kScores) {
-        scores[t] = (t == 127) ? 0.0f : -INFINITY;
-        scores[kSlots + t] = s1;
-    }
-    int my_k0 = k0;                                      // band origins: band b in lane b & 31 (bands 0, 1: -51)
-    uint32_t tw = 0u;                                    // backpointers of bands 4m..4m+3, byte b & 3
-    uint32_t from_p = (t == 127) ? ABEA_FROM_U : 0u;     // band b-1's backpointer (band 1: the trim cell)
     unsigned long long slow = 0;
-    // Band bk's bookkeeping; q1 = bk & 3 when known at compile time, else -1.  No
-    // branches: a branch in the unrolled band body splits the code the compiler
-    // schedules as one block (measured: a band-uniform branch around the
-    // last-column store cost 27 cycles per band).  The placement of every fourth
-    // band (the one E reads) goes to the ring k0h; band origins are kept one per
-    // lane of warp 0 and stored 32 bands at a time.
-    auto book = [&](int bk, int q1, bool last_col, bool mine) {
-        if (q1 >= 0) {  // the byte's place known when compiled: one byte insert
-            constexpr unsigned kSel[4] = {0x3214u, 0x3240u, 0x3410u, 0x4210u};
-            tw = __byte_perm(tw, from_p, kSel[q1 & 3]);
-        } else {
-            tw |= from_p << (8 * (bk & 3));
-        }
-        // band bk's placement is still k0: the band after it moves k0 after this
-        my_k0 = mine ? k0 : my_k0;
-        if (t == 0 && (bk & 3) == 0) ws.k0h[bk & 63] = k0;
+    // band b's last-column score and, optionally, its scores
+    auto keep = [&](int b, bool last_col) {
         if (last_col) {
-            const int ol = n_kmers - 1 - k0, e0p = bk - 2 - k0;
-            int lop, hip;  // band bk's computed offsets
-            band_range(k0, e0p, n_events, n_kmers, lop, hip);
-            if (t == sl_last && ol >= lop && ol < hip && in_bounds(e0p - ol, n_events, a.counters))
-                lastc[e0p - ol] = s1;
+            const int ol = n_kmers - 1 - k0, e0 = b - 2 - k0;
+            int lo, hi;
+            band_range(k0, e0, n_events, n_kmers, lo, hi);
+            if (t == sl_last && ol >= lo && ol < hi && in_bounds(e0 - ol, n_events, a.counters)) lastc[e0 - ol] = s1;
         }
-        if (kScores && in_bounds(bk, n_bands, a.counters)) scores[(int64_t)bk * kSlots + t] = s1;
+        if (kScores && in_bounds(b, n_bands, a.counters)) w.scores[(int64_t)b * kSlots + t] = s1;
     };
-    auto store_tile = [&](int bk) {
-        if (in_bounds(bk >> 2, (n_bands + 3) / 4, a.counters))
-            reinterpret_cast<uint32_t*>(trace + (int64_t)(bk >> 2) * 512)[t] = tw;
-        tw = 0u;
-    };
-    auto store_origins = [&](int bk, bool now) {  // bands (bk & ~31) .. bk, when `now`
-        const int band = (bk & ~31) + lane;
-        if (now && warp == 0 && lane <= (bk & 31) && in_bounds(band, n_bands, a.counters)) bk0[band] = my_k0;
-    };
-    // One chunk of kWideChunk bands; kLast: the read may end inside it (the only
-    // chunk that tests for the end: a test per band is a branch in the band body).
-    // kMid: a chunk inside the read, where every band's computed cells are all 100
-    // (offsets [0, 100)), none is the trim cell and none lies on the last k-mer
-    // column (and neither does band bb-1, whose bookkeeping the chunk finishes): k0
-    // and e0 each move by at most one per band, so the placement of band bb-1
-    // decides it for the whole chunk.
-    // kOpt: optimistic (middle chunks only): no per-band check of the exactness
-    // proofs; each thread ORs its failed proofs into `dirty`, the barrier that ends
-    // the chunk reduces them (open_chunk), and a chunk with any is done again with
-    // the checks (kRedo: its emissions are still in the ring, whose slot is
-    // released only after that barrier).  The chunk's first chain barrier is the
-    // caller's (open_chunk), except in a redo.
-    bool dirty = false;
-    auto chunk = [&](int j, auto last, auto mid, auto opt, auto redo) {
-        constexpr bool kLast = decltype(last)::value, kMid = decltype(mid)::value;
-        constexpr bool kOpt = decltype(opt)::value, kRedo = decltype(redo)::value;
-        static_assert(!kOpt || kMid, "only middle chunks run optimistic");
-        const int s = j % kRing, bb = 2 + kWideChunk * j;
-        const int dl = (lane - 1 - kWideChunk * j) & 31;  // band bb-1+q's origin goes to lane (bb-1+q) & 31: dl == q
+    // One chunk, its bands unrolled; band b-1's last-column store runs beside band b's
+    // loads.  kEdge: the read may begin or end inside it (the only chunks that test for
+    // it: a test per band is a branch in the band body, measured 27 cycles per band).
+    // kMid: all 100 cells of its bands are computed, none of them the trim cell or on the
+    // last k-mer column.
+    auto chunk = [&](int j, auto edge, auto mid) {
+        constexpr bool kEdge = decltype(edge)::value, kMid = decltype(mid)::value;
+        const int s = (j - j0) & (kExactRing - 1), b0 = kWideChunk * j;
+        const int r0 = b0 & (kScoreRing - 1);
+        uint32_t word = (kEdge && j == 0 && t == 127) ? ABEA_FROM_U << 8 : 0u;  // band 1's trim cell
+        bool begun = false;
+        named_bar_sync(kBarFull + s, kBoth);  // chunk j's emissions, and band b0-1's scores
 #pragma unroll
         for (int q = 0; q < kWideChunk; ++q) {
-            const int b = bb + q;
-            if (kLast && b >= n_bands) break;
-            if (q > 0 || kRedo) named_bar_sync(kBarChain, kSlots);  // band b-1's scores are in shared memory
-            if (q == 0 && !kRedo) named_bar_sync(kBarFull + s, kPair);  // chunk j's emissions are in the ring
-            const int pb = (b - 1) & 1;
-            const float ll = ws.sc[pb][k0 & 127];
-            const float ur = ws.sc[pb][(k0 + kBand - 1) & 127];
-            const float left = ws.sc[pb][(t + 127) & 127];
+            const int b = b0 + q;
+            if (kEdge && (b < 2 || b >= n_bands)) continue;
+            if (q > 0) named_bar_sync(kBarChain, kSlots);  // band b-1's scores are in shared memory
+            const int row = q > 0 ? r0 + q - 1 : (r0 - 1) & (kScoreRing - 1);
+            float ll, ur;
+            w.ends(row, k0, ll, ur);
+            const float left = ws.sc[row][tl];
             const float4 ep = ws.ems[s][q][t];
             const float2 mm = ws.emm[s][q][t];
             const float tv = ws.trim[s][q];
-            // band b-1's bookkeeping (bands 2 + 4j + q - 1: b-1 & 3 == (q + 1) & 3)
-            book(b - 1, (q + 1) & 3, !kMid, dl == q);
-            if (q == 2) {  // band b-1 closes a tile of four bands, every eighth one 32 bands
-                store_tile(b - 1);
-                store_origins(b - 1, ((b - 1) & 31) == 31);
-            }
-            // the exact diagonal and up candidates of band b
+            if (kEdge ? begun : q > 0) keep(b - 1, !kMid);
+            begun = true;
+            // the exact diagonal and up candidates
             bool okd, oku;
             const float d = exact_from_split(lp, EmSplit{ep.x, ep.z}, mm.x, okd);
             const float u = exact_from_split(s1, EmSplit{ep.y, ep.w}, mm.y, oku);
             const bool right = band_moves_right(ll, ur, b);
             k0 += right ? 1 : 0;
+            if (t == 0) ws.kb[r0 + q] = 4 * k0;
             const int e0 = b - 2 - k0;
             int lo = 0, hi = kBand;
             if (!kMid) band_range(k0, e0, n_events, n_kmers, lo, hi);
@@ -849,21 +845,16 @@ __device__ void fill_chain(const CoreArgs& a, const ReadDesc& r, ChainSmem<kRing
             uint32_t from_du, from;
             const float best_du = pick_du(d, u, from_du);
             bool okl;
-            const float l = exact_skip(left, cc.skip_h, cc.skip_l, okl);
+            const float l = exact_skip(left, w.cc.skip_h, w.cc.skip_l, okl);
             float best = pick_l(best_du, from_du, l, from);
-            const bool proven = okd && oku && okl;
-            const bool bad = valid && !proven;
+            const bool bad = valid && !(okd && oku && okl);
             best = valid ? best : -INFINITY;
-            if (!kMid) from = valid ? from : 0u;  // a middle chunk's invalid slots are outside the band
-            const bool here = !kMid && (t == 127) && (k0 <= -1) && (k0 >= -kBand);
+            if (!kMid) from = valid ? from : 0u;  // a mid chunk's invalid slots are outside the band
+            const bool here = !kMid && (t == 127) && (k0 <= -1) && (k0 >= -kBand);  // the trim cell
             best = here ? tv : best;
             from = here ? (tv == -INFINITY ? 0u : ABEA_FROM_U) : from;
-            ws.sc[b & 1][t] = best;  // stored before the check: only the rare path stores again
-            if (kOpt) {
-                // out-of-band cells count too: one test fewer per band, a redo
-                // seldom more (measured 1.6% faster)
-                dirty = dirty || !proven;
-            } else if (__any_sync(kFull, bad)) {
+            ws.sc[r0 + q][t] = best;  // stored before the check: only the rare path stores again
+            if (__any_sync(kFull, bad)) {
                 // Rare: a proof failed in some lane, whose cell takes the reference's
                 // FP64 arithmetic and stores its score again.  The whole warp calls (a
                 // divergent branch around the call cost 20 cycles per band); the other
@@ -871,83 +862,421 @@ __device__ void fill_chain(const CoreArgs& a, const ReadDesc& r, ChainSmem<kRing
                 // bad lane's cell does, and drop the result.
                 const int64_t ko = r.km_off + (bad ? k0 + o : 0);
                 const SlowCell c = slow_cell_call(lp, s1, left, a.ev_mean[r.ev_off + (bad ? e0 - o : 0)], a.km_gm[ko],
-                                                  a.km_sd[ko], a.km_k1[ko], cc.lp_step, cc.lp_stay, cc.lp_skip);
+                                                  a.km_sd[ko], a.km_k1[ko], w.cc.lp_step, w.cc.lp_stay, w.cc.lp_skip);
                 const bool use = bad && !here;
                 best = use ? c.best : best;
                 from = use ? c.from : from;
                 slow += use ? 1 : 0;
-                ws.sc[b & 1][t] = best;
+                ws.sc[r0 + q][t] = best;
             }
-            if (!kOpt && !kRedo && q == kWideChunk - 1 && j + kRing < n_chunks)
-                named_bar_arrive(kBarEmpty + s, kPair);  // chunk j read: E may refill its slot
+            word |= from << (8 * q);
             lp = left;
             s1 = best;
-            from_p = from;
+        }
+        if (j + kExactRing < j1) named_bar_arrive(kBarExEmpty + s, kBoth);  // E may refill its slot
+        keep(min(b0 + kWideChunk, n_bands) - 1, !kMid);
+        if (w.tile_in(j)) reinterpret_cast<uint32_t*>(w.trace + (int64_t)j * 512)[t] = word;
+        if (warp == 0) {
+            __syncwarp();  // thread 0 wrote the placements
+            w.store_origins(j, t);
         }
     };
-    // The state an optimistic chunk starts from (band bb-1's placement, score,
-    // backpointer and the diagonal of band bb, the backpointer word, the band
-    // origins: its last band may have started the next 32), for its redo.
-    int sv_k0 = 0, sv_myk0 = 0, pj = -1;
-    float sv_s1 = 0.f, sv_lp = 0.f;
-    uint32_t sv_from = 0u, sv_tw = 0u;
     using F = std::false_type;
     using T = std::true_type;
-    // The barrier that ends band bb-1 before chunk j (bb = 2 + 4j), or before the
-    // last band's bookkeeping (j = n_chunks).  After an optimistic chunk it also
-    // reduces that chunk's failed proofs; with any, the chunk is done again from
-    // its saved state, with the checks.  Then the chunk's ring slot is released.
-    auto open_chunk = [&](int j) {
-        if (pj < 0) {
-            named_bar_sync(kBarChain, kSlots);
-            return;
-        }
-        if (named_bar_any(kBarChain, kSlots, dirty)) {
-            k0 = sv_k0;
-            s1 = sv_s1;
-            lp = sv_lp;
-            from_p = sv_from;
-            tw = sv_tw;
-            my_k0 = sv_myk0;
-            ws.sc[(1 + kWideChunk * pj) & 1][t] = s1;  // band bb-1's scores, which the chunk overwrote
-            chunk(pj, F{}, T{}, F{}, T{});              // its first barrier publishes them
-            named_bar_sync(kBarChain, kSlots);
-        }
-        if (pj + kRing < n_chunks) named_bar_arrive(kBarEmpty + pj % kRing, kPair);  // E may refill the slot
-        pj = -1;
-        dirty = false;
-        (void)j;
-    };
-    const int n_full = (n_bands - 2) / kWideChunk;
-    for (int j = 0; j < n_full; ++j) {
-        open_chunk(j);
-        const int e0 = kWideChunk * j - 1 - k0;  // band bb-1's event (bb = 2 + 4j)
-        if (k0 >= 0 && k0 + kWideChunk <= n_kmers - 1 - kBand && e0 >= kBand - 1 && e0 + kWideChunk <= n_events - 1) {
-            sv_k0 = k0;
-            sv_s1 = s1;
-            sv_lp = lp;
-            sv_from = from_p;
-            sv_tw = tw;
-            sv_myk0 = my_k0;
-            pj = j;
-            chunk(j, F{}, T{}, T{}, F{});
-        } else {
-            chunk(j, F{}, F{}, F{}, F{});
-        }
-    }
-    if (n_full < n_chunks) {
-        open_chunk(n_full);
-        chunk(n_full, T{}, F{}, F{}, F{});
-    } else if (n_bands > 2) {
-        open_chunk(n_chunks);  // the last chunk may have been optimistic
-    }
-    if (n_bands > 2) {  // the last band's bookkeeping and the stores it closes
-        const int bl = n_bands - 1;
-        book(bl, -1, true, (bl & 31) == lane);
-        store_tile(bl);
-        store_origins(bl, true);
+    for (int j = j0; j < j1; ++j) {
+        // band 4j - 1's placement decides for the whole chunk: k0 and e0 each move by at
+        // most one per band
+        const int e0 = kWideChunk * j - 3 - k0;
+        if (j == 0 || kWideChunk * (j + 1) > n_bands)
+            chunk(j, T{}, F{});
+        else if (k0 >= 0 && k0 + kWideChunk + kBand <= n_kmers - 1 && e0 >= kBand - 1 && e0 + kWideChunk <= n_events - 1)
+            chunk(j, F{}, T{});
+        else
+            chunk(j, F{}, F{});
     }
     if (slow) atomicAdd(&a.counters[0], slow);
+}
+
+// ---- grid engine
+// E: a chunk's candidate parts (grid_pair) for thread t's slots into ring slot s.
+// chunk_mode keeps such chunks inside the read: every slot of the window has a k-mer and
+// its four events.
+template <bool kLow>
+__device__ __forceinline__ void grid_chunk(WideSmem& ws, const float4* km4, const float* ev, const Grid& G, int t, int s,
+                                           int b0, int kp) {
+    float4 km[kPerLane];
+    float x[kPerLane][kWideChunk];
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) {
+        const int kk = kp + ((kPerLane * t + i - kp) & (kSlots - 1));
+        km[i] = km4[kk];
+        const float* e = ev + (b0 - 2 - kk);
+#pragma unroll
+        for (int q = 0; q < kWideChunk; ++q) x[i][q] = e[q];
+    }
+#pragma unroll
+    for (int q = 0; q < kWideChunk; ++q) {
+        const float2 g0 = grid_pair<kLow>(x[0][q], km[0].x, km[0].y, km[0].z, km[0].w, G);
+        const float2 g1 = grid_pair<kLow>(x[1][q], km[1].x, km[1].y, km[1].z, km[1].w, G);
+        *reinterpret_cast<float4*>(&ws.x[s][q][kPerLane * t]) = make_float4(g0.x, g0.y, g1.x, g1.y);
+    }
+}
+
+// The grid for a band's scores (its row of the ring; 0: none), the same in every warp:
+// the binade of the largest one, when the smallest is at most 4 times it.  It serves
+// chunks that end up to 68 bands on, whose scores are above -38 * 2^m (-50 * 2^m when a
+// run of chunks began on the way, at above -16 * 2^m): a band's scores fall by less than
+// 2^(m-1) from its predecessors'.
+__device__ __forceinline__ int grid_of(const float* row, int lane, uint32_t modes) {
+    const float4 v = reinterpret_cast<const float4*>(row)[lane];
+    auto fin = [](float x) { return x > -INFINITY ? x : 0.0f; };
+    const float mx = warp_max(fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+    const float mn = warp_min(fminf(fminf(fin(v.x), fin(v.y)), fminf(fin(v.z), fin(v.w))));
+    const int m = (__float_as_int(-mx) >> 23) - 127;  // a positive mx: negative; -inf: 128
+    const int mlo = (__float_as_int(-mn) >> 23) - 127;
+    return m >= kGridMin && m <= kGridMax && mlo < m + 2 && ((modes >> (m & 31)) & 1u) ? m : 0;
+}
+static_assert(kWideChunk * (kGridRing + 2 * kGridGroups) <= 68, "bands from the one that decides a grid to the chunk's last");
+
+// Grid `want` for the chunk of bands b0 .. b0 + 3 if the 128-slot window at the placement
+// kp of a band up to 28 bands before its last lies inside the read with every event of
+// the chunk (so do the chunk's cells, none of them the trim cell or on the last k-mer
+// column); else 0.
+__device__ __forceinline__ int chunk_mode(int want, int kp, int b0, int n_events, int n_kmers) {
+    const bool in = kp >= 0 && kp <= n_kmers - kSlots && b0 - 1 - kSlots - kp >= 0 &&
+                    b0 + kWideChunk - 3 - kp <= n_events - 1;
+    return in ? want : 0;
+}
+
+// Chunks from j0 on, until one that no grid serves (ws.exit), from the bands before them
+// in the score ring; `first`: the grid of those.  Every thread of the block calls it, with
+// ws.head and ws.flag zero and ws.exit the largest int.
+template <bool kScores>
+__device__ __forceinline__ void chain_grid(const WideRead& w, int tid, int j0, int first, uint32_t modes) {
+    const int warp = tid >> 5, lane = tid & 31;
+    if ((warp & 3) < 2 && warp >= 6) return;
+    WideSmem& ws = w.ws;
+    const ReadDesc& r = w.r;
+    const CoreArgs& a = w.a;
+    const CellConsts& cc = w.cc;
+    const int n_events = w.n_events, n_kmers = w.n_kmers;
+    const int t = tid & (kTeam - 1);  // slots 2t and 2t + 1
+    const int tl = (kPerLane * t + kSlots - 1) & (kSlots - 1);
+    const int k_start = ws.kb[(kWideChunk * j0 - 1) & (kScoreRing - 1)] >> 2;
+    auto store_scores = [&](int b, float v0, float v1) {
+        if (kScores && in_bounds(b, w.n_bands, a.counters))
+            reinterpret_cast<float2*>(w.scores + (int64_t)b * kSlots)[t] = make_float2(v0, v1);
+    };
+    auto store_tile = [&](int j, uint32_t w0, uint32_t w1) {
+        if (w.tile_in(j)) reinterpret_cast<uint2*>(w.trace + (int64_t)j * 512)[t] = make_uint2(w0, w1);
+    };
+
+    if (warp >= 2) {
+        // ------------------------------------------------ E: closes chunk j - kGridRing and makes chunk j
+        const int group = warp & 2 ? warp >> 2 : kGridGroups - 1;
+        const float4* km4 = a.km4 + r.km_off;
+        const float* ev = a.ev_mean + r.ev_off;
+        Grid G{};
+        int g_mode = 0, want = first;  // want: the grid of the scores at one of the group's last two turns
+        for (int j = j0 + group, s = group, turn = 0;; j += kGridGroups, ++turn) {
+            const int jr = j - kGridRing, b0 = kWideChunk * j, br = kWideChunk * jr;
+            int kp = k_start;
+            const bool closes = jr >= j0;
+            if (closes) {
+                named_bar_sync(kBarEmpty + s, kPair);  // B released chunk jr
+                if (jr >= ws.exit) break;
+                kp = ws.kb[(br + kWideChunk - 1) & (kScoreRing - 1)] >> 2;
+            }
+            const int mode = chunk_mode(want, kp, b0, n_events, n_kmers);
+            if (closes) {
+                const float2 sk = ws.skip[jr & (kHeadRing - 1)];
+                if (turn & 1) want = grid_of(ws.sc[(br + 3) & (kScoreRing - 1)], lane, modes);
+                if (sk.y == 0.0f) {
+                    // the moves from the scores, as the comparison took them
+                    const float xl = sk.x;
+                    const float* row = ws.sc[(br - 1) & (kScoreRing - 1)];
+                    float2 up = *reinterpret_cast<const float2*>(row + kPerLane * t);
+                    float left = row[tl];
+                    uint32_t w0 = 0u, w1 = 0u;
+#pragma unroll
+                    for (int q = 0; q < kWideChunk; ++q) {
+                        row = ws.sc[(br & (kScoreRing - 1)) + q];
+                        const float2 v = *reinterpret_cast<const float2*>(row + kPerLane * t);
+                        const float4 x = *reinterpret_cast<const float4*>(&ws.x[s][q][kPerLane * t]);
+                        const float l0 = __fadd_rn(left, xl), l1 = __fadd_rn(up.x, xl);
+                        const float u0 = __fadd_rn(up.x, x.y), u1 = __fadd_rn(up.y, x.w);
+                        if (v.x == l0) w0 |= ABEA_FROM_L << (8 * q);
+                        if (v.x == u0 && v.x != l0) w0 |= ABEA_FROM_U << (8 * q);
+                        if (v.y == l1) w1 |= ABEA_FROM_L << (8 * q);
+                        if (v.y == u1 && v.y != l1) w1 |= ABEA_FROM_U << (8 * q);
+                        store_scores(br + q, v.x, v.y);
+                        up = v;
+                        left = row[tl];
+                    }
+                    store_tile(jr, w0, w1);
+                    w.store_origins(jr, t);
+                }
+            }
+            if (mode) {
+                if (mode != g_mode) G = make_grid(cc, mode);
+                g_mode = mode;
+                if (mode < kGridWide)
+                    grid_chunk<true>(ws, km4, ev, G, t, s, b0, kp);
+                else
+                    grid_chunk<false>(ws, km4, ev, G, t, s, b0, kp);
+            }
+            named_bar_sync(kBarGroup + group, kTeam);
+            if (t == 0) {
+                ws.skip[j & (kHeadRing - 1)] = make_float2(G.skip, 0.0f);
+                __threadfence_block();
+                *(volatile int32_t*)&ws.head[j & (kHeadRing - 1)] = chunk_head(j, mode);
+            }
+            s = s + kGridGroups >= kGridRing ? s + kGridGroups - kGridRing : s + kGridGroups;
+        }
+        return;
+    }
+
+    // ------------------------------------------------ B: the chain
+    // Every cell of the chunks' bands is computed (100 per band) and finite when the first
+    // band's predecessors are (checked on entry): a cell has its up neighbour or, at the
+    // band's new right end, its left one.  No score exceeds those before it, E bounds how
+    // far they fall, and a NaN in a cell reaches the next band (its own slot's up candidate
+    // or, where the slot left the band, its right neighbour's skip): so the scores that a
+    // chunk ends with show a failed proof.
+    //   A chunk's check runs in the next one: `pend` says that one awaits it, kb_pend and
+    // kb_cur are 4 * the placements that it and the current one started from.
+    int k0 = k_start;
+    float s1[kPerLane], lp[kPerLane];  // band b-1's scores of the slots; band b's diagonals
+    float xl = 0.0f, g_lim = 0.0f;
+    int g_mode = 0;
+    int pen = 0;  // 8 for a failed chunk, -1 for a good one
+    unsigned long long slow = 0;
+    constexpr uint32_t kOne = 1u << 25, kIn = (uint32_t)kBand << 25;
+    auto release = [&](int s) { named_bar_arrive(kBarEmpty + s, kPair); };  // E closes the chunk and refills its slot
+    // the state before chunk j, from the score ring
+    auto restore = [&](int j, int kb) {
+        const int row = kWideChunk * j;
+        const float2 v = *reinterpret_cast<const float2*>(&ws.sc[(row - 1) & (kScoreRing - 1)][kPerLane * t]);
+        k0 = kb >> 2;
+        s1[0] = v.x;
+        s1[1] = v.y;
+        lp[0] = ws.sc[(row - 2) & (kScoreRing - 1)][tl];
+        lp[1] = ws.sc[(row - 2) & (kScoreRing - 1)][kPerLane * t];
+    };
+    // A failed chunk again from its start in the reference's FP64 arithmetic, rare.
+    auto redo = [&](int j, int kb) {
+        restore(j, kb);
+        pen += 8;
+        uint32_t word[kPerLane] = {0u, 0u};
+#pragma unroll 1
+        for (int q = 0; q < kWideChunk; ++q) {
+            const int b = kWideChunk * j + q, row = (b - 1) & (kScoreRing - 1);
+            float ll, ur;
+            w.ends(row, k0, ll, ur);
+            const float left[kPerLane] = {ws.sc[row][tl], s1[0]};
+            k0 += band_moves_right(ll, ur, b) ? 1 : 0;
+            if (t == 0) ws.kb[b & (kScoreRing - 1)] = 4 * k0;
+#pragma unroll
+            for (int i = 0; i < kPerLane; ++i) {
+                const int o = (kPerLane * t + i - k0) & (kSlots - 1);
+                const bool valid = o < kBand;
+                const int kk = k0 + (valid ? o : 0);  // the chunk's bands lie inside the read
+                const int64_t ko = r.km_off + kk;
+                const SlowCell c = slow_cell_call(lp[i], s1[i], left[i], a.ev_mean[r.ev_off + (b - 2 - kk)], a.km_gm[ko],
+                                                  a.km_sd[ko], a.km_k1[ko], cc.lp_step, cc.lp_stay, cc.lp_skip);
+                lp[i] = left[i];
+                s1[i] = valid ? c.best : -INFINITY;
+                word[i] |= (valid ? c.from : 0u) << (8 * q);
+                slow += valid ? 1 : 0;
+            }
+            *reinterpret_cast<float2*>(&ws.sc[b & (kScoreRing - 1)][kPerLane * t]) = make_float2(s1[0], s1[1]);
+            store_scores(b, s1[0], s1[1]);
+            named_bar_sync(kBarChain, kTeam);
+        }
+        store_tile(j, word[0], word[1]);
+        w.store_origins(j, t);
+        if (t == 0) ws.skip[j & (kHeadRing - 1)].y = 1.0f;
+    };
+    // Runs chunks from chunk j (made, its start checked, every warp past a barrier after
+    // band 4j-1) until one that has another grid or none, or a failed check; j is then that
+    // chunk.  true: the check of chunk j-1 failed (and chunk j has begun).  The last barrier
+    // passed is the one after band 4j-1.
+    int kb_cur = 0, kb_pend = 0;
+    bool pend = false;
+    auto run = [&](int& j, int& s, auto low) {
+        constexpr bool kLow = decltype(low)::value;  // emissions may be below the range
+        uint32_t vs = (uint32_t)(kPerLane * t - k0) << 25;  // slot 2t's offset in the band, mod 128, at the top of the word
+        int kb = 4 * k0;
+        bool below = false;
+        pend = false;
+        char* const sc = reinterpret_cast<char*>(&ws.sc[0][0]);
+        constexpr int kRow = 4 * kSlots, kRows = kScoreRing * kRow;
+        int rw = (kWideChunk * j * kRow) & (kRows - 1);  // byte offset of the chunk's first score row
+        while (true) {
+            kb_cur = kb;
+            int fl = 0, head = 0;
+#pragma unroll
+            for (int q = 0; q < kWideChunk; ++q) {
+                if (q > 0) named_bar_sync(kBarChain, kTeam);
+                const char* row = sc + (q > 0 ? rw + (q - 1) * kRow : (rw - kRow) & (kRows - 1));
+                const float ll = *reinterpret_cast<const float*>(row + (kb & (kRow - 4)));
+                const float ur = *reinterpret_cast<const float*>(row + ((kb + 4 * (kBand - 1)) & (kRow - 4)));
+                const float left[kPerLane] = {*reinterpret_cast<const float*>(row + 4 * tl), s1[0]};
+                const float4 x4 = *reinterpret_cast<const float4*>(&ws.x[s][q][kPerLane * t]);
+                const float xd[kPerLane] = {x4.x, x4.z}, xu[kPerLane] = {x4.y, x4.w};
+                if (q == 0) {
+                    const float mx = max_nan(s1[0], s1[1]);
+                    if (below | (mx != mx)) ws.flag = 1;
+                    below = false;
+                }
+                if (q == 1) {
+                    fl = ws.flag;
+                    head = *(volatile int32_t*)&ws.head[(j + 1) & (kHeadRing - 1)];
+                }
+                if (q == 2) {
+                    if (fl) return true;
+                    if (pend) release(s == 0 ? kGridRing - 1 : s - 1);  // chunk j - 1 stands
+                }
+                const bool right = ll < ur;  // both ends are finite
+                const uint32_t vr = vs - kOne;
+#pragma unroll
+                for (int i = 0; i < kPerLane; ++i) {
+                    const float d = __fadd_rn(lp[i], xd[i]), u = __fadd_rn(s1[i], xu[i]), l = __fadd_rn(left[i], xl);
+                    const float best = max3_nan(d, u, l);
+                    // the slot's in-band test under either placement, chosen last
+                    const float b_stay = vs + (uint32_t)i * kOne < kIn ? best : -INFINITY;
+                    const float b_right = vr + (uint32_t)i * kOne < kIn ? best : -INFINITY;
+                    if (kLow) below |= (xu[i] < g_lim) & (best != l);  // it must not win
+                    lp[i] = left[i];
+                    s1[i] = right ? b_right : b_stay;
+                }
+                *reinterpret_cast<float2*>(sc + rw + q * kRow + 8 * t) = make_float2(s1[0], s1[1]);
+                vs = right ? vr : vs;
+                kb += right ? 4 : 0;
+                if (t == 0) ws.kb[((rw / kRow) & (kScoreRing - 1)) + q] = kb;
+            }
+            pend = true;
+            kb_pend = kb_cur;
+            ++j;
+            s = s + 1 == kGridRing ? 0 : s + 1;
+            rw = (rw + kWideChunk * kRow) & (kRows - 1);
+            if (kLow && below) ws.flag = 2;  // (for the check when the run ends here)
+            // chunk j, usually made by now; both warps leave on another grid
+            for (int i = 0; head >> 5 != j + 1 && i < kReadyPolls; ++i)
+                head = *(volatile int32_t*)&ws.head[j & (kHeadRing - 1)];
+            named_bar_sync(kBarChain, kTeam);
+            if (head != chunk_head(j, g_mode)) {
+                k0 = kb >> 2;
+                return false;
+            }
+        }
+    };
+    // chunk j's header, once it is made
+    auto header = [&](int j) {
+        int h = *(volatile int32_t*)&ws.head[j & (kHeadRing - 1)];
+        for (int i = 0; h >> 5 != j + 1 && i < kReadyPolls; ++i) h = *(volatile int32_t*)&ws.head[j & (kHeadRing - 1)];
+        return h;
+    };
+    restore(j0, 4 * k_start);
+    int j = j0, s = 0;
+    while (true) {
+        // chunk j's header; also the barrier after band 4j-1
+        const int h = header(j);
+        const bool late = h >> 5 != j + 1;
+        if (late && t == 0) atomicAdd(&a.counters[2], 1ull);  // the run reports a timeout
+        __threadfence_block();
+        const int m = named_bar_any(kBarChain, kTeam, late) ? 0 : h & 31;
+        if (m == 0 || pen > 32) break;
+        if (m != g_mode) {
+            bool ok;
+            g_mode = m;
+            xl = grid_step(cc.skip_h, cc.skip_l, m, ok).o0;
+            g_lim = -(pow2f(m - 1) - 128.0f) * kGridLimLo;
+        }
+        // the start: the scores finite in the band and within the grid's range
+        const float top = -pow2f(m), bot = -pow2f(m + 4);
+        bool bad = !(max_nan(max3_nan(s1[0], s1[1], lp[0]), lp[1]) < top);
+#pragma unroll
+        for (int i = 0; i < kPerLane; ++i)
+            bad |= (((uint32_t)(kPerLane * t + i - k0) << 25 < kIn) & !(s1[i] >= bot)) | ((lp[i] < bot) & (lp[i] > -INFINITY));
+        if (named_bar_any(kBarChain, kTeam, bad)) {
+            redo(j, 4 * k0);
+            release(s);
+            ++j;
+            s = s + 1 == kGridRing ? 0 : s + 1;
+            continue;
+        }
+        const int j1 = j;
+        const bool failed = m < kGridWide ? run(j, s, std::true_type{}) : run(j, s, std::false_type{});
+        pen = max(pen - (j - j1), 0);
+        if (pend) {
+            // chunk j - 1 awaits its check (or has failed it)
+            const float mx = max_nan(s1[0], s1[1]);
+            const bool again = named_bar_any(kBarChain, kTeam, failed | (mx != mx) | (ws.flag != 0));
+            if (t == 0) ws.flag = 0;  // every thread has read it
+            if (again) redo(j - 1, kb_pend);
+            release(s == 0 ? kGridRing - 1 : s - 1);
+        }
+    }
+    // Every chunk before j is released; each E group ends up waiting for one of chunks j ..
+    // j + 4, and once chunk j + g is made no group waits for an older chunk of its slot.
+    if (t == 0) {
+        ws.exit = j;
+        ws.failing = pen > 32 ? 1 : 0;
+    }
+    for (int g = 0; g < kGridGroups; ++g) {
+        header(j + g);
+        __syncwarp();
+        release(s + g >= kGridRing ? s + g - kGridRing : s + g);
+    }
+    if (slow) atomicAdd(&a.counters[0], slow);
+}
+
+// One read's fill.  `grids`: the read's k-mers allow grids (grid_kmer_ok).
+template <bool kScores>
+__device__ void fill_chain(const CoreArgs& a, const ReadDesc& r, WideSmem& ws, int tid, bool grids) {
+    const int lane = tid & 31;
+    WideRead w{a, r, ws, make_consts(r, a.g), r.n_events, r.n_kmers, r.n_bands, (r.n_bands + kWideChunk - 1) / kWideChunk,
+               a.trace + r.trace_off * kSlots, a.band_k0 + r.band_off, kScores ? a.scores + r.band_off * kSlots : nullptr};
+    const uint32_t modes = grids ? grid_modes(w.cc) : 0u;
+    // band 0: the start cell (slot 127) = 0; band 1: the trim cell; both at k0 = -51
+    if (tid < kSlots) {
+        ws.sc[0][tid] = tid == 127 ? 0.0f : -INFINITY;
+        ws.sc[1][tid] = tid == 127 ? a.g.trim_f : -INFINITY;
+        if (kScores) {
+            w.scores[tid] = ws.sc[0][tid];
+            w.scores[kSlots + tid] = ws.sc[1][tid];
+        }
+    }
+    if (tid == 0) ws.kb[0] = ws.kb[1] = ws.kb[kScoreRing - 1] = 4 * (-1 - kBand / 2);
+    __syncthreads();
+    int j = 0, seg = kFirstExact, retry = kNextExact;
+    while (true) {
+        const int j1 = min(j + seg, w.n_chunks);
+        chain_exact<kScores>(w, tid, j, j1);
+        j = j1;
+        if (tid < kHeadRing) ws.head[tid] = 0;
+        if (tid == 0) {
+            ws.flag = 0;
+            ws.exit = INT32_MAX;
+        }
+        __syncthreads();
+        if (j >= w.n_chunks) break;
+        // the grid engine, if its chunks can begin here and there is room for a run
+        const int b0 = kWideChunk * j, kp = ws.kb[(b0 - 1) & (kScoreRing - 1)] >> 2;
+        const int first = grid_of(ws.sc[(b0 - 1) & (kScoreRing - 1)], lane, modes);
+        const bool room = chunk_mode(1, kp + 40, b0 + 2 * 40, w.n_events, w.n_kmers);
+        seg = kp < 0 || kp + 40 <= w.n_kmers - kSlots ? retry : w.n_chunks;  // near the end: to the end
+        if (first && room && chunk_mode(first, kp, b0, w.n_events, w.n_kmers)) {
+            chain_grid<kScores>(w, tid, j, first, modes);
+            __syncthreads();
+            j = ws.exit;
+            if (ws.failing) retry = min(2 * retry, 1 << 20);
+            const int k_end = ws.kb[(kWideChunk * j - 1) & (kScoreRing - 1)] >> 2;
+            seg = k_end + 64 <= w.n_kmers - kSlots ? retry : w.n_chunks;
+            __syncthreads();  // everyone has read the exit
+        }
+    }
 }
 
 // ---------------------------------------------------------------- wide shape on a cluster pair
@@ -2075,31 +2404,25 @@ __global__ void __launch_bounds__(32) abea_post_kernel(CoreArgs ca, PostArgs a) 
 constexpr int kBatchedWarps = kWideThreads / 32;
 
 struct BatchedSmem {
-    WideSmem wide;                     // phase 1: the block's wide read
+    union {
+        WideSmem wide;                 // phase 1: the block's wide read
+        PostSmem post[kBatchedWarps];  // phase 2: every warp's post staging
+    };
     Rings warp_rings[kBatchedWarps];   // phase 2: one per warp
-    // every warp's post staging; in phase 1b each half's medium read uses its eight
-    // warps' entries (post[8 * half] on), which no other warp touches meanwhile
-    PostSmem post[kBatchedWarps];
     int32_t pick;                      // the block's wide read, or -1
     int32_t wide_slot;                 // the block's first pick: its traceback scratch slot
-    int32_t free_rank;                 // rank among the blocks with neither a wide nor medium reads, or -1
-    int32_t mid_block;                 // 1: a block of the medium reads
-    int32_t mid_pick[2];               // each half's medium read
+    int32_t free_rank;                 // rank among the blocks without a wide read, or -1
 };
 static_assert(offsetof(BatchedSmem, warp_rings) % 16 == 0 && offsetof(BatchedSmem, post) % 16 == 0 &&
                   sizeof(Rings) % 16 == 0 && sizeof(PostSmem) % 16 == 0,
               "cp.async destinations must be 16-byte aligned");
 static_assert(sizeof(BatchedSmem) <= 227 * 1024, "batched kernel shared memory exceeds the per-block limit");
-static_assert(offsetof(WideSmem, ems) % 16 == 0 && offsetof(WideSmem, emm) % 8 == 0,
-              "vector accesses to the emission ring must be aligned");
+static_assert(offsetof(WideSmem, ems) % 16 == 0 && offsetof(WideSmem, emm) % 8 == 0 && offsetof(WideSmem, x) % 16 == 0 &&
+                  offsetof(WideSmem, sc) % 16 == 0,
+              "vector accesses to the emission and score rings must be aligned");
 static_assert(sizeof(WideSmem) >= kPostRingDeep * kPostChunkBands * kSlots && alignof(WideSmem) >= 16,
               "the wide read's traceback ring lives in the wide fill's shared memory");
 static_assert(sizeof(WidePostSmem) <= sizeof(WideSmem), "the wide read's traceback state fits the fill's memory");
-static_assert(sizeof(MidSmem) <= (kBatchedWarps / 2) * sizeof(PostSmem) &&
-                  sizeof(MidSmem) >= kPostRingDeep * kPostChunkBands * kSlots,
-              "a medium read's fill, and then its traceback ring, fit its half's post staging");
-
-
 
 template <bool kScores>
 __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(CoreArgs a, PostArgs p, PreArgs pa) {
@@ -2109,26 +2432,22 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(CoreArgs 
     // phase 1: the wide reads, longest first
     // Each block's first pick decides its role: the first blocks to arrive take a
     // wide read each (and then pull the wide reads past the first wave, one after
-    // another); the next ones the medium reads (two at a time per block, enough
-    // blocks for each half to start one); the others the first wave of the
-    // warp-shape reads.
-    const int n_midb = min((a.n_mid + 1) / 2, max((int)gridDim.x - a.n_wide, 0));
+    // another); the others the first wave of the warp-shape reads.
     if (t == 0) {
         const int q = atomicAdd(&a.queue[0], 1);
         sm.pick = q < a.n_wide ? a.order[q] : -1;
         sm.wide_slot = q;  // the block's traceback scratch slot: wide reads go longest first, so only
                            // the first blocks' reads (and the reads they pull later) need one
-        sm.mid_block = (q >= a.n_wide && q < a.n_wide + n_midb) ? 1 : 0;
-        sm.free_rank = q < a.n_wide + n_midb ? -1 : q - a.n_wide - n_midb;
+        sm.free_rank = q < a.n_wide ? -1 : q - a.n_wide;
     }
     __syncthreads();
     int wide_read = sm.pick;
     const int free_rank = sm.free_rank, wide_slot = sm.wide_slot;
     while (wide_read >= 0) {
         const ReadDesc& r = a.reads[wide_read];
-        pre_read(pa, wide_read, t, kWideThreads);
-        __syncthreads();  // the read's parameters are in memory for the whole block
-        if (!r.skip) fill_chain<kScores, 2, kWideRing>(a, r, sm.wide, t, 1);
+        const bool odd = pre_read(pa, wide_read, t, kWideThreads);
+        const bool grids = !__syncthreads_or(odd);  // the read's parameters are in memory for the whole block
+        if (!r.skip) fill_chain<kScores>(a, r, sm.wide, t, grids);
         __syncthreads();
         __threadfence_block();
         // the whole block walks the wide read's traceback (the fill's shared memory is free)
@@ -2142,35 +2461,12 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(CoreArgs 
         __syncthreads();
         wide_read = sm.pick;
     }
-    // phase 1b: the medium reads, each half of a medium block (eight warps) pulling
-    // one at a time: pre, fill, and the traceback by the half's first warp; the
-    // blocks done with their wide reads join in
-    if (a.n_mid > 0 && free_rank < 0) {
-        const int half = warp >> 3, ht = t & (kMidThreads - 1), hw = ht >> 5;
-        MidSmem& ms = *reinterpret_cast<MidSmem*>(&sm.post[half * (kBatchedWarps / 2)]);
-        const int bar0 = 1 + half * kMidBars, bar_half = bar0 + kMidBars - 1;
-        while (true) {
-            if (ht == 0) sm.mid_pick[half] = atomicAdd(&a.queue[3], 1);
-            named_bar_sync(bar_half, kMidThreads);  // the pick is visible; the last read's traceback is done
-            const int q = sm.mid_pick[half];
-            if (q >= a.n_mid) break;  // the whole half leaves together
-            const int ri = a.order[a.n_wide + q];
-            const ReadDesc& r = a.reads[ri];
-            pre_read(pa, ri, ht, kMidThreads);
-            named_bar_sync(bar_half, kMidThreads);  // the read's parameters are in memory; the pick was read
-            if (!r.skip) fill_chain<kScores, 1, kMidRing>(a, r, ms, ht, bar0);
-            named_bar_sync(bar_half, kMidThreads);  // the fill is done: its memory becomes the traceback ring
-            __threadfence_block();
-            if (hw == 0) post_read_warp<kPostRingDeep>(a, p, ri, reinterpret_cast<uint8_t*>(&ms), sm.warp_rings[warp], lane);
-        }
-    }
-    // phase 2: the first wave is static, the blocks with neither a wide nor medium
-    // reads taking the longest remaining reads round-robin (warp w of free block f:
+    // phase 2: the first wave is static, the blocks without a wide read taking the
+    // longest remaining reads round-robin (warp w of free block f:
     // read f + F*w), so that the long ones spread over the SMs; then every warp
     // pulls the rest longest-first.
-    const int n_pre = a.n_wide + a.n_mid;
-    const int n_rest = a.n_reads - n_pre;
-    const int n_free = max((int)gridDim.x - a.n_wide - n_midb, 0);
+    const int n_rest = a.n_reads - a.n_wide;
+    const int n_free = max((int)gridDim.x - a.n_wide, 0);
     const int wave = min(n_rest, n_free * kBatchedWarps);
     for (int pass = 0;; ++pass) {
         int q;
@@ -2184,7 +2480,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(CoreArgs 
             q = __shfl_sync(kFull, q, 0);
             if (q >= n_rest) break;
         }
-        const int ri = a.order[n_pre + q];
+        const int ri = a.order[a.n_wide + q];
         const ReadDesc& r = a.reads[ri];
         pre_read(pa, ri, lane, 32);
         __syncwarp();  // the read's parameters are in memory for the warp

@@ -32,6 +32,7 @@ struct PreArgs {
     float* km_k1;
     float* last_col;
     const InMirror* inm;  // nullptr, or a device copy of the input mirror
+    float4* km4;          // the four k-mer parameters side by side, for the wide shape (nullptr: not wanted)
 };
 
 struct CoreArgs {
@@ -56,7 +57,7 @@ struct CoreArgs {
     int32_t* spec;                 // traceback cell maps: kSpecRound * kSpecBands int32 per slot
     int32_t n_spec;                // slots (queue[2] hands them out)
     long long spin_limit;          // polls before a device-side wait gives up (counters[2] counts those)
-    int32_t n_mid;                 // the reads after the wide ones that run on the medium shape (batched form)
+    const float4* km4;             // {km_gm, km_sd, km_rsd, km_k1} of each k-mer position (wide shape)
 };
 
 // Host memory the kernels write each read's results into as the read finishes

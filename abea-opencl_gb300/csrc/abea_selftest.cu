@@ -6,6 +6,7 @@
 //   div_rn(n, sd, RN(1/sd))            with __fdiv_rn(n, sd)
 //   exact_sum(a, bh, bl, c)            with RN32(RN64(RN64(a + B) + c))
 //   exact_skip(a, bh, bl)              with RN32(RN64(a + B))
+//   a + grid_pair(...)                 with RN32(RN64(RN64(a + B) + em)), em by IEEE division
 // and counts the cases where the fast routine claims success but differs
 // (must be zero) and the cases where it declines (the kernels then fall back).
 // Adversarial sums are built around float rounding midpoints, where double
@@ -107,6 +108,46 @@ __global__ void selftest_kernel(uint64_t seed, int iters, unsigned long long* co
             const float v2 = exact_from_split(-INFINITY, sp, __fadd_rn(fabsf(c), fabsf(bh)), o2);
             exact_from_split(-INFINITY, sp, __int_as_float(0x7fc00000), o3);
             if (!o1 || v1 != -INFINITY || !o2 || v2 != -INFINITY || o3) ++c2;
+        }
+        // ---- candidates on a grid: a score of the grid's range, an emission (some
+        // far below the range), and transitions, random or aimed so that T = B + em
+        // lies next to an end of its cell
+        {
+            const int m = kGridMin + (int)(it % (kGridMax - kGridMin + 1));
+            const float a = -pow2f(m) * (1.0f + 15.0f * unit(s) * ((it & 16) ? 1.0f : 0.01f));
+            const float gm = 60.0f + 70.0f * unit(s), lsd = logf(sd), k1 = __fsub_rn(kLogInvSqrt2Pi, lsd);
+            const float x = gm + sd * ((it & 3) ? 8.0f : 120.0f) * (unit(s) - 0.5f);
+            const float em = emission_ieee(x, gm, sd, k1);
+            double bb[2];
+            for (int i = 0; i < 2; ++i) {
+                bb[i] = -(0.01 + 5.0 * (double)unit(s)) - (double)unit(s) * 1e-9;
+                if (it & 32) {
+                    const double g2 = (double)pow2f(m - 24);
+                    const double off = ((double)unit(s) - 0.5) * g2 * exp2(-30.0 * (double)unit(s));
+                    bb[i] = g2 * floor(((double)em + bb[i]) / g2) - (double)em + off;
+                }
+            }
+            CellConsts cc{};
+            cc.step_h = (float)bb[0];
+            cc.step_l = (float)(bb[0] - (double)cc.step_h);
+            cc.stay_h = (float)bb[1];
+            cc.stay_l = (float)(bb[1] - (double)cc.stay_h);
+            bool okd, oku;
+            grid_step(cc.step_h, cc.step_l, m, okd);
+            grid_step(cc.stay_h, cc.stay_l, m, oku);
+            const Grid G = make_grid(cc, m);
+            if (okd && oku && grid_kmer_ok(sd, k1, grid_k1_max(cc.step_h, cc.stay_h))) {
+                const float rsd = __frcp_rn(sd);
+                const float2 g = m < kGridWide ? grid_pair<true>(x, gm, sd, rsd, k1, G)
+                                               : grid_pair<false>(x, gm, sd, rsd, k1, G);
+                const bool below = m < kGridWide && g.y < G.lim * kGridLimLo;  // only an upper bound
+                for (int i = 0; i < 2; ++i) {
+                    const float v = __fadd_rn(a, i ? g.y : g.x);
+                    const float w = __double2float_rn(__dadd_rn(__dadd_rn((double)a, bb[i]), (double)em));
+                    // NaN: declined (most aimed cases are; not counted)
+                    if (below ? v < w : v < -pow2f(m) && __float_as_int(v) != __float_as_int(w)) ++c2;
+                }
+            }
         }
     }
     atomicAdd(&counters[0], c0);

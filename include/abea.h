@@ -113,7 +113,7 @@ typedef enum {
  *            scores too only with ABEA_OPT_STORE_SCORES.
  *  BATCHED — one persistent kernel (pre, fill and traceback fused) of one
  *            512-thread block per SM: the longest reads on the wide shape
- *            (twelve warps: four run the band-to-band chain, eight compute the
+ *            (a few warps run the band-to-band chain, the others compute the
  *            emissions ahead of it; the traceback is walked by the whole block),
  *            which the blocks pull longest first, one after another (every read,
  *            when the batch's longest read bounds it or it has few reads per SM);
@@ -138,9 +138,9 @@ typedef enum {
     ABEA_OPT_WIDE_CLUSTER = 7,  /* BATCHED: 1 = the longest reads run on a cluster of two blocks (the
                                    second SM computes the emissions ahead into the first one's shared
                                    memory); 0 = one block per wide read */
-    ABEA_OPT_MEDIUM_READ_BANDS = 8 /* BATCHED: reads with at least this many bands that do not take the
-                                   wide shape run on the medium shape (eight warps per read, two reads
-                                   per block); 0 = autotuned (none when not tuned) */
+    ABEA_OPT_MEDIUM_READ_BANDS = 8 /* BATCHED: a second threshold: reads with at least this many bands
+                                   run on the wide shape too (it once chose a medium shape of two
+                                   reads per block); 0 = that of a loaded cache file, else none */
 } abea_option_t;
 
 typedef struct abea_ctx abea_ctx_t;

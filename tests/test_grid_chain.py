@@ -1,0 +1,80 @@
+"""The wide shape's two engines against the oracle, with every score, backpointer and
+band origin: reads that end around the points where the exact chain hands over to the
+grid chain and back, emissions that no grid serves or that lie far below its range, and
+events that are not finite.  All comparisons are exact: the results are the reference's
+floats, whichever engine computes a band."""
+import numpy as np
+import pytest
+
+from conftest import abea
+
+pytestmark = pytest.mark.gpu
+
+
+def make(rng, length, stdv=(1.0, 3.0), var=1.2, mean_events=1.8, skip=0.01):
+    from abea_gb300 import synth
+    model = synth.make_model(rng)
+    model["level_stdv"] = rng.uniform(*stdv, len(model)).astype(np.float32)
+    model["level_log_stdv"] = np.log(model["level_stdv"].astype(np.float64)).astype(np.float32)
+    seq, ev = synth.make_read(rng, model, length, 1.02, 2.0, var, skip_p=skip, mean_events=mean_events)
+    return model, seq.tobytes(), ev
+
+
+def batch_of(model, reads):
+    sc = np.zeros(len(reads), dtype=abea.types.SCALINGS_DTYPE)
+    sc["scale"], sc["shift"], sc["var"], sc["log_var"] = 1.02, 2.0, 1.2, np.log(1.2)
+    return abea.from_reads([r[0] for r in reads], [r[1] for r in reads], sc, model)
+
+
+def check(oracle_mod, batch):
+    ctx = abea.Context(0, abea.MODE_BATCHED, store_scores=True)
+    ctx.set_option(abea.OPT_LONG_READ_BANDS, 1)  # every read on the wide shape
+    dev = ctx.upload(batch)
+    dev.run()
+    pairs, counts = dev.results()
+    opairs, ocounts, _ = oracle_mod.align_batch(batch, threads=8)
+    assert np.array_equal(counts, ocounts)
+    for got, exp in zip(abea.split_pairs(batch, pairs, counts), abea.split_pairs(batch, opairs, ocounts)):
+        assert np.array_equal(got, exp)
+    for i in range(batch.n_reads):
+        b, t, bll = dev.read_bands(i, scores=True)
+        _, _, info = oracle_mod.align(batch.sequence(i), batch.read_events(i), batch.model, batch.scalings[i],
+                                      want_bands=True)
+        assert np.array_equal(b.view(np.uint32), info["bands"].view(np.uint32)), i
+        assert np.array_equal(t, info["trace"]), i
+        assert np.array_equal(bll, info["bll"]), i
+
+
+@pytest.mark.parametrize("mean_events", [1.05, 1.8, 4.0])
+def test_hand_over_between_the_engines(oracle_mod, mean_events):
+    """Reads of 6 bases up to ones with long grid runs, around the 800 bands after which
+    the grid chain is first tried, at three event rates (few moves right, and many)."""
+    rng = np.random.default_rng(11)
+    model, _, _ = make(rng, 50)
+    from abea_gb300 import synth
+    reads = []
+    for length in (6, 7, 60, 133, 160, 290, 296, 302, 330, 420, 550, 700, 1201, 2503, 4999):
+        seq, ev = synth.make_read(rng, model, length, 1.02, 2.0, 1.2, skip_p=0.01, mean_events=mean_events)
+        if len(ev):
+            reads.append((seq.tobytes(), ev))
+    check(oracle_mod, batch_of(model, reads))
+
+
+@pytest.mark.parametrize("stdv", [(0.05, 0.4), (0.3, 1.0), (0.8, 1.1), (8.0, 30.0)])
+def test_emissions_a_grid_does_not_serve(oracle_mod, stdv):
+    """Deviations so small that emissions are positive (no grid) or lie thousands below
+    (their cells must lose or be done again), and so large that scores fall slowly."""
+    rng = np.random.default_rng(12)
+    model, seq, ev = make(rng, 1800, stdv=stdv)
+    check(oracle_mod, batch_of(model, [(seq, ev)]))
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, 1e30, -1e5, 4000.0])
+def test_outlier_events(oracle_mod, value):
+    """Single events far out or infinite, in and around the grid chain's bands."""
+    rng = np.random.default_rng(13)
+    model, seq, ev = make(rng, 2400)
+    ev = ev.copy()
+    for at in (700, 1500, 1501, 2600, len(ev) - 40):
+        ev["mean"][at] = value
+    check(oracle_mod, batch_of(model, [(seq, ev)]))
