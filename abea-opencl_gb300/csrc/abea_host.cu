@@ -427,7 +427,7 @@ static abea_status_t plan(abea_batch* b, const HostInputs& in, int var_aware, in
     b->n_ck = n_ck;
     int32_t n_spec = 0;
     for (const ReadDesc& r : b->reads)
-        if (!r.skip && !r.ck && r.n_bands >= kSpecMinBands) ++n_spec;
+        if (!r.skip && r.n_bands >= kSpecMinBands) ++n_spec;
     // one scratch slot per block that starts on a wide read (a block walks one wide read
     // at a time and keeps its slot; the first picks take the longest reads, so at most
     // one slot per qualifying read)
@@ -578,103 +578,95 @@ static int64_t d2h_bytes(const abea_batch* b) {
 }
 
 // Heuristic wide-shape threshold.  First, the number n of wide reads (the longest
-// ones whose trace is kept, at most one per block, the other blocks taking the
-// warp-shape reads from the start) that minimises an estimate of the batch's
+// eligible ones: every read, with the cluster pair those whose trace is kept; at most
+// one per block, the other blocks taking the warp-shape reads from the start) that
+// minimises an estimate of the batch's
 // makespan, in cycles:
-//   the longest wide read on the wide shape, kWideCyc per band;
-//   the longest warp-shape read: kWarpFloorCyc per band, or kWarpSmCyc per band
-//     times the warps sharing its SM in the first wave (the blocks without a
-//     wide read share the other reads round-robin, at most 16 warps each);
-//   the warp-shape work spread over those blocks, kWarpSmCyc per band per SM.
+//   the longest wide read (wide_cycles);
+//   the longest warp-shape read, kWarpBase + kWarpMore * w cycles per band with w
+//     warps sharing its SM in the first wave (the blocks without a wide read share
+//     the other reads round-robin, at most 16 warps each);
+//   the warp-shape work spread over those blocks' warps at that rate.
+// A checkpointed read on the warp shape counts its bands twice: its traceback
+// recomputes them on the same warp.
 // Then every read on the wide shape, the blocks pulling them longest first: the
-// longest read at kWideCyc per band, or all the bands over the blocks at
-// kWideSmCyc per band per block.  That wins when it is within 2% of the first
-// (it cannot be shorter than the longest read, which bounds both) and either the
-// longest read bounds it or there are at most 8 reads per block (with more, the
-// warp shape's 16 warps per SM hide each other's latency better than the first
-// estimate assumes: the serving stream's batches of ~4,000 reads of median 8 kb
-// took 1.23 s every read wide against 0.99 s split), except with checkpointed
-// reads, which run on the warp shape and would start last.
-// Calibrated on GB300 by sweeping the number of wide reads: the f5c batch and the
-// 1,024-read batch of 1-10 kb reads are fastest with every read wide (8.46 and
-// 18.5 ms, against 8.49-9.10 and 20.8 at the best one-per-block split); the
-// 4,096-read adjoint batch with none (35.5 ms; 68.5 with every read wide: at 27
-// reads per SM the warp shape's 16 warps issue more per SM).  kWarpFloorCyc
-// includes the warp-shape read's traceback, kWideSmCyc the wide reads' tracebacks
-// and the blocks' tail.  Ties go to fewer wide reads; the threshold is the band
-// count of the n-th wide read (every read: 1; none: INT64_MAX).
-constexpr double kWideCyc = 400, kWarpFloorCyc = 1800, kWarpSmCyc = 250, kWideSmCyc = 380;
-static int64_t heuristic_threshold(const abea_batch* b, int blocks) {
+// longest read, or all of them over the blocks.  That wins when it is within 2% of
+// the first and either the longest read bounds it or there are at most 8 reads per
+// block, unless there are reads that may not be wide: those would start last.
+// Calibrated on GB300 (ms, every read wide / none): 1,024 reads of 1-10 kb 12.7 / 19,
+// 608 reads of 3 kb 4.91 / 4.77, 1,216 of 3 kb 9.52 / 6.68, 2,432 of 3 kb 18.9 / 8.5
+// (sixteen warps on an SM take 131 cycles per band together, one wide read 200-290),
+// 2,432 of 600 b 7.85 / 3.06, 152 of 3 kb 1.29 / 4.53.  Ties go to fewer wide reads;
+// the threshold is the band count of the n-th wide read (every read: 1; none:
+// INT64_MAX).
+constexpr double kWarpBase = 950, kWarpMore = 68;
+// A read on the wide shape, pre stage and traceback included: its bands on the grid
+// engine, the exact engine's share (its start and tail), and what each read costs.
+// A checkpointed one also recomputes its bands, 16 warps at a time.
+static double wide_cycles(const ReadDesc& r) {
+    const double nb = (double)r.n_bands;
+    return (r.ck ? 370 : 220) * nb + 275 * std::min(nb, 1240.0) + 165e3;
+}
+static double warp_bands(const ReadDesc& r) { return (r.ck ? 2.0 : 1.0) * (double)r.n_bands; }
+static int64_t heuristic_threshold(const abea_batch* b, int blocks, bool ck_wide) {
     const size_t n = b->order.size();
-    std::vector<int64_t> wide_ok;  // band counts of the reads that may be wide, longest first
-    double rest_bands = 0;
+    std::vector<const ReadDesc*> wide_ok;  // the reads that may be wide, longest first
+    double rest_bands = 0, all_wide = 0;
     for (int32_t i : b->order) {
         const ReadDesc& r = b->reads[(size_t)i];
-        rest_bands += (double)r.n_bands;
-        if (!r.ck) wide_ok.push_back(r.n_bands);
+        rest_bands += warp_bands(r);
+        all_wide += wide_cycles(r);
+        if (ck_wide || !r.ck) wide_ok.push_back(&r);
     }
-    const double all_bands = rest_bands;
-    const bool any_ck = wide_ok.size() < n;
+    const bool all_ok = wide_ok.size() == n;
     const int max_wide = (int)std::min<size_t>(wide_ok.size(), (size_t)std::max(0, blocks - 1));
     double best_t = 0;
     int best_n = 0;
     int taken = 0;
+    size_t j = 0;  // the longest warp-shape read: the first of the order that is not one of the wide ones
+    int passed = 0;
     for (int k = 0; k <= max_wide; ++k) {
         if (k > 0) {  // the k-th wide read leaves the warp-shape set
-            rest_bands -= (double)wide_ok[(size_t)k - 1];
+            rest_bands -= warp_bands(*wide_ok[(size_t)k - 1]);
             ++taken;
         }
-        // the longest warp-shape read: skip the wide ones (the longest trace-keeping reads)
-        int skip = taken;
-        size_t j = 0;
-        int64_t longest_warp = 0;
-        for (j = 0; j < n; ++j) {
-            const ReadDesc& r = b->reads[(size_t)b->order[j]];
-            if (!r.ck && skip > 0) {
-                --skip;
-                continue;
-            }
-            longest_warp = r.n_bands;
-            break;
-        }
+        for (; j < n && (ck_wide || !b->reads[(size_t)b->order[j]].ck) && passed < taken; ++j) ++passed;
+        const double longest_warp = j < n ? warp_bands(b->reads[(size_t)b->order[j]]) : 0.0;
         const int free_blocks = std::max(1, blocks - k);
         const double warps = std::min(16.0, std::max(1.0, (double)(n - (size_t)k) / free_blocks));
-        const double t_wide = k > 0 ? (double)wide_ok[0] * kWideCyc : 0.0;
-        const double t_warp = (double)longest_warp * std::max(kWarpFloorCyc, kWarpSmCyc * warps);
-        const double t_work = rest_bands * kWarpSmCyc / free_blocks;
-        const double t = std::max(t_wide, std::max(t_warp, t_work));
+        const double per_band = kWarpBase + kWarpMore * warps;
+        const double t_wide = k > 0 ? wide_cycles(*wide_ok[0]) : 0.0;
+        const double t = std::max(t_wide, std::max(longest_warp, rest_bands / (warps * free_blocks)) * per_band);
         if (k == 0 || t < best_t * 0.98) {  // a wide read must buy at least 2%
             best_t = t;
             best_n = k;
         }
     }
-    if (!any_ck && !wide_ok.empty()) {
-        const double t_lat = (double)wide_ok[0] * kWideCyc, t_thr = all_bands * kWideSmCyc / std::max(blocks, 1);
-        // at more than 8 reads per block the warp shape's warps hide each other's
-        // latency and the split's estimate above is too long: every read wide only
-        // where the longest read bounds it anyway, or with few reads per block
+    if (all_ok && !wide_ok.empty()) {
+        const double t_lat = wide_cycles(*wide_ok[0]), t_thr = all_wide / std::max(blocks, 1);
         const bool few = (double)n <= 8.0 * blocks;
         if ((t_thr <= t_lat || few) && std::max(t_lat, t_thr) <= best_t * 1.02) return 1;
     }
-    return best_n > 0 ? wide_ok[(size_t)best_n - 1] : INT64_MAX;
+    return best_n > 0 ? wide_ok[(size_t)best_n - 1]->n_bands : INT64_MAX;
 }
 
-// Reads of the batched form that run on the wide shape: those over the wide
-// threshold (the option, the autotuned value, or the heuristic above) or over the
-// medium one, when there is one (its own shape, two reads per block, is no longer
-// faster than one wide read after another); never a checkpointed read.  The blocks
-// take them longest first, one at a time, as many each as the queue holds; with the
-// cluster pair at most one per cluster, and no medium threshold.  Fills
-// b->dev_order with the wide reads, then the rest, each longest first, and sets n_wide.
+// Reads of the batched form that run on the wide shape: those of at least the wide
+// threshold's bands (the option, the autotuned value, or the heuristic above) or of the
+// second threshold's (ABEA_OPT_MEDIUM_READ_BANDS), when it is set.  The blocks take
+// them longest first, one at a time, as many each as the queue holds; with the cluster
+// pair at most one per cluster, never a checkpointed read, and no second threshold.
+// Fills b->dev_order with the wide reads, then the rest, each longest first, and sets
+// n_wide.  Checkpointed reads are a batch's longest: the blocks that take one have the
+// first traceback slots.
 static void choose_shape_reads(abea_batch* b, int sm_count, int64_t threshold, int64_t mid_threshold, bool scores,
                                bool cluster) {
     const int blocks = cluster ? sm_count / 2 : batched_blocks_per_sm(scores) * sm_count;
-    if (threshold <= 0) threshold = heuristic_threshold(b, blocks);
+    if (threshold <= 0) threshold = heuristic_threshold(b, blocks, !cluster);
     if (mid_threshold > 0 && !cluster) threshold = std::min(threshold, mid_threshold);
     std::vector<int32_t> wide, rest;
     for (int32_t i : b->order) {
         const ReadDesc& r = b->reads[(size_t)i];
-        if ((!cluster || (int)wide.size() < blocks) && !r.ck && r.n_bands >= threshold)
+        if ((!cluster || ((int)wide.size() < blocks && !r.ck)) && r.n_bands >= threshold)
             wide.push_back(i);
         else
             rest.push_back(i);
@@ -833,7 +825,7 @@ extern "C" abea_status_t abea_autotune(abea_ctx_t* c, abea_batch_t* b, int64_t* 
     const int blocks = batched_blocks_per_sm(b->scores_kept) * c->sm_count;
     int64_t longest = 0;
     for (const ReadDesc& r : b->reads) longest = std::max<int64_t>(longest, r.n_bands);
-    std::vector<int64_t> cands = {INT64_MAX, heuristic_threshold(b, blocks)};
+    std::vector<int64_t> cands = {INT64_MAX, heuristic_threshold(b, blocks, c->wide_cluster == 0)};
     if (c->wide_cluster == 0 && std::find(cands.begin(), cands.end(), (int64_t)1) == cands.end())
         cands.push_back(1);  // every read wide
     for (int num : {1, 2, 3, 4, 6, 8, 12, 16}) {  // the longest num/16 of the resident blocks
@@ -1730,8 +1722,7 @@ extern "C" abea_status_t abea_align_stream(abea_ctx_t* c, const abea_stream_conf
         const int64_t rb = read_device_bytes(read_len[i], n_events[i], c->trace_budget, scores);
         const int64_t nk = (int64_t)read_len[i] - ABEA_KMER_SIZE + 1;
         const int64_t nb = nk > 0 && n_events[i] > 0 ? n_events[i] + nk + 2 : 0;
-        const bool trace_kept = c->trace_budget <= 0 || round_up(nb, 4) * kSlots <= c->trace_budget;
-        const int64_t lg = nb >= kSpecMinBands && trace_kept ? 1 : 0;  // a traceback map slot
+        const int64_t lg = nb >= kSpecMinBands ? 1 : 0;  // a traceback map slot
         if (i > cut.back() && acc + rb + spec_bytes(n_long + lg) > budget) {
             cut.push_back(i);
             cut_bytes.push_back(acc + spec_bytes(n_long));
@@ -2045,7 +2036,7 @@ extern "C" const char* abea_internal_set_error(const char* msg) {
 // these band counts on `blocks` resident blocks (no device needed): for tests
 // and for callers who size batches.  INT64_MAX = no wide read; -1 = bad input.
 // The heuristic on band counts alone (host code, for tests); ck (optional) marks
-// the reads whose trace is not kept (checkpointed), which stay on the warp shape.
+// checkpointed reads, which stay on the warp shape (as with the cluster pair).
 extern "C" int64_t abea_internal_wide_threshold_ck(const int64_t* n_bands, const int32_t* ck, int32_t n_reads,
                                                    int32_t blocks) {
     if (n_reads < 0 || blocks < 1 || (n_reads > 0 && !n_bands)) return -1;
@@ -2062,7 +2053,7 @@ extern "C" int64_t abea_internal_wide_threshold_ck(const int64_t* n_bands, const
     std::stable_sort(b.order.begin(), b.order.end(), [&](int32_t x, int32_t y) {
         return b.reads[(size_t)x].n_bands > b.reads[(size_t)y].n_bands;
     });
-    return heuristic_threshold(&b, blocks);
+    return heuristic_threshold(&b, blocks, false);
 }
 
 extern "C" int64_t abea_internal_wide_threshold(const int64_t* n_bands, int32_t n_reads, int32_t blocks) {

@@ -190,6 +190,7 @@ struct alignas(16) Rings {
     float rsd[kSlots];
     float k1[kSlots];
     float ev[kEvRing];
+    float4 save[2][32];  // the warp shape's state before a chunk on a grid
 };
 
 struct RingState {
@@ -489,22 +490,171 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
             if (lane <= (b & 31) && in_bounds((b & ~31) + lane, r.n_bands, a.counters)) bk0[(b & ~31) + lane] = my_k0;
         }
     };
+    // Four bands at a time on a grid (abea_cell.cuh, "candidates on a grid") where the
+    // band lies inside the read and its scores are in a grid's range: the diagonal and up
+    // candidates are one add each, their parts made and proven here, band by band.  The
+    // same conditions and the same end-of-chunk check as the wide shape's grid engine; a
+    // chunk that fails it runs again in the exact loop below.  Not unrolled over the bands:
+    // the loop body stays small (up to sixteen warps on an SM, each at its own place).
+    //   grid: the grid in use until band grid_until; grid_from: the first band that may try.
+    const uint32_t modes = grid_modes(cc);
+    const float k1_max = grid_k1_max(cc.step_h, cc.stay_h);
+    Grid G{};
+    int grid = 0, g_made = 0, grid_until = 0, grid_from = sp.b_begin, pen = 0;
+    auto grid_now = [&]() {
+        bool hole = false;
+        float mx = -INFINITY, mn = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            hole |= (((4 * lane + j - k0) & 127) < kBand) & (S1[j] == -INFINITY);
+            mx = max_nan(max_nan(mx, S1[j]), LP[j]);
+            mn = fminf(fminf(mn, S1[j] > -INFINITY ? S1[j] : 0.0f), LP[j] > -INFINITY ? LP[j] : 0.0f);
+        }
+        const bool none = __any_sync(kFull, hole || mx != mx);
+        mx = warp_max(mx);
+        mn = warp_min(mn);
+        const int m = (__float_as_int(-mx) >> 23) - 127, mlo = (__float_as_int(-mn) >> 23) - 127;
+        return !none && m >= kGridMin && m <= kGridMax && mlo < m + 2 && ((modes >> (m & 31)) & 1u) ? m : 0;
+    };
+    // bands b .. b + 3; false (and the state as it was) when the check fails
+    auto grid_bands = [&](auto low) {
+        constexpr bool kLow = decltype(low)::value;
+        constexpr uint32_t kOne = 1u << 25, kIn = (uint32_t)kBand << 25;
+        const int k_was = k0, my_was = my_k0;
+        rg.save[0][lane] = make_float4(S1[0], S1[1], S1[2], S1[3]);
+        rg.save[1][lane] = make_float4(LP[0], LP[1], LP[2], LP[3]);
+        float4 km[4];  // {gm, sd, rsd, k1} of the lane's slots
+        {
+            const float4 gm4 = *reinterpret_cast<const float4*>(&rg.gm[4 * lane]);
+            const float4 sd4 = *reinterpret_cast<const float4*>(&rg.sd[4 * lane]);
+            const float4 rs4 = *reinterpret_cast<const float4*>(&rg.rsd[4 * lane]);
+            const float4 k14 = *reinterpret_cast<const float4*>(&rg.k1[4 * lane]);
+            km[0] = make_float4(gm4.x, sd4.x, rs4.x, k14.x);
+            km[1] = make_float4(gm4.y, sd4.y, rs4.y, k14.y);
+            km[2] = make_float4(gm4.z, sd4.z, rs4.z, k14.z);
+            km[3] = make_float4(gm4.w, sd4.w, rs4.w, k14.w);
+        }
+        int e[4];  // event of each slot in band b
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            km[j].x = grid_kmer_ok(km[j].y, km[j].w, k1_max) ? km[j].x : __int_as_float(0x7fc00000);
+            e[j] = b - 2 - (k0 + ((4 * lane + j - k0) & 127));
+        }
+        const float g_lim = G.lim * kGridLimLo;
+        uint32_t vs = (uint32_t)(4 * lane - k0) << 25, w[4] = {0u, 0u, 0u, 0u};
+        bool below = false;
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+            const int sl = k0 & 127, su = (k0 + kBand - 1) & 127;
+            const float ll = __shfl_sync(kFull, sel4(S1, sl & 3), sl >> 2);
+            const float ur = __shfl_sync(kFull, sel4(S1, su & 3), su >> 2);
+            const float left0 = __shfl_sync(kFull, S1[3], (lane + 31) & 31);
+            const float l4[4] = {left0, S1[0], S1[1], S1[2]};
+            float top[4], sk[4], up[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 x = grid_pair<kLow>(rg.ev[(e[j] + q) & (kEvRing - 1)], km[j].x, km[j].y, km[j].z, km[j].w, G);
+                const float d = __fadd_rn(LP[j], x.x);
+                up[j] = __fadd_rn(S1[j], x.y);
+                sk[j] = __fadd_rn(l4[j], G.skip);
+                top[j] = max3_nan(d, up[j], sk[j]);
+                if (kLow) below |= (x.y < g_lim) & (top[j] != sk[j]);
+            }
+            const bool right = ll < ur;  // both ends are finite
+            k0 += right ? 1 : 0;
+            vs -= right ? kOne : 0u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (top[j] == sk[j]) w[j] |= ABEA_FROM_L << (8 * q);
+                if (top[j] == up[j] && top[j] != sk[j]) w[j] |= ABEA_FROM_U << (8 * q);
+                LP[j] = l4[j];
+                S1[j] = vs + (uint32_t)j * kOne < kIn ? top[j] : -INFINITY;
+            }
+            my_k0 = (((b + q) & 31) == lane) ? k0 : my_k0;
+            if (kScores && scores && in_bounds(b + q, r.n_bands, a.counters))
+                reinterpret_cast<float4*>(scores + (int64_t)(b + q) * kSlots)[lane] = make_float4(S1[0], S1[1], S1[2], S1[3]);
+        }
+        const float mx = max_nan(max_nan(S1[0], S1[1]), max_nan(S1[2], S1[3]));
+        if (__any_sync(kFull, below | (mx != mx))) {
+            const float4 s4 = rg.save[0][lane], l4 = rg.save[1][lane];
+            S1[0] = s4.x; S1[1] = s4.y; S1[2] = s4.z; S1[3] = s4.w;
+            LP[0] = l4.x; LP[1] = l4.y; LP[2] = l4.z; LP[3] = l4.w;
+            k0 = k_was;
+            my_k0 = my_was;
+            return false;
+        }
+        e0 = b + 3 - 2 - k0;
+        if ((!kSpan || trace) && in_bounds((b - sp.trace_band0) >> 2, sp.trace_tiles, a.counters))
+            reinterpret_cast<uint4*>(trace + (int64_t)((b - sp.trace_band0) >> 2) * 512)[lane] = make_uint4(w[0], w[1], w[2], w[3]);
+        if (sp.side && ((b + 3) & 31) == 31) {
+            if (in_bounds(((b + 3) & ~31) + lane, r.n_bands, a.counters)) bk0[((b + 3) & ~31) + lane] = my_k0;
+        }
+        return true;
+    };
+    // checkpoint b / kCkBands, when band b has one: the state this loop resumes from there
+    auto checkpoint = [&]() {
+        if (kSpan && sp.ck_out && (b & (kCkBands - 1)) == 0 &&
+            in_bounds(b / kCkBands, r.n_bands / kCkBands + 1, a.counters)) {
+            float* rec = sp.ck_out + (int64_t)(b / kCkBands) * kCkStride;
+            reinterpret_cast<float4*>(rec)[lane] = make_float4(S1[0], S1[1], S1[2], S1[3]);
+            reinterpret_cast<float4*>(rec + kSlots)[lane] = make_float4(LP[0], LP[1], LP[2], LP[3]);
+            if (lane == 0) {
+                rec[2 * kSlots] = __int_as_float(k0);
+                rec[2 * kSlots + 1] = __int_as_float(e0);
+            }
+        }
+    };
+    // all 100 cells of bands b .. b + 3 are computed, none on the last k-mer column, and
+    // their scores are in a grid's range
+    auto grid_next = [&]() {
+        if (b < grid_from || b + 4 > n_bands || k0 < 0 || k0 + 4 + kBand > n_kmers - 1 || e0 < kBand - 1 ||
+            e0 + 4 > n_events - 1)
+            return false;
+        if (b >= grid_until) {
+            grid = grid_now();
+            grid_until = b + 16;
+            if (grid && grid != g_made) {
+                G = make_grid(cc, grid);
+                g_made = grid;
+            }
+        }
+        return grid != 0;
+    };
     while (true) {
         bool to_slow = false;
         for (; b < n_bands; ++b) {
-            if (kSpan && sp.ck_out && (b & (kCkBands - 1)) == 0 &&
-                in_bounds(b / kCkBands, r.n_bands / kCkBands + 1, a.counters)) {
-                // checkpoint s = b / kCkBands: the state this loop resumes from at band b
-                float* rec = sp.ck_out + (int64_t)(b / kCkBands) * kCkStride;
-                reinterpret_cast<float4*>(rec)[lane] = make_float4(S1[0], S1[1], S1[2], S1[3]);
-                reinterpret_cast<float4*>(rec + kSlots)[lane] = make_float4(LP[0], LP[1], LP[2], LP[3]);
-                if (lane == 0) {
-                    rec[2 * kSlots] = __int_as_float(k0);
-                    rec[2 * kSlots + 1] = __int_as_float(e0);
-                }
-            }
+            checkpoint();
             if ((b & 3) == 0) {
                 if (rings_step(rg, rs, a, r, lane, k0, e0, 6)) __syncwarp();
+                if (grid_next()) {
+                    while (true) {
+                        if (!(grid < kGridWide ? grid_bands(std::true_type{}) : grid_bands(std::false_type{}))) {
+                            // these four bands exact; many more after repeated failures
+                            pen = pen < 32 ? pen + 8 : min(2 * pen, 4096);
+                            grid_from = b + 4 + (pen > 32 ? 4 * pen : 0);
+                            grid_until = 0;
+                            break;
+                        }
+                        pen = max(pen - 1, 0);
+                        b += 4;
+                        checkpoint();
+                        if (rings_step(rg, rs, a, r, lane, k0, e0, 6)) __syncwarp();
+                        if (!grid_next()) break;
+                    }
+                    if (b >= n_bands) break;
+                    // back to the exact loop: band b's emission side
+                    const float4 gm4 = *reinterpret_cast<const float4*>(&rg.gm[4 * lane]);
+                    const float4 sd4 = *reinterpret_cast<const float4*>(&rg.sd[4 * lane]);
+                    const float4 rs4 = *reinterpret_cast<const float4*>(&rg.rsd[4 * lane]);
+                    const float4 k14 = *reinterpret_cast<const float4*>(&rg.k1[4 * lane]);
+                    const float gmv[4] = {gm4.x, gm4.y, gm4.z, gm4.w}, sdv[4] = {sd4.x, sd4.y, sd4.z, sd4.w};
+                    const float rsv[4] = {rs4.x, rs4.y, rs4.z, rs4.w}, k1v[4] = {k14.x, k14.y, k14.z, k14.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        ep[j] = e0 - ((4 * lane + j - k0) & 127);
+                        nc[j] = next_cell(LP[j], rg.ev[(ep[j] + 1) & (kEvRing - 1)], gmv[j], sdv[j], rsv[j], k1v[j], cc);
+                    }
+                }
             }
             // ---- exchange: end cells for the placement, left neighbour of slot 4*lane
             const int sl = k0 & 127, su = (k0 + kBand - 1) & 127;
@@ -572,6 +722,19 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
     cp_async_wait_all();  // no copy may land in shared memory after the read is done
     __syncwarp();
     if (slow && sp.side) atomicAdd(&a.counters[0], slow);
+}
+
+// The forward pass of a checkpointed read by one warp, as a call: its code stays out of
+// the kernels that mostly run the other.
+// Shared memory goes by its own address, so that its accesses stay shared ones.
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+template <class T>
+__device__ __forceinline__ T& smem_ref(unsigned at) {
+    return *reinterpret_cast<T*>(__cvta_shared_to_generic(at));
+}
+template <bool kScores>
+__device__ __noinline__ void fill_warp_ck(const CoreArgs& a, const ReadDesc& r, unsigned rg_at, int lane) {
+    fill_warp<kScores, true>(a, r, smem_ref<Rings>(rg_at), lane, forward_span(a, r));
 }
 
 // ---------------------------------------------------------------- wide shape
@@ -696,6 +859,8 @@ __device__ __noinline__ SlowCell slow_cell_call(float diag, float up, float left
 }
 
 // A read as the two engines see it.
+// kCk: a checkpointed read (code of its own: its tests cost the other reads 3%).
+template <bool kCk>
 struct WideRead {
     const CoreArgs& a;
     const ReadDesc& r;
@@ -712,7 +877,22 @@ struct WideRead {
         if (t < kWideChunk && band < n_bands && in_bounds(band, n_bands, a.counters))
             bk0[band] = ws.kb[band & (kScoreRing - 1)] >> 2;
     }
-    __device__ __forceinline__ bool tile_in(int j) const { return in_bounds(j, (n_bands + 3) / 4, a.counters); }
+    // whether tile j of the trace is to be stored
+    __device__ __forceinline__ bool tile_in(int j) const { return !kCk && in_bounds(j, (n_bands + 3) / 4, a.counters); }
+    // A checkpointed read's record after chunk j, the state before band 4(j + 1), when that
+    // band has one (nullptr: none).  The record: the scores of band 4j + 3, those of band
+    // 4j + 2 shifted by one slot, and band 4j + 3's placement (record_end, one thread).
+    __device__ __forceinline__ float* record(int j) const {
+        constexpr int kEvery = kCkBands / kWideChunk;
+        const int s = (j + 1) / kEvery;
+        return kCk && (j + 1) % kEvery == 0 && in_bounds(s, n_bands / kCkBands + 1, a.counters)
+                   ? a.ck + r.ck_off + (int64_t)s * kCkStride
+                   : nullptr;
+    }
+    __device__ __forceinline__ void record_end(float* rec, int j, int k0) const {
+        rec[2 * kSlots] = __int_as_float(k0);
+        rec[2 * kSlots + 1] = __int_as_float(kWideChunk * j + 1 - k0);  // the event of band 4j + 3
+    }
     // the end cells of band b-1 (its row of the ring) and the left neighbour of a slot
     __device__ __forceinline__ void ends(int row, int k0, float& ll, float& ur) const {
         ll = ws.sc[row][k0 & (kSlots - 1)];
@@ -723,7 +903,8 @@ struct WideRead {
 // ---- exact engine
 // E: chunk j's emissions for slot t into ring slot s, from the placement kp of an earlier
 // band.
-__device__ __forceinline__ void exact_chunk(const WideRead& w, int t, int s, int j, int kp) {
+template <bool kCk>
+__device__ __forceinline__ void exact_chunk(const WideRead<kCk>& w, int t, int s, int j, int kp) {
     const ReadDesc& r = w.r;
     const int kk = kp + ((t - kp) & (kSlots - 1));  // slot t's k-mer in the window
     const bool kin = kk >= 0 && kk < w.n_kmers;
@@ -760,8 +941,8 @@ __device__ __forceinline__ void exact_chunk(const WideRead& w, int t, int s, int
 
 // Chunks j0 .. j1 - 1, from the bands before them in the score ring; every thread of the
 // block calls it.
-template <bool kScores>
-__device__ __forceinline__ void chain_exact(const WideRead& w, int tid, int j0, int j1) {
+template <bool kScores, bool kCk>
+__device__ __forceinline__ void chain_exact(const WideRead<kCk>& w, int tid, int j0, int j1) {
     const int warp = tid >> 5;
     if (warp >= 4 + 4 * kExactGroups) return;
     WideSmem& ws = w.ws;
@@ -875,6 +1056,11 @@ __device__ __forceinline__ void chain_exact(const WideRead& w, int tid, int j0, 
         }
         if (j + kExactRing < j1) named_bar_arrive(kBarExEmpty + s, kBoth);  // E may refill its slot
         keep(min(b0 + kWideChunk, n_bands) - 1, !kMid);
+        if (float* rec = kEdge ? nullptr : w.record(j)) {
+            rec[t] = s1;
+            rec[kSlots + t] = lp;
+            if (t == 0) w.record_end(rec, j, k0);
+        }
         if (w.tile_in(j)) reinterpret_cast<uint32_t*>(w.trace + (int64_t)j * 512)[t] = word;
         if (warp == 0) {
             __syncwarp();  // thread 0 wrote the placements
@@ -951,8 +1137,8 @@ __device__ __forceinline__ int chunk_mode(int want, int kp, int b0, int n_events
 // Chunks from j0 on, until one that no grid serves (ws.exit), from the bands before them
 // in the score ring; `first`: the grid of those.  Every thread of the block calls it, with
 // ws.head and ws.flag zero and ws.exit the largest int.
-template <bool kScores>
-__device__ __forceinline__ void chain_grid(const WideRead& w, int tid, int j0, int first, uint32_t modes) {
+template <bool kScores, bool kCk>
+__device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int j0, int first, uint32_t modes) {
     const int warp = tid >> 5, lane = tid & 31;
     if ((warp & 3) < 2 && warp >= 6) return;
     WideSmem& ws = w.ws;
@@ -1015,6 +1201,13 @@ __device__ __forceinline__ void chain_grid(const WideRead& w, int tid, int j0, i
                     }
                     store_tile(jr, w0, w1);
                     w.store_origins(jr, t);
+                }
+                if (float* rec = w.record(jr)) {
+                    const float* last = ws.sc[(br + 3) & (kScoreRing - 1)];
+                    const float* prev = ws.sc[(br + 2) & (kScoreRing - 1)];
+                    reinterpret_cast<float2*>(rec)[t] = *reinterpret_cast<const float2*>(last + kPerLane * t);
+                    reinterpret_cast<float2*>(rec + kSlots)[t] = make_float2(prev[tl], prev[kPerLane * t]);
+                    if (t == 0) w.record_end(rec, jr, kp);
                 }
             }
             if (mode) {
@@ -1232,11 +1425,13 @@ __device__ __forceinline__ void chain_grid(const WideRead& w, int tid, int j0, i
     if (slow) atomicAdd(&a.counters[0], slow);
 }
 
-// One read's fill.  `grids`: the read's k-mers allow grids (grid_kmer_ok).
-template <bool kScores>
-__device__ void fill_chain(const CoreArgs& a, const ReadDesc& r, WideSmem& ws, int tid, bool grids) {
+// One read's fill.  `grids`: the read's k-mers allow grids (grid_kmer_ok).  A call, as
+// fill_warp_ck is: each has the block's registers to itself.
+template <bool kScores, bool kCk>
+__device__ __noinline__ void fill_chain(const CoreArgs& a, const ReadDesc& r, unsigned ws_at, int tid, bool grids) {
+    WideSmem& ws = smem_ref<WideSmem>(ws_at);
     const int lane = tid & 31;
-    WideRead w{a, r, ws, make_consts(r, a.g), r.n_events, r.n_kmers, r.n_bands, (r.n_bands + kWideChunk - 1) / kWideChunk,
+    WideRead<kCk> w{a, r, ws, make_consts(r, a.g), r.n_events, r.n_kmers, r.n_bands, (r.n_bands + kWideChunk - 1) / kWideChunk,
                a.trace + r.trace_off * kSlots, a.band_k0 + r.band_off, kScores ? a.scores + r.band_off * kSlots : nullptr};
     const uint32_t modes = grids ? grid_modes(w.cc) : 0u;
     // band 0: the start cell (slot 127) = 0; band 1: the trim cell; both at k0 = -51
@@ -1326,8 +1521,6 @@ struct ClShared {
     int32_t progress;        // block 1: block 0 is done with the emissions of bands <= progress
     int32_t pick;
 };
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -1825,14 +2018,16 @@ __device__ bool walk_segment(const uint8_t* trace, int trace_band0, int bands_en
 }
 
 // Recomputes the trace of segment seg (bands [seg*kCkBands, (seg+1)*kCkBands)) of
-// a checkpointed read into its scratch slot.  The whole warp calls it.
-__device__ __forceinline__ void recompute_segment(const CoreArgs& ca, const ReadDesc& r, Rings& rg, int lane, int seg) {
+// a checkpointed read into `mem` (kCkBands * kSlots bytes).  The whole warp calls it.
+__device__ __noinline__ void recompute_segment(const CoreArgs& ca, const ReadDesc& r, unsigned rg_at, int lane, int seg,
+                                               uint8_t* mem) {
+    Rings& rg = smem_ref<Rings>(rg_at);
     FillSpan sp;
     sp.b_begin = max(2, seg * kCkBands);
     sp.b_end = min((seg + 1) * kCkBands, r.n_bands);
     sp.ck_in = seg > 0 ? ca.ck + r.ck_off + (int64_t)seg * kCkStride : nullptr;
     sp.ck_out = nullptr;
-    sp.trace = ca.ck_scratch + (int64_t)r.ck_slot * (kCkBands * kSlots);
+    sp.trace = mem;
     sp.trace_band0 = seg * kCkBands;
     sp.trace_tiles = kCkBands / 4;
     sp.side = false;
@@ -1879,7 +2074,7 @@ __device__ void best_end_warp(const PostArgs& a, const ReadDesc& r, int lane, fl
 template <int kRing>
 __device__ void post_tail(const CoreArgs& ca, const PostArgs& a, int ri, const ReadDesc& r, uint8_t* ring, Rings& rg,
                           int lane, float best, int best_e, int n_out, int max_gap, int status, int last_k,
-                          int last_from);
+                          int last_from, uint8_t* ck_seg);
 
 // `ring`: kRing * 2 KB of shared memory (16-byte aligned) for the traceback's trace chunks.
 // A finished read's pairs out[0, n) into the caller's host buffer, when the batch
@@ -1911,7 +2106,7 @@ __device__ void post_read_warp(const CoreArgs& ca, const PostArgs& a, int ri, ui
 
     abea_aligned_pair_t* out = a.pairs + r.out_off;
     const uint8_t* trace = a.trace + r.trace_off * kSlots;
-    const uint8_t* ck_seg = ca.ck_scratch + (int64_t)r.ck_slot * (kCkBands * kSlots);
+    uint8_t* ck_seg = r.ck ? ca.ck_scratch + (int64_t)r.ck_slot * (kCkBands * kSlots) : nullptr;  // recompute scratch
     const int32_t* bk0 = a.band_k0 + r.band_off;
     const int cap = r.out_cap;
     int n_out = 0, max_gap = 0, status = 0, last_k = n_kmers - 1, last_from = 0;
@@ -1925,7 +2120,7 @@ __device__ void post_read_warp(const CoreArgs& ca, const PostArgs& a, int ri, ui
             // the trace was not kept: recompute it kCkBands bands at a time from
             // the checkpoints, top segment first, and walk each
             for (int seg = (w.k + w.e + 2) / kCkBands; seg >= 0; --seg) {
-                recompute_segment(ca, r, rg, lane, seg);
+                recompute_segment(ca, r, smem_u32(&rg), lane, seg, ck_seg);
                 if (walk_segment<kWalkPairs, kRing>(ck_seg, seg * kCkBands, min((seg + 1) * kCkBands, n_bands),
                                                seg * kCkBands, ring, lane, w, out, cap, a, r))
                     break;
@@ -1968,17 +2163,16 @@ __device__ void post_read_warp(const CoreArgs& ca, const PostArgs& a, int ri, ui
     last_from = __shfl_sync(kFull, last_from, 0);
     __syncwarp();
     __threadfence_block();
-    post_tail<kRing>(ca, a, ri, r, ring, rg, lane, best, best_e, n_out, max_gap, status, last_k, last_from);
+    post_tail<kRing>(ca, a, ri, r, ring, rg, lane, best, best_e, n_out, max_gap, status, last_k, last_from, ck_seg);
 }
 
 template <int kRing>
 __device__ void post_tail(const CoreArgs& ca, const PostArgs& a, int ri, const ReadDesc& r, uint8_t* ring, Rings& rg,
                           int lane, float best, int best_e, int n_out, int max_gap, int status, int last_k,
-                          int last_from) {
+                          int last_from, uint8_t* ck_seg) {
     const int n_kmers = r.n_kmers, n_bands = r.n_bands;
     abea_aligned_pair_t* out = a.pairs + r.out_off;
     const uint8_t* trace = a.trace + r.trace_off * kSlots;
-    const uint8_t* ck_seg = ca.ck_scratch + (int64_t)r.ck_slot * (kCkBands * kSlots);
     const int32_t* bk0 = a.band_k0 + r.band_off;
     const int cap = r.out_cap;
     int result = 0;
@@ -2021,7 +2215,7 @@ __device__ void post_tail(const CoreArgs& ca, const PostArgs& a, int ri, const R
             // recompute and walk again, summing the emissions in walk order
             Walk w{n_kmers - 1, best_e, 0, 0, 0, n_kmers - 1, 0, 0.0};
             for (int seg = (w.k + w.e + 2) / kCkBands; seg >= 0; --seg) {
-                recompute_segment(ca, r, rg, lane, seg);
+                recompute_segment(ca, r, smem_u32(&rg), lane, seg, ck_seg);
                 if (walk_segment<kWalkSum, kRing>(ck_seg, seg * kCkBands, min((seg + 1) * kCkBands, n_bands),
                                               seg * kCkBands, ring, lane, w, out, cap, a, r))
                     break;
@@ -2361,7 +2555,7 @@ __device__ void post_wide_block(const CoreArgs& ca, const PostArgs& a, int ri, u
         // emissions outside the exact integer form: warp 0 sums serially in walk order
         if (warp == 0)
             post_tail<kPostRingDeep>(ca, a, ri, r, wide_mem, rg0, lane, best, best_e, n_out, max_gap, 0, last_k,
-                                     last_from);
+                                     last_from, nullptr);
         return;
     }
     const bool pass = ps.pass != 0;
@@ -2378,6 +2572,53 @@ __device__ void post_wide_block(const CoreArgs& ca, const PostArgs& a, int ri, u
     if (t == 0) post_write(a, ri, pass ? n_out : 0, best, best_e, 0, n_out, cap, pass, last_from);
 }
 
+// ---------------------------------------------------------------- wide checkpointed read's traceback
+static_assert(sizeof(int32_t) * kSpecRound * kSpecBands >= (size_t)(kWideThreads / 32) * kCkBands * kSlots,
+              "a traceback map's memory holds one segment's trace per warp");
+// A checkpointed read on the wide shape: the block's 16 warps recompute 16 segments of
+// kCkBands bands at a time, top ones first, each into a part of `mem` (a traceback
+// map's memory: the two never meet in one read), and warp 0 walks them.  One segment at a time on one warp, the
+// recompute alone took 390 cycles per band (560 before the warp shape's grid loop) with
+// the SM otherwise idle.  Every thread of the block calls it; `ended` in shared memory.
+__device__ void post_ck_block(const CoreArgs& ca, const PostArgs& a, int ri, uint8_t* wide_mem, Rings* rings,
+                              int32_t& ended, int t, uint8_t* mem) {
+    constexpr int kSegBytes = kCkBands * kSlots;
+    const int warp = t >> 5, lane = t & 31;
+    const ReadDesc r = a.reads[ri];
+    abea_aligned_pair_t* out = a.pairs + r.out_off;
+    float best;
+    int best_e;
+    best_end_warp(a, r, lane, best, best_e);  // every warp alike
+    Walk w{r.n_kmers - 1, best_e, 0, 0, 0, r.n_kmers - 1, 0, 0.0};
+    if (best > -INFINITY) {
+        for (int top = (w.k + w.e + 2) / kCkBands; top >= 0; top -= kWideThreads / 32) {
+            if (top - warp >= 0)
+                recompute_segment(ca, r, smem_u32(&rings[warp]), lane, top - warp, mem + (int64_t)warp * kSegBytes);
+            if (t == 0) ended = 0;
+            __syncthreads();  // the segments are in memory
+            if (warp == 0) {
+                for (int i = 0; i < kWideThreads / 32 && top - i >= 0; ++i) {
+                    const int seg = top - i;
+                    if (walk_segment<kWalkPairs, kPostRingDeep>(mem + (int64_t)i * kSegBytes, seg * kCkBands,
+                                                                min((seg + 1) * kCkBands, r.n_bands), seg * kCkBands,
+                                                                wide_mem, lane, w, out, r.out_cap, a, r)) {
+                        if (lane == 0) ended = 1;
+                        break;
+                    }
+                }
+            }
+            __syncthreads();
+            if (ended) break;
+        }
+    }
+    if (warp != 0) return;
+    __syncwarp();
+    __threadfence_block();
+    // without a finite end the reference's flat-array walk needs the whole trace: undefined
+    post_tail<kPostRingDeep>(ca, a, ri, r, wide_mem, rings[0], lane, best, best_e, w.n_out, w.max_gap,
+                             best > -INFINITY ? 0 : ABEA_ERR_UNDEFINED, w.last_k, w.last_from, mem);
+}
+
 // ---------------------------------------------------------------- plain form kernels
 template <bool kScores>
 __global__ void __launch_bounds__(32) abea_core_warp_kernel(CoreArgs a) {
@@ -2392,7 +2633,7 @@ __global__ void __launch_bounds__(32) abea_core_warp_kernel(CoreArgs a) {
         fill_warp<kScores, false>(a, r, rg, threadIdx.x, forward_span(a, r));
 }
 
-__global__ void __launch_bounds__(32) abea_post_kernel(CoreArgs ca, PostArgs a) {
+__global__ void __launch_bounds__(32) abea_post_kernel(const __grid_constant__ CoreArgs ca, const __grid_constant__ PostArgs a) {
     __shared__ __align__(16) uint8_t ring[kPostRingDeep * kPostChunkBands * kSlots];
     __shared__ __align__(16) Rings rg;  // recompute of checkpointed reads
     const int i = blockIdx.x;
@@ -2412,6 +2653,7 @@ struct BatchedSmem {
     int32_t pick;                      // the block's wide read, or -1
     int32_t wide_slot;                 // the block's first pick: its traceback scratch slot
     int32_t free_rank;                 // rank among the blocks without a wide read, or -1
+    int32_t ended;                     // a checkpointed read's path has ended
 };
 static_assert(offsetof(BatchedSmem, warp_rings) % 16 == 0 && offsetof(BatchedSmem, post) % 16 == 0 &&
                   sizeof(Rings) % 16 == 0 && sizeof(PostSmem) % 16 == 0,
@@ -2425,7 +2667,8 @@ static_assert(sizeof(WideSmem) >= kPostRingDeep * kPostChunkBands * kSlots && al
 static_assert(sizeof(WidePostSmem) <= sizeof(WideSmem), "the wide read's traceback state fits the fill's memory");
 
 template <bool kScores>
-__global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(CoreArgs a, PostArgs p, PreArgs pa) {
+__global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(const __grid_constant__ CoreArgs a, const __grid_constant__ PostArgs p,
+                                                                       const __grid_constant__ PreArgs pa) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BatchedSmem& sm = *reinterpret_cast<BatchedSmem*>(smem_raw);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -2447,11 +2690,20 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(CoreArgs 
         const ReadDesc& r = a.reads[wide_read];
         const bool odd = pre_read(pa, wide_read, t, kWideThreads);
         const bool grids = !__syncthreads_or(odd);  // the read's parameters are in memory for the whole block
-        if (!r.skip) fill_chain<kScores>(a, r, sm.wide, t, grids);
+        if (!r.skip) {
+            if (r.ck)
+                fill_chain<kScores, true>(a, r, smem_u32(&sm.wide), t, grids);
+            else
+                fill_chain<kScores, false>(a, r, smem_u32(&sm.wide), t, grids);
+        }
         __syncthreads();
         __threadfence_block();
         // the whole block walks the wide read's traceback (the fill's shared memory is free)
-        post_wide_block(a, p, wide_read, reinterpret_cast<uint8_t*>(&sm.wide), sm.warp_rings[0], t, wide_slot);
+        if (r.ck && !r.skip && wide_slot < a.n_spec)
+            post_ck_block(a, p, wide_read, reinterpret_cast<uint8_t*>(&sm.wide), sm.warp_rings, sm.ended, t,
+                          reinterpret_cast<uint8_t*>(a.spec + (int64_t)wide_slot * (kSpecRound * kSpecBands)));
+        else
+            post_wide_block(a, p, wide_read, reinterpret_cast<uint8_t*>(&sm.wide), sm.warp_rings[0], t, wide_slot);
         // then the next wide read past the first wave (one per block), longest first
         __syncthreads();  // the traceback is done with the block's shared memory and the pick
         if (t == 0) {
@@ -2486,7 +2738,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(CoreArgs 
         __syncwarp();  // the read's parameters are in memory for the warp
         if (!r.skip) {
             if (r.ck)
-                fill_warp<kScores, true>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
+                fill_warp_ck<kScores>(a, r, smem_u32(&sm.warp_rings[warp]), lane);
             else
                 fill_warp<kScores, false>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
         }
@@ -2513,7 +2765,7 @@ static_assert(sizeof(BatchedClSmem) <= 227 * 1024, "cluster kernel shared memory
 // single-block kernel.
 template <bool kScores>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
-    abea_batched_cl_kernel(CoreArgs a, PostArgs p) {
+    abea_batched_cl_kernel(const __grid_constant__ CoreArgs a, const __grid_constant__ PostArgs p) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BatchedClSmem& sm = *reinterpret_cast<BatchedClSmem*>(smem_raw);
@@ -2548,7 +2800,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
         const ReadDesc& r = a.reads[ri];
         if (!r.skip) {
             if (r.ck)
-                fill_warp<kScores, true>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
+                fill_warp_ck<kScores>(a, r, smem_u32(&sm.warp_rings[warp]), lane);
             else
                 fill_warp<kScores, false>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
         }

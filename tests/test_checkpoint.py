@@ -88,3 +88,42 @@ def test_f5c_batch_with_reads_over_8kb_checkpointed(oracle_mod, mode):
     _, dev, gp, gc = align(batch, mode, budget)
     op, oc, _ = oracle_mod.align_batch(batch, threads=os.cpu_count())
     same_alignments(batch, gp, gc, op, oc)
+
+
+@pytest.mark.parametrize("kept", [0, 2])
+def test_checkpointed_reads_on_the_wide_shape(oracle_mod, kept):
+    """Reads whose band counts lie around one checkpoint (256), a traceback slot's least
+    read (512) and one round of sixteen recomputed segments (4,096), every read on the
+    wide shape: all checkpointed, or only the longest ones."""
+    from abea_gb300 import synth
+    rng = np.random.default_rng(5)
+    model = synth.make_model(rng)
+    reads = []
+    for target in (254, 256, 257, 511, 512, 513, 516, 4093, 4095, 4096, 4097, 4100, 8192, 8193):
+        seq, ev = synth.make_read(rng, model, int(target / 2.4), 1.02, 2.0, 1.2, skip_p=0.01, mean_events=1.8)
+        over = len(ev) + len(seq) - 5 + 2 - target  # a longer read, less its end
+        assert over >= 0
+        reads.append((seq.tobytes()[:len(seq) - over * 10 // 27], ev[:len(ev) - (over - over * 10 // 27)]))
+    sc = np.zeros(len(reads), dtype=abea.types.SCALINGS_DTYPE)
+    sc["scale"], sc["shift"], sc["var"], sc["log_var"] = 1.02, 2.0, 1.2, np.log(1.2)
+    batch = abea.from_reads([r[0] for r in reads], [r[1] for r in reads], sc, model)
+    assert 4096 in batch.n_bands() and 512 in batch.n_bands()
+    budget = int(np.sort(batch.n_bands())[-kept - 1]) // 4 * 4 * BYTES_PER_BAND if kept else 1
+    ctx = abea.Context(0, abea.MODE_BATCHED)
+    ctx.set_option(abea.OPT_TRACE_BUDGET, budget)
+    ctx.set_option(abea.OPT_LONG_READ_BANDS, 1)
+    dev = ctx.upload(batch)
+    dev.run()
+    pairs, counts = dev.results()
+    op, oc, obest = oracle_mod.align_batch(batch)
+    same_alignments(batch, pairs, counts, op, oc)
+    assert np.array_equal(dev.best_scores().view(np.uint32), obest.view(np.uint32))
+
+
+def test_more_checkpointed_reads_than_blocks(oracle_mod):
+    from abea_gb300 import synth
+    batch = synth.make_batch("small", seed=6, lengths=[230, 260, 90] * 150)
+    _, dev, gp, gc = align(batch, abea.MODE_BATCHED, 1)
+    op, oc, obest = oracle_mod.align_batch(batch)
+    same_alignments(batch, gp, gc, op, oc)
+    assert np.array_equal(dev.best_scores().view(np.uint32), obest.view(np.uint32))

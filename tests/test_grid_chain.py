@@ -1,8 +1,8 @@
-"""The wide shape's two engines against the oracle, with every score, backpointer and
-band origin: reads that end around the points where the exact chain hands over to the
-grid chain and back, emissions that no grid serves or that lie far below its range, and
-events that are not finite.  All comparisons are exact: the results are the reference's
-floats, whichever engine computes a band."""
+"""The wide shape's two engines, and the warp shape's two loops, against the oracle, with
+every score, backpointer and band origin: reads that end around the points where the
+exact chain hands over to the grid chain and back, emissions that no grid serves or that
+lie far below its range, and events that are not finite.  All comparisons are exact: the
+results are the reference's floats, whichever engine computes a band."""
 import numpy as np
 import pytest
 
@@ -26,9 +26,9 @@ def batch_of(model, reads):
     return abea.from_reads([r[0] for r in reads], [r[1] for r in reads], sc, model)
 
 
-def check(oracle_mod, batch):
+def check(oracle_mod, batch, shape):
     ctx = abea.Context(0, abea.MODE_BATCHED, store_scores=True)
-    ctx.set_option(abea.OPT_LONG_READ_BANDS, 1)  # every read on the wide shape
+    ctx.set_option(abea.OPT_LONG_READ_BANDS, 1 if shape == "wide" else 1 << 40)
     dev = ctx.upload(batch)
     dev.run()
     pairs, counts = dev.results()
@@ -45,8 +45,9 @@ def check(oracle_mod, batch):
         assert np.array_equal(bll, info["bll"]), i
 
 
+@pytest.mark.parametrize("shape", ["wide", "warp"])
 @pytest.mark.parametrize("mean_events", [1.05, 1.8, 4.0])
-def test_hand_over_between_the_engines(oracle_mod, mean_events):
+def test_hand_over_between_the_engines(oracle_mod, mean_events, shape):
     """Reads of 6 bases up to ones with long grid runs, around the 800 bands after which
     the grid chain is first tried, at three event rates (few moves right, and many)."""
     rng = np.random.default_rng(11)
@@ -57,24 +58,26 @@ def test_hand_over_between_the_engines(oracle_mod, mean_events):
         seq, ev = synth.make_read(rng, model, length, 1.02, 2.0, 1.2, skip_p=0.01, mean_events=mean_events)
         if len(ev):
             reads.append((seq.tobytes(), ev))
-    check(oracle_mod, batch_of(model, reads))
+    check(oracle_mod, batch_of(model, reads), shape)
 
 
+@pytest.mark.parametrize("shape", ["wide", "warp"])
 @pytest.mark.parametrize("stdv", [(0.05, 0.4), (0.3, 1.0), (0.8, 1.1), (8.0, 30.0)])
-def test_emissions_a_grid_does_not_serve(oracle_mod, stdv):
+def test_emissions_a_grid_does_not_serve(oracle_mod, stdv, shape):
     """Deviations so small that emissions are positive (no grid) or lie thousands below
     (their cells must lose or be done again), and so large that scores fall slowly."""
     rng = np.random.default_rng(12)
     model, seq, ev = make(rng, 1800, stdv=stdv)
-    check(oracle_mod, batch_of(model, [(seq, ev)]))
+    check(oracle_mod, batch_of(model, [(seq, ev)]), shape)
 
 
+@pytest.mark.parametrize("shape", ["wide", "warp"])
 @pytest.mark.parametrize("value", [np.inf, -np.inf, 1e30, -1e5, 4000.0])
-def test_outlier_events(oracle_mod, value):
+def test_outlier_events(oracle_mod, value, shape):
     """Single events far out or infinite, in and around the grid chain's bands."""
     rng = np.random.default_rng(13)
     model, seq, ev = make(rng, 2400)
     ev = ev.copy()
     for at in (700, 1500, 1501, 2600, len(ev) - 40):
         ev["mean"][at] = value
-    check(oracle_mod, batch_of(model, [(seq, ev)]))
+    check(oracle_mod, batch_of(model, [(seq, ev)]), shape)
