@@ -1109,9 +1109,16 @@ extern "C" abea_status_t abea_batch_read_bands(abea_ctx_t* c, abea_batch_t* b, i
 static abea_status_t queue_backward(abea_ctx* c, abea_batch* b, bool model_grad) {
     if (model_grad)
         CUDA_TRY(cudaMemsetAsync(b->d_grad_model, 0, sizeof(double) * 2 * ABEA_NUM_KMER, c->stream));
+    // One block per read takes as long as the longest read or the SMs' share of all of
+    // them, whichever is more: where the longest read decides, a cluster per read.
+    int64_t longest = 0, all = 0;
+    for (const ReadDesc& r : b->reads) {
+        longest = std::max<int64_t>(longest, r.n_events);
+        all += r.n_events;
+    }
     AdjArgs a{b->d_reads, b->n_reads, b->var_aware, b->d_seq, b->d_model, b->d_ev_mean, b->d_pairs,
               b->d_path_len, b->d_path_flags, b->d_grad_sc, b->d_gn, b->d_path_em,
-              model_grad ? b->d_grad_model : nullptr, b->d_adj_status};
+              model_grad ? b->d_grad_model : nullptr, b->d_adj_status, longest * c->sm_count > all};
     cudaError_t e = launch_adjoint(a, c->stream);
     if (e != cudaSuccess) return fail(ABEA_ERR_CUDA, "adjoint launch failed: %s", cudaGetErrorString(e));
     return ABEA_OK;

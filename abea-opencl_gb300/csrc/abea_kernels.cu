@@ -3077,26 +3077,42 @@ extern "C" abea_status_t abea_align_noalloc(abea_aligned_pair_t* pairs, int32_t*
 // sd = stdv (times var when var-aware).  Everything is evaluated and accumulated
 // in FP64.  Also accumulated: the Gauss-Newton normal equations of the residuals
 // a in (shift, scale) — J^T J and J^T a with J = (-1/sd, -mu/sd) — and the FP64
-// emission sum of the path.
+// emission sum of the path.  One block per read, or a cluster of kAdjSplit blocks
+// (a.split), over the path in up to kAdjSplit parts.  The parts and the order in which
+// sums are combined (warps, lanes, parts) depend on the path's length alone, so a read's
+// result does not depend on its batch.
+// Bounded by the FP64 rate (some 60 operations per cell); on one warp per read it was
+// the latency of three dependent loads per 32 cells (see launch_adjoint).
 namespace abea {
 
-__global__ void __launch_bounds__(32) abea_adjoint_kernel(AdjArgs a) {
-    const int ri = blockIdx.x, lane = threadIdx.x;
-    if (ri >= a.n_reads) return;
+constexpr int kAdjThreads = 256, kAdjSums = 9;
+constexpr int kAdjPart = 4096;  // least cells of a part
+
+template <int kBlocks>
+__global__ void __cluster_dims__(kBlocks, 1, 1) __launch_bounds__(kAdjThreads) abea_adjoint_kernel(AdjArgs a) {
+    namespace cg = cooperative_groups;
+    __shared__ double sums[kAdjSums][kAdjThreads];
+    __shared__ double part_sums[kAdjSplit][kAdjSums];  // the cluster's first block's are used
+    const int ri = blockIdx.x / kBlocks, rank = blockIdx.x % kBlocks;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    if (kBlocks > 1) cg::this_cluster().sync();  // every block of the cluster runs before its memory is written
     const ReadDesc r = a.reads[ri];
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // shift, scale, var, j11, j12, j22, t1, t2, em
-    int st = 0;
     const int len = r.skip ? 0 : a.path_len[ri];
     const int flags = r.skip ? 0 : a.path_flags[ri];
-    if (len > 0 && (flags & (kPathTruncated | kPathNoEnd | kPathError))) {
+    int st = 0;
+    if (len > 0 && (flags & (kPathTruncated | kPathNoEnd | kPathError)))
         st = (flags & kPathTruncated) ? ABEA_ERR_CAPACITY : ABEA_ERR_UNDEFINED;
-    } else if (len > 0) {
-        const abea_aligned_pair_t* out = a.pairs + r.out_off;
-        const bool rev = (flags & kPathReversed) != 0;
-        const int last_from = flags >> 8;
-        const char* s = a.seq + r.seq_off;
-        const double scale = r.scale, shift = r.shift, var = r.var, log_var = r.log_var;
-        for (int j = lane; j < len; j += 32) {
+    const int cells = st == 0 ? max(len, 0) : 0;
+    const int parts = min(kAdjSplit, 1 + cells / kAdjPart), per_part = (cells + parts - 1) / parts;
+    const abea_aligned_pair_t* out = a.pairs + r.out_off;
+    const bool rev = (flags & kPathReversed) != 0;
+    const int last_from = flags >> 8;
+    const char* s = a.seq + r.seq_off;
+    const double scale = r.scale, shift = r.shift, var = r.var, log_var = r.log_var;
+    for (int part = rank; part < parts; part += kBlocks) {
+        double acc[kAdjSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // shift, scale, var, j11, j12, j22, t1, t2, em
+        const int end = min(cells, (part + 1) * per_part);
+        for (int j = part * per_part + t; j < end; j += kAdjThreads) {
             const int w = rev ? len - 1 - j : j;  // walk position, 0 = best end
             const abea_aligned_pair_t c = out[j];
             bool counted;
@@ -3107,10 +3123,10 @@ __global__ void __launch_bounds__(32) abea_adjoint_kernel(AdjArgs a) {
                 counted = last_from != (int)ABEA_FROM_L;
             }
             if (!counted) continue;
-            uint32_t rank = 0;
+            uint32_t rank_k = 0;
 #pragma unroll
-            for (int q = 0; q < ABEA_KMER_SIZE; ++q) rank = (rank << 2) | base_rank(s[c.ref_pos + q]);
-            const abea_model_t m = a.model[rank];
+            for (int q = 0; q < ABEA_KMER_SIZE; ++q) rank_k = (rank_k << 2) | base_rank(s[c.ref_pos + q]);
+            const abea_model_t m = a.model[rank_k];
             const double mu = m.level_mean, sig = m.level_stdv;
             const double sd = a.var_aware ? sig * var : sig;
             const double lsd = a.var_aware ? (double)m.level_log_stdv + log_var : (double)m.level_log_stdv;
@@ -3127,25 +3143,55 @@ __global__ void __launch_bounds__(32) abea_adjoint_kernel(AdjArgs a) {
             acc[7] -= av * mu * isd;
             acc[8] += -0.91893853320467274 - lsd - 0.5 * av * av;
             if (a.grad_model) {
-                atomicAdd(&a.grad_model[2 * rank], av * scale * isd);
-                atomicAdd(&a.grad_model[2 * rank + 1], (av * av - 1.0) / sig);
+                atomicAdd(&a.grad_model[2 * rank_k], av * scale * isd);
+                atomicAdd(&a.grad_model[2 * rank_k + 1], (av * av - 1.0) / sig);
             }
         }
-    }
+        // A warp per sum: 3,700 additions, a third of butterflies over every warp (which were
+        // a fifth of the FP64 work of a 600-base read).
 #pragma unroll
-    for (int i = 0; i < 9; ++i)
+        for (int i = 0; i < kAdjSums; ++i) sums[i][t] = acc[i];
+        __syncthreads();
+        for (int i = warp; i < kAdjSums; i += kAdjThreads / 32) {
+            double v = sums[i][lane];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) acc[i] += __shfl_xor_sync(kFull, acc[i], off);
-    if (lane == 0) {
-        for (int i = 0; i < 3; ++i) a.grad_scalings[3 * ri + i] = acc[i];
-        for (int i = 0; i < 5; ++i) a.gn[5 * ri + i] = acc[3 + i];
-        a.path_em[ri] = acc[8];
-        a.adj_status[ri] = st;
+            for (int q = 32; q < kAdjThreads; q += 32) v += sums[i][q + lane];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFull, v, off);
+            if (lane == 0) {
+                if (kBlocks > 1)
+                    *cg::this_cluster().map_shared_rank(&part_sums[part][i], 0) = v;
+                else
+                    part_sums[part][i] = v;
+            }
+        }
+        __syncthreads();  // the sums may be written again; part_sums is
     }
+    if (kBlocks > 1) {
+        cg::this_cluster().sync();  // the other blocks' sums are in the first block's memory
+        if (rank != 0) return;
+    }
+    if (t < kAdjSums) {
+        double v = 0.0;
+        for (int i = 0; i < parts; ++i) v += part_sums[i][t];
+        if (t < 3)
+            a.grad_scalings[3 * ri + t] = v;
+        else if (t < 8)
+            a.gn[5 * ri + t - 3] = v;
+        else
+            a.path_em[ri] = v;
+    }
+    if (t == 0) a.adj_status[ri] = st;
 }
 
+// One warp per read took as long as the longest read: 1.7 ms of 512 reads of 1-10 kb, now
+// 0.1-0.2; some 20 ms of a 12 Mb batch with a 65 kb read.
 cudaError_t launch_adjoint(const AdjArgs& a, cudaStream_t stream) {
-    if (a.n_reads > 0) abea_adjoint_kernel<<<a.n_reads, 32, 0, stream>>>(a);
+    if (a.n_reads <= 0) return cudaSuccess;
+    if (a.split)
+        abea_adjoint_kernel<kAdjSplit><<<a.n_reads * kAdjSplit, kAdjThreads, 0, stream>>>(a);
+    else
+        abea_adjoint_kernel<1><<<a.n_reads, kAdjThreads, 0, stream>>>(a);
     return cudaGetLastError();
 }
 

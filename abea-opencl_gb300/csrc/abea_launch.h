@@ -106,7 +106,9 @@ struct AdjArgs {
     double* path_em;        // [n]: sum of the path's emissions (FP64)
     double* grad_model;     // [4096][2]: d/d level_mean, level_stdv, summed over reads
     int32_t* adj_status;    // [n]: 0, or why the read has no gradient
+    int split;              // a cluster of kAdjSplit blocks per read instead of one block
 };
+constexpr int kAdjSplit = 8;
 
 // Backward pass over the stored paths of a finished forward run.
 cudaError_t launch_adjoint(const AdjArgs& a, cudaStream_t stream);

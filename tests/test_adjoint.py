@@ -255,3 +255,28 @@ def test_gpu_recalibration_recovers_perturbed_scalings():
     assert np.array_equal(gc, c2)
     for x, y in zip(abea.split_pairs(batch, gp, gc), abea.split_pairs(b2, p2, c2)):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length", [8, 900, 2250, 4600, 20000])
+def test_gpu_adjoint_in_parts(oracle_mod, length):
+    """Paths of one part, around 4,096 cells (one part or two) and of all eight: a read
+    alone (a cluster of blocks) against the oracle, and the same bits as among 152 more
+    of its kind (one block per read)."""
+    from abea_gb300 import synth
+    b = synth.make_batch("adjoint", seed=31, lengths=[length])
+    ctx = abea.Context(0, abea.MODE_BATCHED)
+    dev = ctx.upload(b)
+    dev.run()
+    one = dev.backward()
+    g, em, gm, lens = oracle_adjoint(oracle_mod, b, 0)
+    assert np.all(np.abs(one["grad_scalings"] - g) <= 1e-9 * (np.abs(g) + 100.0 * lens[:, None]))
+    assert np.all(np.abs(one["path_emission"] - em) <= 1e-9 * (np.abs(em) + 100.0 * lens))
+    assert np.allclose(one["grad_model"], gm, rtol=1e-9, atol=1e-9)
+    seq, ev = read_of(b, 0)
+    many = abea.from_reads([seq] * 153, [ev] * 153, np.repeat(b.scalings[:1], 153), b.model)
+    dev = ctx.upload(many)
+    dev.run()
+    out = dev.backward()
+    for key in ("grad_scalings", "path_emission"):
+        assert np.array_equal(out[key], np.repeat(one[key][:1], 153, axis=0)), key
