@@ -1084,9 +1084,14 @@ __device__ __forceinline__ void chain_exact(const WideRead<kCk>& w, int tid, int
 }
 
 // ---- grid engine
+// The trim cell (k = -1) of event e: (float)(lp_trim * (e + 1)) (GPU/align_cuda.cl:431-443).
+__device__ __forceinline__ float trim_score(const GlobalConsts& g, int e) {
+    return __double2float_rn(__dmul_rn(g.lp_trim, (double)(e + 1)));
+}
+
 // E: a chunk's candidate parts (grid_pair) for thread t's slots into ring slot s.
-// chunk_mode keeps such chunks inside the read: every slot of the window has a k-mer and
-// its four events.
+// chunk_mode sees to it that every slot of the window has a k-mer and its four events,
+// but for (edge_chunk) k-mer -1 and events past the read's last.
 template <bool kLow>
 __device__ __forceinline__ void grid_chunk(WideSmem& ws, const float4* km4, const float* ev, const Grid& G, int t, int s,
                                            int b0, int kp) {
@@ -1108,6 +1113,53 @@ __device__ __forceinline__ void grid_chunk(WideSmem& ws, const float4* km4, cons
     }
 }
 
+// The same on a band that has lost the path, at the read's edges: the adaptive band of a
+// read whose scalings are off follows the trim cells (k-mer -1, the cheapest way through
+// the events) to the last event, then the first invalid event (n_events, its lower left
+// cell) through the k-mers.
+// Such bands took 437 cycles each on the exact engine, now 160-185 (20,000 bands).
+//   The trim cell is the up candidate of the one before it: their difference is a float
+// (two neighbours' within a factor of two), and so is their sum; its other two candidates
+// come from -inf.  A cell past the last event gets parts of -inf: its score is -inf, its
+// left neighbour's event is the same.
+__device__ __forceinline__ bool edge_chunk(int b0, int kp, int n_events) {
+    return kp < 0 || b0 + kWideChunk - 3 - kp > n_events - 1;
+}
+template <bool kLow>
+__device__ __forceinline__ void grid_chunk_edge(WideSmem& ws, const float4* km4, const float* ev, const Grid& G,
+                                                const GlobalConsts& g0, int n_events, int t, int s, int b0, int kp) {
+    int kk[kPerLane];
+    float4 km[kPerLane];
+    float x[kPerLane][kWideChunk];
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) {
+        kk[i] = kp + ((kPerLane * t + i - kp) & (kSlots - 1));
+        km[i] = km4[max(kk[i], 0)];
+#pragma unroll
+        for (int q = 0; q < kWideChunk; ++q) x[i][q] = ev[min(b0 - 2 - kk[i] + q, n_events - 1)];
+    }
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) {
+        float2 g[kWideChunk];
+#pragma unroll
+        for (int q = 0; q < kWideChunk; ++q) g[q] = grid_pair<kLow>(x[i][q], km[i].x, km[i].y, km[i].z, km[i].w, G);
+        if (kk[i] < 0) {  // one thread
+            float last = trim_score(g0, b0 - 2);
+#pragma unroll
+            for (int q = 0; q < kWideChunk; ++q) {
+                const float next = trim_score(g0, b0 - 1 + q);
+                g[q].x = g[q].y = __fsub_rn(next, last);
+                last = next;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kWideChunk; ++q) {
+            if (b0 - 2 - kk[i] + q >= n_events) g[q].x = g[q].y = -INFINITY;
+            ws.x[s][q][kPerLane * t + i] = g[q];
+        }
+    }
+}
+
 // The grid for a band's scores (its row of the ring; 0: none), the same in every warp:
 // the binade of the largest one, when the smallest is at most 4 times it.  It serves
 // chunks that end up to 68 bands on, whose scores are above -38 * 2^m (-50 * 2^m when a
@@ -1125,12 +1177,13 @@ __device__ __forceinline__ int grid_of(const float* row, int lane, uint32_t mode
 static_assert(kWideChunk * (kGridRing + 2 * kGridGroups) <= 68, "bands from the one that decides a grid to the chunk's last");
 
 // Grid `want` for the chunk of bands b0 .. b0 + 3 if the 128-slot window at the placement
-// kp of a band up to 28 bands before its last lies inside the read with every event of
-// the chunk (so do the chunk's cells, none of them the trim cell or on the last k-mer
-// column); else 0.
-__device__ __forceinline__ int chunk_mode(int want, int kp, int b0, int n_events, int n_kmers) {
-    const bool in = kp >= 0 && kp <= n_kmers - kSlots && b0 - 1 - kSlots - kp >= 0 &&
-                    b0 + kWideChunk - 3 - kp <= n_events - 1;
+// kp of a band up to 28 bands before its last has its k-mers in the read (or its first is
+// the trim cell's; none of the chunk's cells lies on the last k-mer column) and no event
+// before the first; else 0.  Events past the last one are only the lower left cell's of a
+// band (e0 <= n_events holds where a run of chunks begins, and a band with such a cell
+// moves right).
+__device__ __forceinline__ int chunk_mode(int want, int kp, int b0, int n_kmers) {
+    const bool in = kp >= -1 && kp < n_kmers - kSlots && b0 - 1 - kSlots - kp >= 0;
     return in ? want : 0;
 }
 
@@ -1173,7 +1226,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
                 if (jr >= ws.exit) break;
                 kp = ws.kb[(br + kWideChunk - 1) & (kScoreRing - 1)] >> 2;
             }
-            const int mode = chunk_mode(want, kp, b0, n_events, n_kmers);
+            const int mode = chunk_mode(want, kp, b0, n_kmers);
             if (closes) {
                 const float2 sk = ws.skip[jr & (kHeadRing - 1)];
                 if (turn & 1) want = grid_of(ws.sc[(br + 3) & (kScoreRing - 1)], lane, modes);
@@ -1199,6 +1252,13 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
                         up = v;
                         left = row[tl];
                     }
+                    if (br + 1 - kp >= n_events) {  // a cell past the last event has no move
+                        for (int q = 0; q < kWideChunk; ++q) {
+                            const float* v = ws.sc[(br & (kScoreRing - 1)) + q] + kPerLane * t;
+                            if (v[0] == -INFINITY) w0 &= ~(0xffu << (8 * q));
+                            if (v[1] == -INFINITY) w1 &= ~(0xffu << (8 * q));
+                        }
+                    }
                     store_tile(jr, w0, w1);
                     w.store_origins(jr, t);
                 }
@@ -1213,7 +1273,12 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
             if (mode) {
                 if (mode != g_mode) G = make_grid(cc, mode);
                 g_mode = mode;
-                if (mode < kGridWide)
+                if (edge_chunk(b0, kp, n_events)) {
+                    if (mode < kGridWide)
+                        grid_chunk_edge<true>(ws, km4, ev, G, a.g, n_events, t, s, b0, kp);
+                    else
+                        grid_chunk_edge<false>(ws, km4, ev, G, a.g, n_events, t, s, b0, kp);
+                } else if (mode < kGridWide)
                     grid_chunk<true>(ws, km4, ev, G, t, s, b0, kp);
                 else
                     grid_chunk<false>(ws, km4, ev, G, t, s, b0, kp);
@@ -1230,9 +1295,10 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
     }
 
     // ------------------------------------------------ B: the chain
-    // Every cell of the chunks' bands is computed (100 per band) and finite when the first
-    // band's predecessors are (checked on entry): a cell has its up neighbour or, at the
-    // band's new right end, its left one.  No score exceeds those before it, E bounds how
+    // Every cell of the chunks' bands is computed (100 per band; 99 when the lower left one
+    // lies past the last event and is -inf) and finite when the first band's predecessors
+    // are (checked on entry): a cell has its up neighbour or, at the band's new right end,
+    // its left one.  No score exceeds those before it, E bounds how
     // far they fall, and a NaN in a cell reaches the next band (its own slot's up candidate
     // or, where the slot left the band, its right neighbour's skip): so the scores that a
     // chunk ends with show a failed proof.
@@ -1272,14 +1338,17 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
 #pragma unroll
             for (int i = 0; i < kPerLane; ++i) {
                 const int o = (kPerLane * t + i - k0) & (kSlots - 1);
-                const bool valid = o < kBand;
-                const int kk = k0 + (valid ? o : 0);  // the chunk's bands lie inside the read
+                // all of the band but the trim cell and a cell past the last event, both of
+                // them its first; the others compute its second
+                const bool trim = o == 0 && k0 < 0, past = o == 0 && b - 2 - k0 >= n_events;
+                const bool valid = o < kBand && !trim && !past;
+                const int kk = k0 + (valid ? o : 1);
                 const int64_t ko = r.km_off + kk;
                 const SlowCell c = slow_cell_call(lp[i], s1[i], left[i], a.ev_mean[r.ev_off + (b - 2 - kk)], a.km_gm[ko],
                                                   a.km_sd[ko], a.km_k1[ko], cc.lp_step, cc.lp_stay, cc.lp_skip);
                 lp[i] = left[i];
-                s1[i] = valid ? c.best : -INFINITY;
-                word[i] |= (valid ? c.from : 0u) << (8 * q);
+                s1[i] = valid ? c.best : trim && !past ? trim_score(a.g, b - 2 - k0) : -INFINITY;
+                word[i] |= (valid ? c.from : trim && !past ? ABEA_FROM_U : 0u) << (8 * q);
                 slow += valid ? 1 : 0;
             }
             *reinterpret_cast<float2*>(&ws.sc[b & (kScoreRing - 1)][kPerLane * t]) = make_float2(s1[0], s1[1]);
@@ -1330,7 +1399,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
                     if (fl) return true;
                     if (pend) release(s == 0 ? kGridRing - 1 : s - 1);  // chunk j - 1 stands
                 }
-                const bool right = ll < ur;  // both ends are finite
+                const bool right = ll < ur;  // the upper right end is finite
                 const uint32_t vr = vs - kOne;
 #pragma unroll
                 for (int i = 0; i < kPerLane; ++i) {
@@ -1388,10 +1457,13 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
         }
         // the start: the scores finite in the band and within the grid's range
         const float top = -pow2f(m), bot = -pow2f(m + 4);
+        const int past = kWideChunk * j - 3 - k0 >= n_events ? 1 : 0;  // the first cell is none
         bool bad = !(max_nan(max3_nan(s1[0], s1[1], lp[0]), lp[1]) < top);
 #pragma unroll
-        for (int i = 0; i < kPerLane; ++i)
-            bad |= (((uint32_t)(kPerLane * t + i - k0) << 25 < kIn) & !(s1[i] >= bot)) | ((lp[i] < bot) & (lp[i] > -INFINITY));
+        for (int i = 0; i < kPerLane; ++i) {
+            const int o = (kPerLane * t + i - k0) & (kSlots - 1);
+            bad |= ((o >= past) & (o < kBand) & !(s1[i] >= bot)) | ((lp[i] < bot) & (lp[i] > -INFINITY));
+        }
         if (named_bar_any(kBarChain, kTeam, bad)) {
             redo(j, 4 * k0);
             release(s);
@@ -1460,9 +1532,9 @@ __device__ __noinline__ void fill_chain(const CoreArgs& a, const ReadDesc& r, un
         // the grid engine, if its chunks can begin here and there is room for a run
         const int b0 = kWideChunk * j, kp = ws.kb[(b0 - 1) & (kScoreRing - 1)] >> 2;
         const int first = grid_of(ws.sc[(b0 - 1) & (kScoreRing - 1)], lane, modes);
-        const bool room = chunk_mode(1, kp + 40, b0 + 2 * 40, w.n_events, w.n_kmers);
+        const bool room = kp >= -1 && b0 - 3 - kp <= w.n_events && chunk_mode(1, kp + 40, b0 + 2 * 40, w.n_kmers);
         seg = kp < 0 || kp + 40 <= w.n_kmers - kSlots ? retry : w.n_chunks;  // near the end: to the end
-        if (first && room && chunk_mode(first, kp, b0, w.n_events, w.n_kmers)) {
+        if (first && room && chunk_mode(first, kp, b0, w.n_kmers)) {
             chain_grid<kScores>(w, tid, j, first, modes);
             __syncthreads();
             j = ws.exit;

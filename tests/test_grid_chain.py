@@ -81,3 +81,32 @@ def test_outlier_events(oracle_mod, value, shape):
     for at in (700, 1500, 1501, 2600, len(ev) - 40):
         ev["mean"][at] = value
     check(oracle_mod, batch_of(model, [(seq, ev)]), shape)
+
+
+@pytest.mark.parametrize("shape", ["wide", "warp"])
+@pytest.mark.parametrize("mean_events", [1.05, 1.8, 4.0])
+def test_bands_at_the_edges_of_a_read(oracle_mod, mean_events, shape):
+    """Bands that lose the path: scalings off (the band follows the trim cells through the
+    events, then the last event through the k-mers, and on the way is done again for events
+    far out), and reads with 700 events or bases that do not belong to them at either end."""
+    from abea_gb300 import synth
+    rng = np.random.default_rng(14)
+    model, _, _ = make(rng, 50)
+    reads, scale = [], []
+    for length, s in ((300, 1.1), (420, 0.9), (1203, 1.06), (2501, 1.1), (2502, 0.7), (2503, 1.5), (1900, 1.02)):
+        seq, ev = synth.make_read(rng, model, length, 1.02, 2.0, 1.2, skip_p=0.01, mean_events=mean_events)
+        reads.append((seq.tobytes(), ev))
+        scale.append(s)
+    seq, ev = reads[3][0], reads[3][1].copy()
+    for at, value in ((900, np.inf), (1201, 1e30), (1300, -1e5), (1777, 4000.0), (len(ev) - 1, 4000.0), (len(ev) - 2, -np.inf)):
+        ev["mean"][at] = value
+    reads.append((seq, ev))
+    scale.append(1.1)
+    seq, ev = reads[6]
+    junk, junk_ev = synth.make_read(rng, model, 500, 1.02, 2.0, 1.2, skip_p=0.01, mean_events=1.8)
+    reads += [(seq, np.concatenate([ev, junk_ev[:700]])), (seq, np.concatenate([junk_ev[:700], ev])),
+              (seq + junk.tobytes(), ev), (junk.tobytes() + seq, ev)]
+    scale += [1.02] * 4
+    batch = batch_of(model, reads)
+    batch.scalings["scale"] = scale
+    check(oracle_mod, batch, shape)
