@@ -1036,18 +1036,32 @@ __device__ __forceinline__ void chain_exact(const WideRead<kCk>& w, int tid, int
             from = here ? (tv == -INFINITY ? 0u : ABEA_FROM_U) : from;
             ws.sc[r0 + q][t] = best;  // stored before the check: only the rare path stores again
             if (__any_sync(kFull, bad)) {
-                // Rare: a proof failed in some lane, whose cell takes the reference's
-                // FP64 arithmetic and stores its score again.  The whole warp calls (a
-                // divergent branch around the call cost 20 cycles per band); the other
-                // lanes pass k-mer 0 and event 0 of the read, which exist because the
-                // bad lane's cell does, and drop the result.
-                const int64_t ko = r.km_off + (bad ? k0 + o : 0);
-                const SlowCell c = slow_cell_call(lp, s1, left, a.ev_mean[r.ev_off + (bad ? e0 - o : 0)], a.km_gm[ko],
-                                                  a.km_sd[ko], a.km_k1[ko], w.cc.lp_step, w.cc.lp_stay, w.cc.lp_skip);
-                const bool use = bad && !here;
-                best = use ? c.best : best;
-                from = use ? c.from : from;
-                slow += use ? 1 : 0;
+                // A proof failed in some lane: in a read's first bands, three of four, where
+                // an emission far below its score was added to it (Fast2Sum's condition).
+                // TwoSum proves those; with FP64 for them all, the first 800 bands of a read
+                // took 710 cycles each and a read of 1 kb 760 us, now 620.
+                const bool redo = bad && !here;
+                bool okd2, oku2;
+                const float d2 = exact_from_split<true>(lp, EmSplit{ep.x, ep.z}, mm.x, okd2);
+                const float u2 = exact_from_split<true>(s1, EmSplit{ep.y, ep.w}, mm.y, oku2);
+                uint32_t from_du2, from2;
+                const float best_du2 = pick_du(d2, u2, from_du2);
+                const float best2 = pick_l(best_du2, from_du2, l, from2);
+                best = redo ? best2 : best;
+                from = redo ? from2 : from;
+                slow += redo ? 1 : 0;
+                const bool still = redo && !(okd2 && oku2 && okl);
+                if (__any_sync(kFull, still)) {
+                    // Rare: the lane's cell takes the reference's FP64 arithmetic.  The whole
+                    // warp calls (a divergent branch around the call cost 20 cycles per
+                    // band); the other lanes pass k-mer 0 and event 0 of the read, which
+                    // exist because the lane's cell does, and drop the result.
+                    const int64_t ko = r.km_off + (still ? k0 + o : 0);
+                    const SlowCell c = slow_cell_call(lp, s1, left, a.ev_mean[r.ev_off + (still ? e0 - o : 0)], a.km_gm[ko],
+                                                      a.km_sd[ko], a.km_k1[ko], w.cc.lp_step, w.cc.lp_stay, w.cc.lp_skip);
+                    best = still ? c.best : best;
+                    from = still ? c.from : from;
+                }
                 ws.sc[r0 + q][t] = best;
             }
             word |= from << (8 * q);
