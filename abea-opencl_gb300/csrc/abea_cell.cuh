@@ -211,16 +211,19 @@ __device__ __forceinline__ EmSplit em_split(float em, float bh, float bl) {
 // ok = false when not proven.  As in exact_skip, the error terms come from
 // ac = max(a, -FLT_MAX): for a = -inf, s = -inf gives hp = hm = -inf when mag
 // is finite, and NaN (not proven) when it is not.
+// kAny: TwoSum, whichever of a and p is larger (Fast2Sum needs |a| >= |p|).
+template <bool kAny = false>
 __device__ __forceinline__ float exact_from_split(float a, EmSplit sp, float mag, bool& ok) {
     const float ac = fmaxf(a, -FLT_MAX);
     const float s = __fadd_rn(a, sp.p);
     const float sc = __fadd_rn(ac, sp.p);
-    const float e = __fsub_rn(sp.p, __fsub_rn(sc, ac));
+    const float bb = __fsub_rn(sc, ac);
+    const float e = kAny ? __fadd_rn(__fsub_rn(ac, __fsub_rn(sc, bb)), __fsub_rn(sp.p, bb)) : __fsub_rn(sp.p, bb);
     const float t = __fadd_rn(e, sp.w);
     const float eb = __fmul_rn(__fadd_rn(fabsf(ac), mag), kErrScale);
     const float hp = __fadd_rn(s, __fadd_rn(t, eb));
     const float hm = __fadd_rn(s, __fsub_rn(t, eb));
-    ok = (hp == hm) && (fabsf(a) >= fabsf(sp.p));
+    ok = (hp == hm) && (kAny || fabsf(a) >= fabsf(sp.p));
     return hp;
 }
 
