@@ -168,7 +168,7 @@ struct abea_ctx {
     char* h_aux = nullptr;  // pinned: abea_align_batch's mirrors, then its counters and statuses
     size_t h_aux_bytes = 0;
     std::map<uint64_t, int64_t> tuned;      // autotuned wide-shape threshold per workload signature
-    std::map<uint64_t, int64_t> tuned_mid;  // autotuned medium-shape threshold per workload signature
+    std::map<uint64_t, int64_t> tuned_mid;  // second wide threshold per workload signature, from a cache file
 };
 
 // ---------------------------------------------------------------- context
@@ -723,8 +723,8 @@ static abea_status_t queue_work(abea_ctx* c, abea_batch* b, int* launches, bool 
 }
 
 // The batched form's order: wide reads (threshold from the option, else the
-// autotuned value of this workload signature, else the heuristic), medium reads
-// (threshold from the option, else the autotuned value, else none), then the rest.
+// autotuned value of this workload signature, else the heuristic; and a second one from
+// the option, else from a cache file, else none), then the rest.
 static void prepare_order(abea_ctx* c, abea_batch* b) {
     b->n_wide = 0;
     if (c->mode != ABEA_MODE_BATCHED) return;
@@ -819,7 +819,7 @@ extern "C" abea_status_t abea_autotune(abea_ctx_t* c, abea_batch_t* b, int64_t* 
     const abea_mode_t mode0 = c->mode;
     const int64_t thr0 = c->long_read_bands, mid0 = c->mid_read_bands;
     c->mode = ABEA_MODE_BATCHED;
-    // without a medium threshold: neither the option's nor one from a cache file may
+    // without a second threshold: neither the option's nor one from a cache file may
     // shape the timings
     c->mid_read_bands = INT64_MAX;
     const int blocks = batched_blocks_per_sm(b->scores_kept) * c->sm_count;
@@ -872,7 +872,7 @@ extern "C" abea_status_t abea_autotune(abea_ctx_t* c, abea_batch_t* b, int64_t* 
 }
 
 // Autotuner cache: "abea-autotune 2 sm_count <n>" then "<signature> <wide threshold>
-// <medium threshold>" lines (INT64_MAX = none).  Version 1 files (no medium
+// <second threshold>" lines (INT64_MAX = none).  Version 1 files (no second
 // threshold) are read too.
 extern "C" abea_status_t abea_autotune_save(abea_ctx_t* c, const char* path, int32_t* n_entries) {
     if (!c || !path) return fail(ABEA_ERR_INVALID_ARG, "abea_autotune_save: null argument");

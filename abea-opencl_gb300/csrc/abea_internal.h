@@ -66,7 +66,8 @@ struct ReadDesc {
 // every band b = s*kCkBands (s >= 1) the fill stores the state it resumes from
 // (band b-1's scores, band b-2's scores shifted by one slot, band b-1's
 // placement) as one record of kCkStride floats; the traceback recomputes the
-// trace of one kCkBands-band segment at a time into a scratch slot.
+// trace of one kCkBands-band segment at a time into a scratch slot (a wide read's
+// block sixteen at a time into its traceback map's memory).
 constexpr int kCkBands = 256;
 constexpr int kCkStride = 264;  // 128 + 128 scores, k0, e0, padding to 16 bytes
 

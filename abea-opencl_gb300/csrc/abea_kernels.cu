@@ -496,6 +496,8 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
     // same conditions and the same end-of-chunk check as the wide shape's grid engine; a
     // chunk that fails it runs again in the exact loop below.  Not unrolled over the bands:
     // the loop body stays small (up to sixteen warps on an SM, each at its own place).
+    // A read of 20 kb alone: 1,050 cycles per band before, 530 now (the plain form's f5c
+    // batch 33.4 -> 17.5 ms); sixteen warps on an SM 131 together.
     //   grid: the grid in use until band grid_until; grid_from: the first band that may try.
     const uint32_t modes = grid_modes(cc);
     const float k1_max = grid_k1_max(cc.step_h, cc.stay_h);
@@ -768,19 +770,20 @@ constexpr int kExactRing = 4, kExactGroups = 2;
 constexpr int kBarChain = 1, kBarFull = 2, kBarExEmpty = 2 + kExactRing;
 static_assert(kExactRing % kExactGroups == 0, "each ring slot, and its two barriers, belongs to one E group");
 
-// Grid engine.  B = warps 0 and 1, two slots per thread, E = five groups of two warps:
-// the warps w with w & 2, and warps 4 and 5.  A warp runs on scheduler (w & 3) of the SM,
-// so B shares its two with one group only.  Measured on a bare chain, cycles per band: 87
+// Grid engine.  B = warps 0 and 1, two slots per thread, E = four groups of two warps:
+// the warps w with w & 2.  A warp runs on scheduler (w & 3) of the SM, so B has its two to
+// itself; with a fifth group there (warps 4 and 5) a read of 20 kb took 5.2-5.4 ms, now
+// 5.0.  Measured on a bare chain, cycles per band: 87
 // with four B warps alone and 134 with E's load on every scheduler; 94 with two, whatever
 // runs on the other two schedulers; 141 with one warp of four slots per lane.
-//   Named barriers: 1 = B's per-band barrier, 2 + g = E group g's own, 7 + s = EMPTY[s]: B
+//   Named barriers: 1 = B's per-band barrier, 2 + g = E group g's own, 6 + s = EMPTY[s]: B
 // has released the chunk of ring slot s (B arrives, the group of the slot's next chunk
 // waits; fewer groups than slots, so no two wait on one).  The other way round a header
 // in shared memory tells B that a chunk is made: a barrier there costs the chain 68 cycles
 // per chunk, a reduction of the failed checks (bar.red) 78; a header read a chunk ahead
 // and a flag word next to nothing.
 constexpr int kGridRing = 7;        // chunks in the ring
-constexpr int kGridGroups = 5;
+constexpr int kGridGroups = 4;
 constexpr int kPerLane = 2;         // slots per thread of B and of E
 constexpr int kTeam = kSlots / kPerLane;  // threads of B, and of an E group
 constexpr int kPair = 2 * kTeam;          // B and one E group on EMPTY
@@ -1207,7 +1210,7 @@ __device__ __forceinline__ int chunk_mode(int want, int kp, int b0, int n_kmers)
 template <bool kScores, bool kCk>
 __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int j0, int first, uint32_t modes) {
     const int warp = tid >> 5, lane = tid & 31;
-    if ((warp & 3) < 2 && warp >= 6) return;
+    if ((warp & 3) < 2 && warp >= 2) return;
     WideSmem& ws = w.ws;
     const ReadDesc& r = w.r;
     const CoreArgs& a = w.a;
@@ -1226,7 +1229,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
 
     if (warp >= 2) {
         // ------------------------------------------------ E: closes chunk j - kGridRing and makes chunk j
-        const int group = warp & 2 ? warp >> 2 : kGridGroups - 1;
+        const int group = warp >> 2;
         const float4* km4 = a.km4 + r.km_off;
         const float* ev = a.ev_mean + r.ev_off;
         Grid G{};
@@ -1388,13 +1391,15 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
         char* const sc = reinterpret_cast<char*>(&ws.sc[0][0]);
         constexpr int kRow = 4 * kSlots, kRows = kScoreRing * kRow;
         int rw = (kWideChunk * j * kRow) & (kRows - 1);  // byte offset of the chunk's first score row
+        int row0 = (rw - kRow) & (kRows - 1);            // and of the row before it
         while (true) {
             kb_cur = kb;
             int fl = 0, head = 0;
+            bool leave = false;
 #pragma unroll
             for (int q = 0; q < kWideChunk; ++q) {
                 if (q > 0) named_bar_sync(kBarChain, kTeam);
-                const char* row = sc + (q > 0 ? rw + (q - 1) * kRow : (rw - kRow) & (kRows - 1));
+                const char* row = sc + (q > 0 ? rw + (q - 1) * kRow : row0);
                 const float ll = *reinterpret_cast<const float*>(row + (kb & (kRow - 4)));
                 const float ur = *reinterpret_cast<const float*>(row + ((kb + 4 * (kBand - 1)) & (kRow - 4)));
                 const float left[kPerLane] = {*reinterpret_cast<const float*>(row + 4 * tl), s1[0]};
@@ -1410,8 +1415,16 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
                     head = *(volatile int32_t*)&ws.head[(j + 1) & (kHeadRing - 1)];
                 }
                 if (q == 2) {
-                    if (fl) return true;
+                    if (__any_sync(kFull, fl != 0)) return true;
                     if (pend) release(s == 0 ? kGridRing - 1 : s - 1);  // chunk j - 1 stands
+                }
+                if (q == 3) {
+                    // chunk j + 1, usually made by now; both warps leave on another grid
+                    if (__any_sync(kFull, head >> 5 != j + 2)) {
+                        for (int i = 0; head >> 5 != j + 2 && i < kReadyPolls; ++i)
+                            head = *(volatile int32_t*)&ws.head[(j + 1) & (kHeadRing - 1)];
+                    }
+                    leave = __any_sync(kFull, head != chunk_head(j + 1, g_mode));
                 }
                 const bool right = ll < ur;  // the upper right end is finite
                 const uint32_t vr = vs - kOne;
@@ -1435,13 +1448,11 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
             kb_pend = kb_cur;
             ++j;
             s = s + 1 == kGridRing ? 0 : s + 1;
+            row0 = rw + (kWideChunk - 1) * kRow;
             rw = (rw + kWideChunk * kRow) & (kRows - 1);
             if (kLow && below) ws.flag = 2;  // (for the check when the run ends here)
-            // chunk j, usually made by now; both warps leave on another grid
-            for (int i = 0; head >> 5 != j + 1 && i < kReadyPolls; ++i)
-                head = *(volatile int32_t*)&ws.head[j & (kHeadRing - 1)];
             named_bar_sync(kBarChain, kTeam);
-            if (head != chunk_head(j, g_mode)) {
+            if (leave) {
                 k0 = kb >> 2;
                 return false;
             }
