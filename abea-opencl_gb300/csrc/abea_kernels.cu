@@ -1559,7 +1559,11 @@ __device__ __noinline__ void fill_chain(const CoreArgs& a, const ReadDesc& r, un
         const int first = grid_of(ws.sc[(b0 - 1) & (kScoreRing - 1)], lane, modes);
         const bool room = kp >= -1 && b0 - 3 - kp <= w.n_events && chunk_mode(1, kp + 40, b0 + 2 * 40, w.n_kmers);
         seg = kp < 0 || kp + 40 <= w.n_kmers - kSlots ? retry : w.n_chunks;  // near the end: to the end
-        if (first && room && chunk_mode(first, kp, b0, w.n_kmers)) {
+        const bool enter = first && room && chunk_mode(first, kp, b0, w.n_kmers);
+        // Every warp has decided before the chain may overwrite what they decided from: the
+        // warps that the chain leaves idle never wait for it, and all must go the same way.
+        __syncthreads();
+        if (enter) {
             chain_grid<kScores>(w, tid, j, first, modes);
             __syncthreads();
             j = ws.exit;

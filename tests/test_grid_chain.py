@@ -110,3 +110,30 @@ def test_bands_at_the_edges_of_a_read(oracle_mod, mean_events, shape):
     batch = batch_of(model, reads)
     batch.scalings["scale"] = scale
     check(oracle_mod, batch, shape)
+
+
+def test_many_entries_into_the_grid_chain(oracle_mod):
+    """More reads than SMs, each with an event far out every few hundred, so that every
+    block enters and leaves the grid chain time and again with all SMs at work: the whole
+    block has to take each of these decisions alike."""
+    from abea_gb300 import synth
+    rng = np.random.default_rng(15)
+    model, _, _ = make(rng, 50)
+    reads = []
+    for i in range(200):
+        seq, ev = synth.make_read(rng, model, 2000 + 7 * i, 1.02, 2.0, 1.2, skip_p=0.01, mean_events=1.8)
+        ev = ev.copy()
+        ev["mean"][700 + i::150 + i] = 4000.0
+        reads.append((seq.tobytes(), ev))
+    batch = batch_of(model, reads)
+    ctx = abea.Context(0, abea.MODE_BATCHED)
+    ctx.set_option(abea.OPT_LONG_READ_BANDS, 1)
+    dev = ctx.upload(batch)
+    opairs, ocounts, obest = oracle_mod.align_batch(batch, threads=8)
+    for _ in range(3):
+        dev.run()
+        pairs, counts = dev.results()
+        assert np.array_equal(counts, ocounts)
+        for got, exp in zip(abea.split_pairs(batch, pairs, counts), abea.split_pairs(batch, opairs, ocounts)):
+            assert np.array_equal(got, exp)
+        assert np.array_equal(dev.best_scores().view(np.uint32), obest.view(np.uint32))
