@@ -767,6 +767,7 @@ static abea_status_t run_batch(abea_ctx* c, abea_batch* b) {
         std::vector<uint64_t> key = b->carve;
         key.push_back((uint64_t)b->n_reads);
         key.push_back((uint64_t)b->n_wide);
+        key.push_back((uint64_t)c->spin_limit);
         key.push_back((uint64_t)(b->scores_kept ? 1 : 0) | ((uint64_t)b->var_aware << 1) |
                       ((uint64_t)(c->wide_cluster != 0) << 2));
         if (!b->graph || key != b->graph_key) {

@@ -781,14 +781,18 @@ static_assert(kExactRing % kExactGroups == 0, "each ring slot, and its two barri
 // waits; fewer groups than slots, so no two wait on one).  The other way round a header
 // in shared memory tells B that a chunk is made: a barrier there costs the chain 68 cycles
 // per chunk, a reduction of the failed checks (bar.red) 78; a header read a chunk ahead
-// and a flag word next to nothing.
+// and a flag word next to nothing.  B's polls of a header are bounded by the spin limit:
+// when it runs out the run reports a timeout and the read is given up (`dead`), B going on
+// with a fixed bound until it can leave in step with E, whose turn by then waits for nothing
+// but its own work.  (E polling a word for the released chunks in place of EMPTY costs 8% of
+// a long read: its turns bound the chain.)
 constexpr int kGridRing = 7;        // chunks in the ring
 constexpr int kGridGroups = 4;
 constexpr int kPerLane = 2;         // slots per thread of B and of E
 constexpr int kTeam = kSlots / kPerLane;  // threads of B, and of an E group
 constexpr int kPair = 2 * kTeam;          // B and one E group on EMPTY
 constexpr int kBarGroup = 2, kBarEmpty = 2 + kGridGroups;
-constexpr int kReadyPolls = 1 << 22;      // B's polls of a header before it gives up
+constexpr int kReadyPolls = 1 << 22;      // B's polls of a header after the spin limit's
 static_assert(kWideChunk * kGridRing <= kSlots - kBand && kWideChunk * kExactRing <= kSlots - kBand,
               "E's k-mer window must hold the chunk's bands");
 static_assert(kBarEmpty + kGridRing <= 16 && kBarExEmpty + kExactRing <= 16, "named barriers 0-15");
@@ -818,6 +822,7 @@ struct alignas(16) WideSmem {
     float2 skip[kHeadRing];         // {the grid's skip part, 1: B has stored its backpointers and origins}
     int32_t flag;                   // a failed check
     int32_t exit, failing;          // the first chunk not done; failures made it leave
+    int32_t dead;                   // a wait ran out of polls
 };
 __device__ __forceinline__ int chunk_head(int j, int mode) { return (j + 1) << 5 | mode; }  // never 0
 static_assert(kGridMax < 32, "five bits of mode");
@@ -1376,6 +1381,18 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
         w.store_origins(j, t);
         if (t == 0) ws.skip[j & (kHeadRing - 1)].y = 1.0f;
     };
+    // Chunk j's header, once it is made.
+    auto header = [&](int j) {
+        volatile int32_t* at = &ws.head[j & (kHeadRing - 1)];
+        int h = *at;
+        for (long long i = 0; h >> 5 != j + 1 && i < a.spin_limit; ++i) h = *at;
+        if (h >> 5 != j + 1) {
+            ws.dead = 1;
+            if (lane == 0) atomicAdd(&a.counters[2], 1ull);  // the run reports a timeout
+            for (int i = 0; h >> 5 != j + 1 && i < kReadyPolls; ++i) h = *at;
+        }
+        return h;
+    };
     // Runs chunks from chunk j (made, its start checked, every warp past a barrier after
     // band 4j-1) until one that has another grid or none, or a failed check; j is then that
     // chunk.  true: the check of chunk j-1 failed (and chunk j has begun).  The last barrier
@@ -1420,10 +1437,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
                 }
                 if (q == 3) {
                     // chunk j + 1, usually made by now; both warps leave on another grid
-                    if (__any_sync(kFull, head >> 5 != j + 2)) {
-                        for (int i = 0; head >> 5 != j + 2 && i < kReadyPolls; ++i)
-                            head = *(volatile int32_t*)&ws.head[(j + 1) & (kHeadRing - 1)];
-                    }
+                    if (__any_sync(kFull, head >> 5 != j + 2)) head = header(j + 1);
                     leave = __any_sync(kFull, head != chunk_head(j + 1, g_mode));
                 }
                 const bool right = ll < ur;  // the upper right end is finite
@@ -1458,21 +1472,13 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
             }
         }
     };
-    // chunk j's header, once it is made
-    auto header = [&](int j) {
-        int h = *(volatile int32_t*)&ws.head[j & (kHeadRing - 1)];
-        for (int i = 0; h >> 5 != j + 1 && i < kReadyPolls; ++i) h = *(volatile int32_t*)&ws.head[j & (kHeadRing - 1)];
-        return h;
-    };
     restore(j0, 4 * k_start);
     int j = j0, s = 0;
     while (true) {
         // chunk j's header; also the barrier after band 4j-1
         const int h = header(j);
-        const bool late = h >> 5 != j + 1;
-        if (late && t == 0) atomicAdd(&a.counters[2], 1ull);  // the run reports a timeout
         __threadfence_block();
-        const int m = named_bar_any(kBarChain, kTeam, late) ? 0 : h & 31;
+        const int m = named_bar_any(kBarChain, kTeam, *(volatile int32_t*)&ws.dead != 0) ? 0 : h & 31;
         if (m == 0 || pen > 32) break;
         if (m != g_mode) {
             bool ok;
@@ -1522,10 +1528,11 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
     if (slow) atomicAdd(&a.counters[0], slow);
 }
 
-// One read's fill.  `grids`: the read's k-mers allow grids (grid_kmer_ok).  A call, as
+// One read's fill; false when a wait ran out of polls: the read is given up, the rest of it
+// not filled.  `grids`: the read's k-mers allow grids (grid_kmer_ok).  A call, as
 // fill_warp_ck is: each has the block's registers to itself.
 template <bool kScores, bool kCk>
-__device__ __noinline__ void fill_chain(const CoreArgs& a, const ReadDesc& r, unsigned ws_at, int tid, bool grids) {
+__device__ __noinline__ bool fill_chain(const CoreArgs& a, const ReadDesc& r, unsigned ws_at, int tid, bool grids) {
     WideSmem& ws = smem_ref<WideSmem>(ws_at);
     const int lane = tid & 31;
     WideRead<kCk> w{a, r, ws, make_consts(r, a.g), r.n_events, r.n_kmers, r.n_bands, (r.n_bands + kWideChunk - 1) / kWideChunk,
@@ -1540,7 +1547,10 @@ __device__ __noinline__ void fill_chain(const CoreArgs& a, const ReadDesc& r, un
             w.scores[kSlots + tid] = ws.sc[1][tid];
         }
     }
-    if (tid == 0) ws.kb[0] = ws.kb[1] = ws.kb[kScoreRing - 1] = 4 * (-1 - kBand / 2);
+    if (tid == 0) {
+        ws.kb[0] = ws.kb[1] = ws.kb[kScoreRing - 1] = 4 * (-1 - kBand / 2);
+        ws.dead = 0;
+    }
     __syncthreads();
     int j = 0, seg = kFirstExact, retry = kNextExact;
     while (true) {
@@ -1553,7 +1563,7 @@ __device__ __noinline__ void fill_chain(const CoreArgs& a, const ReadDesc& r, un
             ws.exit = INT32_MAX;
         }
         __syncthreads();
-        if (j >= w.n_chunks) break;
+        if (j >= w.n_chunks) return true;
         // the grid engine, if its chunks can begin here and there is room for a run
         const int b0 = kWideChunk * j, kp = ws.kb[(b0 - 1) & (kScoreRing - 1)] >> 2;
         const int first = grid_of(ws.sc[(b0 - 1) & (kScoreRing - 1)], lane, modes);
@@ -1566,6 +1576,7 @@ __device__ __noinline__ void fill_chain(const CoreArgs& a, const ReadDesc& r, un
         if (enter) {
             chain_grid<kScores>(w, tid, j, first, modes);
             __syncthreads();
+            if (ws.dead) return false;
             j = ws.exit;
             if (ws.failing) retry = min(2 * retry, 1 << 20);
             const int k_end = ws.kb[(kWideChunk * j - 1) & (kScoreRing - 1)] >> 2;
@@ -2791,16 +2802,19 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(const __g
         const ReadDesc& r = a.reads[wide_read];
         const bool odd = pre_read(pa, wide_read, t, kWideThreads);
         const bool grids = !__syncthreads_or(odd);  // the read's parameters are in memory for the whole block
+        bool filled = true;
         if (!r.skip) {
             if (r.ck)
-                fill_chain<kScores, true>(a, r, smem_u32(&sm.wide), t, grids);
+                filled = fill_chain<kScores, true>(a, r, smem_u32(&sm.wide), t, grids);
             else
-                fill_chain<kScores, false>(a, r, smem_u32(&sm.wide), t, grids);
+                filled = fill_chain<kScores, false>(a, r, smem_u32(&sm.wide), t, grids);
         }
         __syncthreads();
         __threadfence_block();
         // the whole block walks the wide read's traceback (the fill's shared memory is free)
-        if (r.ck && !r.skip && wide_slot < a.n_spec)
+        if (!filled) {
+            if (t == 0) post_write(p, wide_read, ABEA_ERR_TIMEOUT, -INFINITY, 0, ABEA_ERR_TIMEOUT, 0, r.out_cap, false, 0);
+        } else if (r.ck && !r.skip && wide_slot < a.n_spec)
             post_ck_block(a, p, wide_read, reinterpret_cast<uint8_t*>(&sm.wide), sm.warp_rings, sm.ended, t,
                           reinterpret_cast<uint8_t*>(a.spec + (int64_t)wide_slot * (kSpecRound * kSpecBands)));
         else

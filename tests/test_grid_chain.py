@@ -137,3 +137,30 @@ def test_many_entries_into_the_grid_chain(oracle_mod):
         for got, exp in zip(abea.split_pairs(batch, pairs, counts), abea.split_pairs(batch, opairs, ocounts)):
             assert np.array_equal(got, exp)
         assert np.array_equal(dev.best_scores().view(np.uint32), obest.view(np.uint32))
+
+
+@pytest.mark.parametrize("budget", [0, 400_000])
+def test_a_wait_out_of_polls_ends_in_a_timeout(oracle_mod, budget):
+    """With a limit of one poll the grid chain's waits give up: the run reports a timeout
+    and returns no alignment, and the next run with the usual limit is the oracle's (the
+    same batch, whose captured graph holds the limit)."""
+    rng = np.random.default_rng(16)
+    model, seq, ev = make(rng, 2400)
+    batch = batch_of(model, [(seq, ev)])
+    ctx = abea.Context(0, abea.MODE_BATCHED)
+    ctx.set_option(abea.OPT_LONG_READ_BANDS, 1)
+    ctx.set_option(abea.OPT_TRACE_BUDGET, budget)
+    limit = ctx.get_option(abea.OPT_SPIN_LIMIT)
+    dev = ctx.upload(batch)
+    op, oc, _ = oracle_mod.align_batch(batch)
+    for _ in range(2):
+        ctx.set_option(abea.OPT_SPIN_LIMIT, 1)
+        with pytest.raises(abea.AbeaError) as e:
+            dev.run()
+            dev.results()
+        assert e.value.status == -5
+        ctx.set_option(abea.OPT_SPIN_LIMIT, limit)
+        dev.run()
+        pairs, counts = dev.results()
+        assert np.array_equal(counts, oc)
+        assert np.array_equal(abea.split_pairs(batch, pairs, counts)[0], abea.split_pairs(batch, op, oc)[0])
