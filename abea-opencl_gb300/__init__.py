@@ -239,6 +239,16 @@ class DeviceBatch:
         _check(lib().abea_batch_slow_cells(self.ctx.h, self.h, C.byref(v)))
         return v.value
 
+    def _counters(self) -> dict:
+        """What the last run counted (abea_internal_counters): band cells whose first FP32
+        proof failed, those computed in FP64, waits out of polls, stores out of bounds
+        (bounds-checked build), tiles of four bands on a grid, those done again."""
+        out = np.zeros(8, dtype=np.int64)
+        f = lib().abea_internal_counters
+        f.argtypes, f.restype = [C.c_void_p] * 3, C.c_int
+        _check(f(self.ctx.h, self.h, _p(out)))
+        return dict(zip(("slow", "fp64", "timeouts", "bounds", "grid", "grid_again"), out.tolist()))
+
     def autotune(self):
         """Picks the wide-shape threshold for this workload (abea_autotune)."""
         thr, ms = C.c_int64(), C.c_float()

@@ -468,7 +468,7 @@ static abea_status_t ensure_device(abea_batch* b, bool scores, size_t reserve = 
         sizeof(int32_t) * n,   // n_pairs
         sizeof(float) * n,     // best
         sizeof(int32_t) * n,   // status
-        sizeof(unsigned long long) * 4,  // slow counter
+        sizeof(unsigned long long) * kCounters,
         sizeof(int32_t) * n,   // order
         sizeof(int32_t) * 8,   // queue counters
         sizeof(int32_t) * n,   // path_len
@@ -717,7 +717,7 @@ static uint64_t workload_signature(const abea_batch* b) {
 }
 
 static abea_status_t queue_work(abea_ctx* c, abea_batch* b, int* launches, bool capturing) {
-    CUDA_TRY(cudaMemsetAsync(b->d_slow, 0, sizeof(unsigned long long) * 4, c->stream));
+    CUDA_TRY(cudaMemsetAsync(b->d_slow, 0, sizeof(unsigned long long) * kCounters, c->stream));
     CUDA_TRY(cudaMemsetAsync(b->d_queue, 0, sizeof(int32_t) * 8, c->stream));
     return launch_all(c, b, launches, capturing);
 }
@@ -972,8 +972,11 @@ static abea_status_t check_status(abea_ctx* c, abea_batch* b, const void* host =
     }
     unsigned long long cnt[4];
     memcpy(cnt, host, sizeof(cnt));
-    if (cnt[2]) return fail(ABEA_ERR_TIMEOUT, "%llu device-side waits ran out of polls (ABEA_OPT_SPIN_LIMIT)", cnt[2]);
-    if (cnt[3]) return fail(ABEA_ERR_INTERNAL, "%llu device-side stores out of their region (bounds-checked build)", cnt[3]);
+    if (cnt[kCountTimeouts])
+        return fail(ABEA_ERR_TIMEOUT, "%llu device-side waits ran out of polls (ABEA_OPT_SPIN_LIMIT)", cnt[kCountTimeouts]);
+    if (cnt[kCountBounds])
+        return fail(ABEA_ERR_INTERNAL, "%llu device-side stores out of their region (bounds-checked build)",
+                    cnt[kCountBounds]);
     const int32_t* st = (const int32_t*)((const char*)host + sizeof(cnt));
     for (int32_t i = 0; i < b->n_reads; ++i)
         if (st[i] != 0) return fail((abea_status_t)st[i], "read %d: %s", i, abea_status_string((abea_status_t)st[i]));
@@ -1062,6 +1065,17 @@ extern "C" abea_status_t abea_batch_slow_cells(abea_ctx_t* c, abea_batch_t* b, i
         CUDA_TRY(cudaStreamSynchronize(c->stream));
     }
     *count = (int64_t)v;
+    return ABEA_OK;
+}
+
+// What the last run counted (Counter, out[kCounters]): for tests.
+extern "C" abea_status_t abea_internal_counters(abea_ctx_t* c, abea_batch_t* b, int64_t* out) {
+    if (!c || !b || !out) return fail(ABEA_ERR_INVALID_ARG, "abea_internal_counters: null argument");
+    std::fill(out, out + kCounters, 0);
+    if (b->n_reads) {
+        CUDA_TRY(cudaMemcpyAsync(out, b->d_slow, sizeof(int64_t) * kCounters, cudaMemcpyDeviceToHost, c->stream));
+        CUDA_TRY(cudaStreamSynchronize(c->stream));
+    }
     return ABEA_OK;
 }
 

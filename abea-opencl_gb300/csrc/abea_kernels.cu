@@ -335,11 +335,11 @@ struct FillSpan {
 
 // Debug builds (ABEA_BOUNDS_CHECK): the global stores of the fill and of the
 // traceback check their index against their region; a store out of it is skipped
-// and counted in counters[3] (the run then reports ABEA_ERR_INTERNAL).
+// and counted (the run then reports ABEA_ERR_INTERNAL).
 #ifdef ABEA_BOUNDS_CHECK
 __device__ __forceinline__ bool in_bounds(int64_t i, int64_t n, unsigned long long* counters) {
     const bool ok = i >= 0 && i < n;
-    if (!ok) atomicAdd(&counters[3], 1ull);
+    if (!ok) atomicAdd(&counters[kCountBounds], 1ull);
     return ok;
 }
 #else
@@ -431,7 +431,7 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
             nc[j] = next_cell(LP[j], rg.ev[(ep[j] + 1) & (kEvRing - 1)], gmv[j], sdv[j], rsv[j], k1v[j], cc);
     }
     int my_k0 = k0;  // bands 0 and 1 (lanes 0, 1) both have k0 = -51
-    unsigned long long slow = 0;
+    unsigned slow = 0;
     const int sl_last = (n_kmers - 1) & 127;
     uint32_t tw0 = 0u, tw1 = (lane == 31 && !sp.ck_in) ? (ABEA_FROM_U << 24) : 0u, tw2 = 0u, tw3 = 0u;
 
@@ -629,12 +629,14 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
             if ((b & 3) == 0) {
                 if (rings_step(rg, rs, a, r, lane, k0, e0, 6)) __syncwarp();
                 if (grid_next()) {
+                    const int b_grid = b;
                     while (true) {
                         if (!(grid < kGridWide ? grid_bands(std::true_type{}) : grid_bands(std::false_type{}))) {
                             // these four bands exact; many more after repeated failures
                             pen = pen < 32 ? pen + 8 : min(2 * pen, 4096);
                             grid_from = b + 4 + (pen > 32 ? 4 * pen : 0);
                             grid_until = 0;
+                            if (lane == 0 && sp.side) atomicAdd(&a.counters[kCountGridAgain], 1ull);
                             break;
                         }
                         pen = max(pen - 1, 0);
@@ -643,6 +645,7 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
                         if (rings_step(rg, rs, a, r, lane, k0, e0, 6)) __syncwarp();
                         if (!grid_next()) break;
                     }
+                    if (lane == 0 && sp.side) atomicAdd(&a.counters[kCountGrid], (unsigned long long)((b - b_grid) >> 2));
                     if (b >= n_bands) break;
                     // back to the exact loop: band b's emission side
                     const float4 gm4 = *reinterpret_cast<const float4*>(&rg.gm[4 * lane]);
@@ -723,7 +726,10 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
     }
     cp_async_wait_all();  // no copy may land in shared memory after the read is done
     __syncwarp();
-    if (slow && sp.side) atomicAdd(&a.counters[0], slow);
+    if (slow && sp.side) {
+        atomicAdd(&a.counters[kCountSlow], (unsigned long long)slow);
+        atomicAdd(&a.counters[kCountFp64], (unsigned long long)slow);
+    }
 }
 
 // The forward pass of a checkpointed read by one warp, as a call: its code stays out of
@@ -981,7 +987,7 @@ __device__ __forceinline__ void chain_exact(const WideRead<kCk>& w, int tid, int
     float s1 = ws.sc[j0 ? before : 1][t], lp = ws.sc[j0 ? (before - 1) & (kScoreRing - 1) : 0][tl];
     float* lastc = a.last_col + r.ev_off;
     const int sl_last = (n_kmers - 1) & (kSlots - 1);
-    unsigned long long slow = 0;
+    unsigned slow = 0, fp64 = 0;
     // band b's last-column score and, optionally, its scores
     auto keep = [&](int b, bool last_col) {
         if (last_col) {
@@ -1069,6 +1075,7 @@ __device__ __forceinline__ void chain_exact(const WideRead<kCk>& w, int tid, int
                                                       a.km_sd[ko], a.km_k1[ko], w.cc.lp_step, w.cc.lp_stay, w.cc.lp_skip);
                     best = still ? c.best : best;
                     from = still ? c.from : from;
+                    fp64 += still ? 1 : 0;
                 }
                 ws.sc[r0 + q][t] = best;
             }
@@ -1102,7 +1109,8 @@ __device__ __forceinline__ void chain_exact(const WideRead<kCk>& w, int tid, int
         else
             chunk(j, F{}, F{});
     }
-    if (slow) atomicAdd(&a.counters[0], slow);
+    if (slow) atomicAdd(&a.counters[kCountSlow], (unsigned long long)slow);
+    if (fp64) atomicAdd(&a.counters[kCountFp64], (unsigned long long)fp64);
 }
 
 // ---- grid engine
@@ -1331,7 +1339,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
     float xl = 0.0f, g_lim = 0.0f;
     int g_mode = 0;
     int pen = 0;  // 8 for a failed chunk, -1 for a good one
-    unsigned long long slow = 0;
+    unsigned slow = 0, again_n = 0;
     constexpr uint32_t kOne = 1u << 25, kIn = (uint32_t)kBand << 25;
     auto release = [&](int s) { named_bar_arrive(kBarEmpty + s, kPair); };  // E closes the chunk and refills its slot
     // the state before chunk j, from the score ring
@@ -1348,6 +1356,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
     auto redo = [&](int j, int kb) {
         restore(j, kb);
         pen += 8;
+        ++again_n;
         uint32_t word[kPerLane] = {0u, 0u};
 #pragma unroll 1
         for (int q = 0; q < kWideChunk; ++q) {
@@ -1388,7 +1397,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
         for (long long i = 0; h >> 5 != j + 1 && i < a.spin_limit; ++i) h = *at;
         if (h >> 5 != j + 1) {
             ws.dead = 1;
-            if (lane == 0) atomicAdd(&a.counters[2], 1ull);  // the run reports a timeout
+            if (lane == 0) atomicAdd(&a.counters[kCountTimeouts], 1ull);  // the run reports a timeout
             for (int i = 0; h >> 5 != j + 1 && i < kReadyPolls; ++i) h = *at;
         }
         return h;
@@ -1525,7 +1534,14 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
         __syncwarp();
         release(s + g >= kGridRing ? s + g - kGridRing : s + g);
     }
-    if (slow) atomicAdd(&a.counters[0], slow);
+    if (slow) {  // a chunk done again: FP64 throughout
+        atomicAdd(&a.counters[kCountSlow], (unsigned long long)slow);
+        atomicAdd(&a.counters[kCountFp64], (unsigned long long)slow);
+    }
+    if (t == 0) {
+        atomicAdd(&a.counters[kCountGrid], (unsigned long long)(j - j0) - again_n);
+        atomicAdd(&a.counters[kCountGridAgain], (unsigned long long)again_n);
+    }
 }
 
 // One read's fill; false when a wait ran out of polls: the read is given up, the rest of it
@@ -1605,7 +1621,7 @@ __device__ __noinline__ bool fill_chain(const CoreArgs& a, const ReadDesc& r, un
 // shared memory every kClPublish bands (each release is a cluster-scope fence:
 // once per band they cost ~400 cycles per band).  E reads its inputs straight
 // from the pre stage's arrays (L2), one band ahead.  Every wait is bounded by
-// spin_limit polls; a wait that runs out counts in counters[2] and goes on (the
+// spin_limit polls; a wait that runs out is counted and goes on (the
 // batch then reports a timeout).  Measured: 1,030 cycles per band against 600
 // for the single-block wide shape, so the option is off by default.
 constexpr int kClRing = 16;    // bands of emissions in flight (<= 28: the k-mer window above)
@@ -1864,7 +1880,10 @@ __device__ void fill_wide_cl(const CoreArgs& a, const ReadDesc& r, ClSmem& ws, C
                 ++b;
             }
             cl_barrier();  // B_{n_bands-1}
-            if (slow) atomicAdd(&a.counters[0], slow);
+            if (slow) {
+                atomicAdd(&a.counters[kCountSlow], slow);
+                atomicAdd(&a.counters[kCountFp64], slow);
+            }
         } else if (group == 1) {
             // ------------------------------------------------ D (block 0)
             // band bn's diagonal candidates, inside flags and trim value, with the
@@ -1947,7 +1966,7 @@ __device__ void fill_wide_cl(const CoreArgs& a, const ReadDesc& r, ClSmem& ws, C
             cp_async_wait_all();
         }
     }
-    if (timeouts) atomicAdd(&a.counters[2], timeouts);
+    if (timeouts) atomicAdd(&a.counters[kCountTimeouts], timeouts);
 }
 
 // ---------------------------------------------------------------- post
@@ -3090,7 +3109,8 @@ static size_t noalloc_bytes(int32_t sequence_len, int32_t n_events) {
     const size_t nk_pad = (size_t)round_up(std::max<int64_t>(nk, 1), kChunk);
     const size_t nb_pad = (size_t)round_up(std::max<int64_t>(nb, 4), 4);
     return noalloc_align(sizeof(ReadDesc)) + 2 * noalloc_align(4 * ne_pad) + 4 * noalloc_align(4 * nk_pad) +
-           noalloc_align(nb_pad * kSlots) + noalloc_align(4 * nb_pad) + noalloc_align(16) + noalloc_align(32);
+           noalloc_align(nb_pad * kSlots) + noalloc_align(4 * nb_pad) + noalloc_align(16) +
+           noalloc_align(8 * kCounters);
 }
 
 }  // namespace abea
@@ -3153,12 +3173,12 @@ extern "C" abea_status_t abea_align_noalloc(abea_aligned_pair_t* pairs, int32_t*
     int32_t* band_k0 = (int32_t*)carve(4 * nb_pad);
     float* best = (float*)carve(4);
     int32_t* status = (int32_t*)(best + 1);
-    unsigned long long* counters = (unsigned long long*)carve(32);
+    unsigned long long* counters = (unsigned long long*)carve(8 * kCounters);
 
     const ReadDesc desc = describe_single_read(sequence_len, n_events, scaling, out_capacity);
     const GlobalConsts g = parity_consts();
     // every call shares the array: clear what must start at zero
-    if (cudaMemsetAsync(counters, 0, 32, st) != cudaSuccess) {
+    if (cudaMemsetAsync(counters, 0, 8 * kCounters, st) != cudaSuccess) {
         abea_internal_set_error("abea_align_noalloc: cudaMemsetAsync failed");
         return ABEA_ERR_CUDA;
     }

@@ -35,6 +35,11 @@ struct PreArgs {
     float4* km4;          // the four k-mer parameters side by side, for the wide shape (nullptr: not wanted)
 };
 
+// What a run counts: band cells computed again because the band loop's FP32 proof did not
+// cover them, those of them in FP64, waits that ran out of polls, stores out of their region
+// (bounds-checked build), tiles of four bands computed on a grid, those of them computed again.
+enum Counter { kCountSlow, kCountFp64, kCountTimeouts, kCountBounds, kCountGrid, kCountGridAgain, kCounters = 8 };
+
 struct CoreArgs {
     const ReadDesc* reads;
     int n_reads;
@@ -48,7 +53,7 @@ struct CoreArgs {
     uint8_t* trace;
     float* scores;                 // nullptr: scores not kept
     int32_t* band_k0;
-    unsigned long long* counters;  // [0] cells on the FP64 tier, [1] cells on the exact-all tier
+    unsigned long long* counters;  // [kCounters], zeroed: see Counter
     const int32_t* order;          // read indices, longest first
     int32_t* queue;                // zeroed work counters of the batched form
     int32_t n_wide;                // leading reads of `order` that run on the wide shape
@@ -56,7 +61,7 @@ struct CoreArgs {
     uint8_t* ck_scratch;           // recompute scratch: kCkBands bands of trace per checkpointed read
     int32_t* spec;                 // traceback cell maps: kSpecRound * kSpecBands int32 per slot
     int32_t n_spec;                // slots (queue[2] hands them out)
-    long long spin_limit;          // polls before a device-side wait gives up (counters[2] counts those)
+    long long spin_limit;          // polls before a device-side wait gives up (kCountTimeouts counts those)
     const float4* km4;             // {km_gm, km_sd, km_rsd, km_k1} of each k-mer position (wide shape)
 };
 

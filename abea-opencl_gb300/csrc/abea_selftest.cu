@@ -157,7 +157,89 @@ __global__ void selftest_kernel(uint64_t seed, int iters, unsigned long long* co
     atomicAdd(&counters[4], (unsigned long long)iters);  // per kind (the sums count two per case)
 }
 
+// Candidates on a grid over all the scores that the proof covers, (-60 * 2^m, -2^m), a quarter
+// of them at either end: the step's, the stay's and the skip's against the double arithmetic,
+// with transitions drawn at random or aimed so that T (the skip's B) lies next to an end of its
+// cell.  out: [0] wrong, of the transitions drawn at random [1] cases, [2] of them on a grid
+// (grid_step and grid_kmer_ok), [3] of those proven (neither NaN nor below the range);
+// of the skips drawn at random [4] cases, [5] on a grid; [6] aimed ones on a grid, skips too.
+__global__ void selftest_grid_kernel(uint64_t seed, int iters, unsigned long long* out) {
+    uint64_t s = mix64(seed ^ ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) * 0x632be59bd9b4e019ull));
+    unsigned long long n[7] = {0, 0, 0, 0, 0, 0, 0};
+    for (int it = 0; it < iters; ++it) {
+        const int m = kGridMin + (int)(unit(s) * (kGridMax - kGridMin + 1));
+        const float at = unit(s), lo = pow2f(m);
+        const float w = (it & 3) == 0 ? 1.0f + 1e-5f * at : (it & 3) == 1 ? 60.0f - 1e-4f * at : 1.0f + 59.0f * at;
+        const float a = fminf(-lo * w, __int_as_float(__float_as_int(-lo) + 1));
+        const float sd = 0.3f + 4.0f * unit(s);
+        const float gm = 60.0f + 70.0f * unit(s), k1 = __fsub_rn(kLogInvSqrt2Pi, logf(sd));
+        const float x = gm + sd * 8.0f * (unit(s) - 0.5f);  // within four deviations: in every grid's range
+        const float em = emission_ieee(x, gm, sd, k1);
+        const bool aimed = (it & 4) != 0;
+        double bb[3];  // step, stay, skip
+        for (int i = 0; i < 3; ++i) {
+            bb[i] = -(0.01 + 5.0 * (double)unit(s)) - (double)unit(s) * 1e-9;
+            if (aimed) {
+                const double g2 = (double)pow2f(m - 24), e = i < 2 ? (double)em : 0.0;
+                const double off = ((double)unit(s) - 0.5) * g2 * exp2(-30.0 * (double)unit(s));
+                bb[i] = g2 * floor((e + bb[i]) / g2) - e + off;
+            }
+        }
+        CellConsts cc{};
+        cc.step_h = (float)bb[0];
+        cc.step_l = (float)(bb[0] - (double)cc.step_h);
+        cc.stay_h = (float)bb[1];
+        cc.stay_l = (float)(bb[1] - (double)cc.stay_h);
+        cc.skip_h = (float)bb[2];
+        cc.skip_l = (float)(bb[2] - (double)cc.skip_h);
+        bool okd, oku, okl;
+        grid_step(cc.step_h, cc.step_l, m, okd);
+        grid_step(cc.stay_h, cc.stay_l, m, oku);
+        grid_step(cc.skip_h, cc.skip_l, m, okl);
+        const Grid G = make_grid(cc, m);
+        if (!aimed) {
+            n[1] += 2;
+            ++n[4];
+        }
+        if (okl) {
+            const float v = __fadd_rn(a, G.skip), r = __double2float_rn(__dadd_rn((double)a, bb[2]));
+            if (__float_as_int(v) != __float_as_int(r)) ++n[0];
+            ++n[aimed ? 6 : 5];
+        }
+        if (!okd || !oku || !grid_kmer_ok(sd, k1, grid_k1_max(cc.step_h, cc.stay_h))) continue;
+        const float rsd = __frcp_rn(sd);
+        const float2 g = m < kGridWide ? grid_pair<true>(x, gm, sd, rsd, k1, G) : grid_pair<false>(x, gm, sd, rsd, k1, G);
+        for (int i = 0; i < 2; ++i) {
+            const float part = i ? g.y : g.x, v = __fadd_rn(a, part);
+            const float r = __double2float_rn(__dadd_rn(__dadd_rn((double)a, bb[i]), (double)em));
+            const bool proven = part == part && part >= G.lim * kGridLimLo;
+            if (proven && __float_as_int(v) != __float_as_int(r)) ++n[0];
+            if (aimed)
+                ++n[6];
+            else {
+                ++n[2];
+                n[3] += proven ? 1 : 0;
+            }
+        }
+    }
+    for (int i = 0; i < 7; ++i) atomicAdd(&out[i], n[i]);
+}
+
 }  // namespace abea
+
+// The grid candidates' self-test: out[0..6] as selftest_grid_kernel says.  For tests.
+extern "C" abea_status_t abea_internal_selftest_grid(int64_t cases, uint64_t seed, int64_t* out) {
+    if (!out || cases <= 0) return ABEA_ERR_INVALID_ARG;
+    unsigned long long* d = nullptr;
+    if (cudaMalloc(&d, sizeof(unsigned long long) * 7) != cudaSuccess) return ABEA_ERR_OUT_OF_MEMORY;
+    cudaMemset(d, 0, sizeof(unsigned long long) * 7);
+    const int threads = 256, blocks = 1216;
+    const int iters = (int)std::max<int64_t>(8, cases / (threads * (int64_t)blocks));
+    abea::selftest_grid_kernel<<<blocks, threads>>>(seed, iters, d);
+    cudaError_t e = cudaMemcpy(out, d, sizeof(int64_t) * 7, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? ABEA_OK : ABEA_ERR_CUDA;
+}
 
 // Runs the self-test on the current device: `cases` random cases of each kind.
 // out[0..4]: division wrong, division declined, sum wrong, sum declined, cases.

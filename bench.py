@@ -320,7 +320,7 @@ def run_mode(pkg, batch, mode, device, steps, warmup, autotune=False):
     if autotune and mode == pkg.MODE_BATCHED:
         dev.autotune()
     per_step, core, timing = time_device(pkg, ctx, dev, steps, warmup)
-    res = dict(per_step=per_step, core=core, timing=timing, slow=dev.slow_cells())
+    res = dict(per_step=per_step, core=core, timing=timing, slow=dev._counters()["fp64"])
     dev.close()
     ctx.close()
     return res
@@ -610,7 +610,7 @@ def ours(args, dist):
         launches_per_step = tm["kernel_launches"]
     wall = time.perf_counter() - t_wall0
     clk = clocks.stop()
-    slow = dev.slow_cells()
+    slow = dev._counters()["fp64"]
     best = dev.best_scores()
     gpairs, gcounts = dev.results()
     dev.close()

@@ -272,8 +272,8 @@ abea_status_t abea_batch_read_bands(abea_ctx_t *ctx, abea_batch_t *batch, int32_
  * penalties, GPU/align_cuda.cl:722-746) of the last run, host array [n_reads]. */
 abea_status_t abea_batch_best_scores(abea_ctx_t *ctx, abea_batch_t *batch, float *best_scores);
 
-/* Number of band cells that the last run computed again because the band loop's
- * FP32 proof did not cover them, most of them in FP64 (diagnostic). */
+/* Number of band cells whose first FP32 exactness proof failed in the last run: they were
+ * proven by a second one or computed in FP64 (diagnostic). */
 abea_status_t abea_batch_slow_cells(abea_ctx_t *ctx, abea_batch_t *batch, int64_t *count);
 
 /* Pinned host memory for fast host<->device copies (cudaHostAlloc). */

@@ -139,6 +139,59 @@ def test_many_entries_into_the_grid_chain(oracle_mod):
         assert np.array_equal(dev.best_scores().view(np.uint32), obest.view(np.uint32))
 
 
+def counters(batch, shape):
+    ctx = abea.Context(0, abea.MODE_BATCHED)
+    ctx.set_option(abea.OPT_LONG_READ_BANDS, 1 if shape == "wide" else 1 << 40)
+    dev = ctx.upload(batch)
+    dev.run()
+    dev.results()
+    return dev._counters()
+
+
+def test_grid_candidates_selftest():
+    """Candidates on every grid over the whole range of scores, aimed at the ends of their cells
+    or not: none wrong, and the random ones hardly ever declined.  A k-mer is refused for an
+    emission that may be positive: at most the 5% of deviations below 0.5, and with them
+    margins and divisions of under 1 in 1,000 (as the division's own self-test asks)."""
+    import ctypes as C
+    out = np.zeros(7, dtype=np.int64)
+    f = abea.lib().abea_internal_selftest_grid
+    f.argtypes, f.restype = [C.c_int64, C.c_uint64, C.c_void_p], C.c_int
+    assert f(1 << 26, 7, out.ctypes.data) == 0
+    wrong, cases, on_grid, proven, skips, skips_on_grid, aimed = out.tolist()
+    assert wrong == 0
+    assert on_grid > 0.94 * cases and proven > 0.999 * on_grid
+    assert skips_on_grid > 0.999 * skips
+    assert aimed > 1 << 20
+
+
+@pytest.mark.parametrize("shape", ["wide", "warp"])
+def test_an_ordinary_read_runs_on_the_grid(shape):
+    """All but the first and last bands: scores pass -2^11 after some 950 bands (the wide shape
+    tries after 800, then every 128), and a read's last 170 k-mers are the exact engine's."""
+    rng = np.random.default_rng(18)
+    model, seq, ev = make(rng, 6000)
+    batch = batch_of(model, [(seq, ev)])
+    c = counters(batch, shape)
+    bands = int(batch.n_bands()[0])
+    assert c["grid"] > 0.9 * (bands - 1200 - 170 * bands / 6000) / 4
+    assert c["grid_again"] < 0.1 * c["grid"]
+
+
+@pytest.mark.parametrize("shape", ["wide", "warp"])
+def test_cells_without_a_proof_are_done_again_in_fp64(shape):
+    """An infinite event's emissions are proven by nothing: its cells (one in each of the 100
+    bands or more that hold it) are computed in FP64."""
+    rng = np.random.default_rng(13)
+    model, seq, ev = make(rng, 2400)
+    plain = counters(batch_of(model, [(seq, ev)]), shape)
+    ev = ev.copy()
+    ev["mean"][[700, 1500, 2600, 3300]] = np.inf
+    c = counters(batch_of(model, [(seq, ev)]), shape)
+    assert c["fp64"] >= plain["fp64"] + 4 * 90
+    assert c["fp64"] <= c["slow"]
+
+
 @pytest.mark.parametrize("budget", [0, 400_000])
 def test_a_wait_out_of_polls_ends_in_a_timeout(oracle_mod, budget):
     """With a limit of one poll the grid chain's waits give up: the run reports a timeout
