@@ -829,6 +829,7 @@ struct alignas(16) WideSmem {
     int32_t flag;                   // a failed check
     int32_t exit, failing;          // the first chunk not done; failures made it leave
     int32_t dead;                   // a wait ran out of polls
+    int32_t k_odd;                  // the next k-mer that is none for a grid
 };
 __device__ __forceinline__ int chunk_head(int j, int mode) { return (j + 1) << 5 | mode; }  // never 0
 static_assert(kGridMax < 32, "five bits of mode");
@@ -906,6 +907,11 @@ struct WideRead {
     __device__ __forceinline__ void record_end(float* rec, int j, int k0) const {
         rec[2 * kSlots] = __int_as_float(k0);
         rec[2 * kSlots + 1] = __int_as_float(kWideChunk * j + 1 - k0);  // the event of band 4j + 3
+    }
+    // whether k-mer k may be on a grid
+    __device__ __forceinline__ bool grid_kmer(int k) const {
+        const float4 km = a.km4[r.km_off + k];
+        return grid_kmer_ok(km.y, km.w, grid_k1_max(cc.step_h, cc.stay_h));
     }
     // the end cells of band b-1 (its row of the ring) and the left neighbour of a slot
     __device__ __forceinline__ void ends(int row, int k0, float& ll, float& ur) const {
@@ -1219,16 +1225,17 @@ __device__ __forceinline__ int chunk_mode(int want, int kp, int b0, int n_kmers)
 
 // Chunks from j0 on, until one that no grid serves (ws.exit), from the bands before them
 // in the score ring; `first`: the grid of those.  Every thread of the block calls it, with
-// ws.head and ws.flag zero and ws.exit the largest int.
+// ws.head and ws.flag zero and ws.exit the largest int.  k_end: the k-mer that E's windows
+// stay before (the read's end, or one that is none for a grid).
 template <bool kScores, bool kCk>
-__device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int j0, int first, uint32_t modes) {
+__device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int j0, int first, uint32_t modes, int k_end) {
     const int warp = tid >> 5, lane = tid & 31;
     if ((warp & 3) < 2 && warp >= 2) return;
     WideSmem& ws = w.ws;
     const ReadDesc& r = w.r;
     const CoreArgs& a = w.a;
     const CellConsts& cc = w.cc;
-    const int n_events = w.n_events, n_kmers = w.n_kmers;
+    const int n_events = w.n_events;
     const int t = tid & (kTeam - 1);  // slots 2t and 2t + 1
     const int tl = (kPerLane * t + kSlots - 1) & (kSlots - 1);
     const int k_start = ws.kb[(kWideChunk * j0 - 1) & (kScoreRing - 1)] >> 2;
@@ -1256,7 +1263,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
                 if (jr >= ws.exit) break;
                 kp = ws.kb[(br + kWideChunk - 1) & (kScoreRing - 1)] >> 2;
             }
-            const int mode = chunk_mode(want, kp, b0, n_kmers);
+            const int mode = chunk_mode(want, kp, b0, k_end);
             if (closes) {
                 const float2 sk = ws.skip[jr & (kHeadRing - 1)];
                 if (turn & 1) want = grid_of(ws.sc[(br + 3) & (kScoreRing - 1)], lane, modes);
@@ -1545,15 +1552,16 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
 }
 
 // One read's fill; false when a wait ran out of polls: the read is given up, the rest of it
-// not filled.  `grids`: the read's k-mers allow grids (grid_kmer_ok).  A call, as
-// fill_warp_ck is: each has the block's registers to itself.
+// not filled.  `odd`: some k-mer of the read is none for a grid (grid_kmer_ok); the grid
+// chain then runs between such k-mers.  A call, as fill_warp_ck is: each has the block's
+// registers to itself.
 template <bool kScores, bool kCk>
-__device__ __noinline__ bool fill_chain(const CoreArgs& a, const ReadDesc& r, unsigned ws_at, int tid, bool grids) {
+__device__ __noinline__ bool fill_chain(const CoreArgs& a, const ReadDesc& r, unsigned ws_at, int tid, bool odd) {
     WideSmem& ws = smem_ref<WideSmem>(ws_at);
     const int lane = tid & 31;
     WideRead<kCk> w{a, r, ws, make_consts(r, a.g), r.n_events, r.n_kmers, r.n_bands, (r.n_bands + kWideChunk - 1) / kWideChunk,
                a.trace + r.trace_off * kSlots, a.band_k0 + r.band_off, kScores ? a.scores + r.band_off * kSlots : nullptr};
-    const uint32_t modes = grids ? grid_modes(w.cc) : 0u;
+    const uint32_t modes = grid_modes(w.cc);
     // band 0: the start cell (slot 127) = 0; band 1: the trim cell; both at k0 = -51
     if (tid < kSlots) {
         ws.sc[0][tid] = tid == 127 ? 0.0f : -INFINITY;
@@ -1577,26 +1585,36 @@ __device__ __noinline__ bool fill_chain(const CoreArgs& a, const ReadDesc& r, un
         if (tid == 0) {
             ws.flag = 0;
             ws.exit = INT32_MAX;
+            ws.k_odd = INT32_MAX;
         }
         __syncthreads();
         if (j >= w.n_chunks) return true;
         // the grid engine, if its chunks can begin here and there is room for a run
         const int b0 = kWideChunk * j, kp = ws.kb[(b0 - 1) & (kScoreRing - 1)] >> 2;
         const int first = grid_of(ws.sc[(b0 - 1) & (kScoreRing - 1)], lane, modes);
-        const bool room = kp >= -1 && b0 - 3 - kp <= w.n_events && chunk_mode(1, kp + 40, b0 + 2 * 40, w.n_kmers);
+        int k_end = w.n_kmers;
+        if (odd) {
+            // up to the next k-mer that is none for a grid, looked for among the next 4,096
+            const int k_from = max(kp, 0), k_stop = min(w.n_kmers, k_from + 8 * kWideThreads);
+            for (int k = k_from + tid; k < k_stop; k += kWideThreads)
+                if (!w.grid_kmer(k)) atomicMin(&ws.k_odd, k);
+            __syncthreads();
+            k_end = min(k_stop, ws.k_odd);
+        }
+        const bool room = kp >= -1 && b0 - 3 - kp <= w.n_events && chunk_mode(1, kp + 40, b0 + 2 * 40, k_end);
         seg = kp < 0 || kp + 40 <= w.n_kmers - kSlots ? retry : w.n_chunks;  // near the end: to the end
-        const bool enter = first && room && chunk_mode(first, kp, b0, w.n_kmers);
+        const bool enter = first && room && chunk_mode(first, kp, b0, k_end);
         // Every warp has decided before the chain may overwrite what they decided from: the
         // warps that the chain leaves idle never wait for it, and all must go the same way.
         __syncthreads();
         if (enter) {
-            chain_grid<kScores>(w, tid, j, first, modes);
+            chain_grid<kScores>(w, tid, j, first, modes, k_end);
             __syncthreads();
             if (ws.dead) return false;
             j = ws.exit;
             if (ws.failing) retry = min(2 * retry, 1 << 20);
-            const int k_end = ws.kb[(kWideChunk * j - 1) & (kScoreRing - 1)] >> 2;
-            seg = k_end + 64 <= w.n_kmers - kSlots ? retry : w.n_chunks;
+            const int k_now = ws.kb[(kWideChunk * j - 1) & (kScoreRing - 1)] >> 2;
+            seg = k_now + 64 <= w.n_kmers - kSlots ? retry : w.n_chunks;
             __syncthreads();  // everyone has read the exit
         }
     }
@@ -2819,14 +2837,13 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(const __g
     const int free_rank = sm.free_rank, wide_slot = sm.wide_slot;
     while (wide_read >= 0) {
         const ReadDesc& r = a.reads[wide_read];
-        const bool odd = pre_read(pa, wide_read, t, kWideThreads);
-        const bool grids = !__syncthreads_or(odd);  // the read's parameters are in memory for the whole block
+        const bool odd = __syncthreads_or(pre_read(pa, wide_read, t, kWideThreads));  // the read's parameters are in memory for the whole block
         bool filled = true;
         if (!r.skip) {
             if (r.ck)
-                filled = fill_chain<kScores, true>(a, r, smem_u32(&sm.wide), t, grids);
+                filled = fill_chain<kScores, true>(a, r, smem_u32(&sm.wide), t, odd);
             else
-                filled = fill_chain<kScores, false>(a, r, smem_u32(&sm.wide), t, grids);
+                filled = fill_chain<kScores, false>(a, r, smem_u32(&sm.wide), t, odd);
         }
         __syncthreads();
         __threadfence_block();

@@ -179,6 +179,29 @@ def test_an_ordinary_read_runs_on_the_grid(shape):
 
 
 @pytest.mark.parametrize("shape", ["wide", "warp"])
+@pytest.mark.parametrize("every", [4000, 1500, 400, 60])
+def test_a_grid_between_kmers_that_none_serves(oracle_mod, every, shape):
+    """k-mers whose emissions may be positive (a deviation of 0.2), one in `every` bases: the
+    bands between them still run on a grid where 128-slot windows fit between them (not at one
+    in 60), and every score is the oracle's."""
+    rng = np.random.default_rng(19)
+    model, seq, ev = make(rng, 6000)
+    model = model.copy()
+    codes = np.searchsorted(np.frombuffer(b"ACGT", np.uint8), np.frombuffer(seq, np.uint8)).astype(np.int64)
+    ranks = sum(codes[i:len(codes) - 5 + i] << (2 * (5 - i)) for i in range(6))
+    hits = np.bincount(ranks, minlength=4096)
+    for at in range(every // 2, len(ranks), every):
+        once = at + int(np.argmin(hits[ranks[at:at + 40]]))  # a k-mer that is rare in the read
+        model["level_stdv"][ranks[once]] = 0.2
+        model["level_log_stdv"][ranks[once]] = np.log(0.2)
+    batch = batch_of(model, [(seq, ev)])
+    check(oracle_mod, batch, shape)
+    c = counters(batch, shape)
+    if shape == "wide":
+        assert c["grid"] > 100 if every >= 400 else c["grid"] < 100
+
+
+@pytest.mark.parametrize("shape", ["wide", "warp"])
 def test_cells_without_a_proof_are_done_again_in_fp64(shape):
     """An infinite event's emissions are proven by nothing: its cells (one in each of the 100
     bands or more that hold it) are computed in FP64."""
