@@ -583,38 +583,56 @@ static int64_t d2h_bytes(const abea_batch* b) {
 // minimises an estimate of the batch's
 // makespan, in cycles:
 //   the longest wide read (wide_cycles);
-//   the longest warp-shape read, kWarpBase + kWarpMore * w cycles per band with w
-//     warps sharing its SM in the first wave (the blocks without a wide read share
-//     the other reads round-robin, at most 16 warps each);
+//   the longest warp-shape read (warp_cycles) with w warps sharing its SM in the
+//     first wave (the blocks without a wide read share the other reads round-robin,
+//     at most 16 warps each);
 //   the warp-shape work spread over those blocks' warps at that rate.
-// A checkpointed read on the warp shape counts its bands twice: its traceback
-// recomputes them on the same warp.
 // Then every read on the wide shape, the blocks pulling them longest first: the
 // longest read, or all of them over the blocks.  That wins when it is within 2% of
 // the first and either the longest read bounds it or there are at most 8 reads per
 // block, unless there are reads that may not be wide: those would start last.
-// Calibrated on GB300 (ms, every read wide / none): 1,024 reads of 1-10 kb 12.7 / 19,
-// 608 reads of 3 kb 4.91 / 4.77, 1,216 of 3 kb 9.52 / 6.68, 2,432 of 3 kb 18.9 / 8.5
+// Calibrated on GB300 (ms, every read wide / none): 1,024 reads of 1-10 kb 11.8 / 14.3,
+// 608 reads of 3 kb 4.90 / 5.74, 1,216 of 3 kb 9.30 / 6.78, 2,432 of 3 kb 18.9 / 9.7
 // (sixteen warps on an SM take 131 cycles per band together, one wide read 200-290),
-// 2,432 of 600 b 7.85 / 3.06, 152 of 3 kb 1.29 / 4.53.  Ties go to fewer wide reads;
-// the threshold is the band count of the n-th wide read (every read: 1; none:
+// 608 of 600 b 1.60 / 1.71, 1,216 of 600 b 3.05 / 2.06, 152 of 3 kb 1.71 / 5.57; one read of
+// 100 b 0.11 / 0.51, of 300 b 0.24 / 1.01, 304 of 300 b 0.45 / 1.12.  Ties go to fewer wide
+// reads; the threshold is the band count of the n-th wide read (every read: 1; none:
 // INT64_MAX).
+// A read on the warp shape: kWarpBase + kWarpMore * w cycles per band, and what its first
+// bands add, where a cell without a proof in three of four takes FP64 (its warps' FP64 units
+// are shared from 8 on).  A checkpointed one twice: its traceback recomputes it on the same
+// warp.
 constexpr double kWarpBase = 950, kWarpMore = 68;
+static double warp_bands(const ReadDesc& r) { return (r.ck ? 2.0 : 1.0) * (double)r.n_bands; }
+static double warp_start(const ReadDesc& r) {
+    const double nb = (double)r.n_bands;
+    return (r.ck ? 2.0 : 1.0) * (2400 * std::min(nb, 300.0) + 900 * std::min(std::max(nb - 300, 0.0), 900.0));
+}
+static double warp_cycles(double bands, double start, double w) {
+    return bands * (kWarpBase + kWarpMore * w) + start * std::max(1.0, w / 8);
+}
 // A read on the wide shape, pre stage and traceback included: its bands on the grid
-// engine, the exact engine's share (its start and tail), and what each read costs.
-// A checkpointed one also recomputes its bands, 16 warps at a time.
+// engine, the exact engine's share (its start and, once the grid has run, its tail), and
+// what each read costs.  A checkpointed one also recomputes its bands, 16 segments at a time,
+// the first of them (or the whole of a read without a traceback slot) through a read's
+// start on one warp.
 static double wide_cycles(const ReadDesc& r) {
     const double nb = (double)r.n_bands;
-    return (r.ck ? 370 : 220) * nb + 275 * std::min(nb, 1240.0) + 165e3;
+    double c = 220 * nb + 275 * std::min(nb, 1240.0) + 20e3 + 145e3 * std::min(std::max((nb - 800) / 900, 0.0), 1.0);
+    if (r.ck) {
+        const double alone = r.n_bands < kSpecMinBands ? nb : (double)kCkBands;
+        c += 150 * nb + alone * (kWarpBase + 2400);
+    }
+    return c;
 }
-static double warp_bands(const ReadDesc& r) { return (r.ck ? 2.0 : 1.0) * (double)r.n_bands; }
 static int64_t heuristic_threshold(const abea_batch* b, int blocks, bool ck_wide) {
     const size_t n = b->order.size();
     std::vector<const ReadDesc*> wide_ok;  // the reads that may be wide, longest first
-    double rest_bands = 0, all_wide = 0;
+    double rest_bands = 0, rest_start = 0, all_wide = 0;
     for (int32_t i : b->order) {
         const ReadDesc& r = b->reads[(size_t)i];
         rest_bands += warp_bands(r);
+        rest_start += warp_start(r);
         all_wide += wide_cycles(r);
         if (ck_wide || !r.ck) wide_ok.push_back(&r);
     }
@@ -628,15 +646,16 @@ static int64_t heuristic_threshold(const abea_batch* b, int blocks, bool ck_wide
     for (int k = 0; k <= max_wide; ++k) {
         if (k > 0) {  // the k-th wide read leaves the warp-shape set
             rest_bands -= warp_bands(*wide_ok[(size_t)k - 1]);
+            rest_start -= warp_start(*wide_ok[(size_t)k - 1]);
             ++taken;
         }
         for (; j < n && (ck_wide || !b->reads[(size_t)b->order[j]].ck) && passed < taken; ++j) ++passed;
-        const double longest_warp = j < n ? warp_bands(b->reads[(size_t)b->order[j]]) : 0.0;
         const int free_blocks = std::max(1, blocks - k);
         const double warps = std::min(16.0, std::max(1.0, (double)(n - (size_t)k) / free_blocks));
-        const double per_band = kWarpBase + kWarpMore * warps;
+        const ReadDesc* longest = j < n ? &b->reads[(size_t)b->order[j]] : nullptr;
+        const double t_warp = longest ? warp_cycles(warp_bands(*longest), warp_start(*longest), warps) : 0.0;
         const double t_wide = k > 0 ? wide_cycles(*wide_ok[0]) : 0.0;
-        const double t = std::max(t_wide, std::max(longest_warp, rest_bands / (warps * free_blocks)) * per_band);
+        const double t = std::max(t_wide, std::max(t_warp, warp_cycles(rest_bands, rest_start, warps) / (warps * free_blocks)));
         if (k == 0 || t < best_t * 0.98) {  // a wide read must buy at least 2%
             best_t = t;
             best_n = k;

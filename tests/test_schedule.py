@@ -67,6 +67,22 @@ def test_fewer_reads_than_blocks_and_edge_inputs():
     assert wide_threshold([10], blocks=0) == -1
 
 
+def test_short_reads_that_leave_sms_free_are_wide():
+    """A read's first bands are where the warp shape's cells most often need FP64: one read of
+    20 to 300 bases, or up to four per SM, is two to five times as fast on the wide shape
+    (one of 100 bases 0.11 ms against 0.51; 304 of 300 bases 0.45 against 1.12)."""
+    for bands in (40, 145, 263, 407, 842):
+        assert n_wide([bands]) == 1, bands
+    for n in (4, 64, 152):
+        assert n_wide([276] * n) == n
+    assert n_wide([58] * 152) == 152
+    assert n_wide([878] * 304) == 304
+    assert n_wide([304] * 608) == 608
+    # with 16 reads and more per SM the warps' number wins again (0.88 ms; 3.2 against 7.9)
+    assert n_wide([110] * 4000) == 0
+    assert n_wide([1759] * 2432) == 0
+
+
 def test_checkpointed_reads_keep_the_split():
     """A latency-bound batch with checkpointed reads (trace over the budget): those
     run on the warp shape and would start last behind every wide read, so the
