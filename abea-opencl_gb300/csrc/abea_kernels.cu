@@ -378,8 +378,6 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
     const int n_events = r.n_events, n_kmers = r.n_kmers, n_bands = sp.b_end;
     uint8_t* trace = sp.trace;
     float* scores = kScores && sp.side ? a.scores + r.band_off * kSlots : nullptr;
-    int32_t* bk0 = a.band_k0 + r.band_off;
-    float* lastc = a.last_col + r.ev_off;
 
     // band 0: start cell (e=-1,k=-1) = 0 in slot 127; band 1: trim cell (e=0,k=-1)
     // = (float)lp_trim, FROM_U, slot 127 (GPU/align_cuda.cl:249-268).  A resumed
@@ -464,7 +462,7 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
                 word = here ? ((word & 0x00ffffffu) | (in ? (ABEA_FROM_U << 24) : 0u)) : word;
             }
             if (sp.side && ol >= lo && ol < hi && lane == (sl_last >> 2) && in_bounds(e0 - ol, n_events, a.counters))
-                lastc[e0 - ol] = sel4(best, sl_last & 3);
+                (a.last_col + r.ev_off)[e0 - ol] = sel4(best, sl_last & 3);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -487,7 +485,7 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
             reinterpret_cast<float4*>(scores + (int64_t)b * kSlots)[lane] = make_float4(best[0], best[1], best[2], best[3]);
         my_k0 = ((b & 31) == lane) ? k0 : my_k0;
         if (sp.side && ((b & 31) == 31 || b == n_bands - 1)) {
-            if (lane <= (b & 31) && in_bounds((b & ~31) + lane, r.n_bands, a.counters)) bk0[(b & ~31) + lane] = my_k0;
+            if (lane <= (b & 31) && in_bounds((b & ~31) + lane, r.n_bands, a.counters)) (a.band_k0 + r.band_off)[(b & ~31) + lane] = my_k0;
         }
     };
     // Four bands at a time on a grid (abea_cell.cuh, "candidates on a grid") where the
@@ -498,11 +496,11 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
     // the loop body stays small (up to sixteen warps on an SM, each at its own place).
     // A read of 20 kb alone: 1,050 cycles per band before, 530 now (the plain form's f5c
     // batch 33.4 -> 17.5 ms); sixteen warps on an SM 131 together.
-    //   grid: the grid in use until band grid_until; grid_from: the first band that may try.
-    const uint32_t modes = grid_modes(cc);
-    const float k1_max = grid_k1_max(cc.step_h, cc.stay_h);
-    Grid G{};
-    int grid = 0, g_made = 0, grid_until = 0, grid_from = sp.b_begin, pen = 0;
+    //   The exact loop carries no more of it than grid_from, the first band that may try, and
+    // pen, the recent failures: a grid is made anew for each run of tiles (kept between runs it
+    // cost the exact loop its registers: 300 reads of 0.5-6 kb two to an SM 7.57 ms, now 6.53,
+    // with scalings off, where no band tries, 13.0 and 12.2; the exact loop alone had 11.6).
+    int grid_from = sp.b_begin, pen = 0;
     auto grid_now = [&]() {
         bool hole = false;
         float mx = -INFINITY, mn = 0.0f;
@@ -516,10 +514,11 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
         mx = warp_max(mx);
         mn = warp_min(mn);
         const int m = (__float_as_int(-mx) >> 23) - 127, mlo = (__float_as_int(-mn) >> 23) - 127;
-        return !none && m >= kGridMin && m <= kGridMax && mlo < m + 2 && ((modes >> (m & 31)) & 1u) ? m : 0;
+        return !none && m >= kGridMin && m <= kGridMax && mlo < m + 2 ? m : 0;
     };
     // bands b .. b + 3; false (and the state as it was) when the check fails
-    auto grid_bands = [&](auto low) {
+    auto grid_bands = [&](auto low, const Grid& G) {
+        const float k1_max = grid_k1_max(cc.step_h, cc.stay_h);
         constexpr bool kLow = decltype(low)::value;
         constexpr uint32_t kOne = 1u << 25, kIn = (uint32_t)kBand << 25;
         const int k_was = k0, my_was = my_k0;
@@ -589,7 +588,7 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
         if ((!kSpan || trace) && in_bounds((b - sp.trace_band0) >> 2, sp.trace_tiles, a.counters))
             reinterpret_cast<uint4*>(trace + (int64_t)((b - sp.trace_band0) >> 2) * 512)[lane] = make_uint4(w[0], w[1], w[2], w[3]);
         if (sp.side && ((b + 3) & 31) == 31) {
-            if (in_bounds(((b + 3) & ~31) + lane, r.n_bands, a.counters)) bk0[((b + 3) & ~31) + lane] = my_k0;
+            if (in_bounds(((b + 3) & ~31) + lane, r.n_bands, a.counters)) (a.band_k0 + r.band_off)[((b + 3) & ~31) + lane] = my_k0;
         }
         return true;
     };
@@ -606,21 +605,9 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
             }
         }
     };
-    // all 100 cells of bands b .. b + 3 are computed, none on the last k-mer column, and
-    // their scores are in a grid's range
-    auto grid_next = [&]() {
-        if (b < grid_from || b + 4 > n_bands || k0 < 0 || k0 + 4 + kBand > n_kmers - 1 || e0 < kBand - 1 ||
-            e0 + 4 > n_events - 1)
-            return false;
-        if (b >= grid_until) {
-            grid = grid_now();
-            grid_until = b + 16;
-            if (grid && grid != g_made) {
-                G = make_grid(cc, grid);
-                g_made = grid;
-            }
-        }
-        return grid != 0;
+    // all 100 cells of bands b .. b + 3 are computed, none on the last k-mer column
+    auto inside = [&]() {
+        return b + 4 <= n_bands && k0 >= 0 && k0 + 4 + kBand <= n_kmers - 1 && e0 >= kBand - 1 && e0 + 4 <= n_events - 1;
     };
     while (true) {
         bool to_slow = false;
@@ -628,14 +615,32 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
             checkpoint();
             if ((b & 3) == 0) {
                 if (rings_step(rg, rs, a, r, lane, k0, e0, 6)) __syncwarp();
-                if (grid_next()) {
-                    const int b_grid = b;
-                    while (true) {
-                        if (!(grid < kGridWide ? grid_bands(std::true_type{}) : grid_bands(std::false_type{}))) {
+                if (b >= grid_from && inside()) {
+                    const int b_first = b;
+                    Grid G{};
+                    int made = 0, until = 0;
+                    do {
+                        if (b >= until) {
+                            int m = grid_now();
+                            until = b + 16;
+                            if (m && m != made) {
+                                bool ok1, ok2, ok3;
+                                grid_step(cc.step_h, cc.step_l, m, ok1);
+                                grid_step(cc.stay_h, cc.stay_l, m, ok2);
+                                grid_step(cc.skip_h, cc.skip_l, m, ok3);
+                                G = make_grid(cc, m);
+                                if (!(ok1 && ok2 && ok3)) m = 0;
+                            }
+                            made = m;
+                            if (!m) {
+                                grid_from = until;
+                                break;
+                            }
+                        }
+                        if (!(made < kGridWide ? grid_bands(std::true_type{}, G) : grid_bands(std::false_type{}, G))) {
                             // these four bands exact; many more after repeated failures
                             pen = pen < 32 ? pen + 8 : min(2 * pen, 4096);
                             grid_from = b + 4 + (pen > 32 ? 4 * pen : 0);
-                            grid_until = 0;
                             if (lane == 0 && sp.side) atomicAdd(&a.counters[kCountGridAgain], 1ull);
                             break;
                         }
@@ -643,9 +648,8 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
                         b += 4;
                         checkpoint();
                         if (rings_step(rg, rs, a, r, lane, k0, e0, 6)) __syncwarp();
-                        if (!grid_next()) break;
-                    }
-                    if (lane == 0 && sp.side) atomicAdd(&a.counters[kCountGrid], (unsigned long long)((b - b_grid) >> 2));
+                    } while (inside());
+                    if (lane == 0 && sp.side) atomicAdd(&a.counters[kCountGrid], (unsigned long long)((b - b_first) >> 2));
                     if (b >= n_bands) break;
                     // back to the exact loop: band b's emission side
                     const float4 gm4 = *reinterpret_cast<const float4*>(&rg.gm[4 * lane]);
@@ -712,12 +716,13 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
             finish();
         }
         if (!to_slow) break;
+        const CellConsts cs = make_consts(r, a.g);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (bad[j]) {  // a proof failed: the reference's FP64 arithmetic
                 const int sj = 4 * lane + j;
                 best[j] = cell_slow(LP[j], S1[j], left[j], rg.ev[ep[j] & (kEvRing - 1)], rg.gm[sj], rg.sd[sj],
-                                    rg.k1[sj], cc, from[j]);
+                                    rg.k1[sj], cs, from[j]);
                 ++slow;
             }
         }
@@ -732,17 +737,11 @@ __device__ void fill_warp(const CoreArgs& a, const ReadDesc& r, Rings& rg, int l
     }
 }
 
-// The forward pass of a checkpointed read by one warp, as a call: its code stays out of
-// the kernels that mostly run the other.
-// Shared memory goes by its own address, so that its accesses stay shared ones.
+// Shared memory goes into a function by its own address, so that its accesses stay shared ones.
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 template <class T>
 __device__ __forceinline__ T& smem_ref(unsigned at) {
     return *reinterpret_cast<T*>(__cvta_shared_to_generic(at));
-}
-template <bool kScores>
-__device__ __noinline__ void fill_warp_ck(const CoreArgs& a, const ReadDesc& r, unsigned rg_at, int lane) {
-    fill_warp<kScores, true>(a, r, smem_ref<Rings>(rg_at), lane, forward_span(a, r));
 }
 
 // ---------------------------------------------------------------- wide shape
@@ -1553,7 +1552,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
 
 // One read's fill; false when a wait ran out of polls: the read is given up, the rest of it
 // not filled.  `odd`: some k-mer of the read is none for a grid (grid_kmer_ok); the grid
-// chain then runs between such k-mers.  A call, as fill_warp_ck is: each has the block's
+// chain then runs between such k-mers.  A call: it has the block's
 // registers to itself.
 template <bool kScores, bool kCk>
 __device__ __noinline__ bool fill_chain(const CoreArgs& a, const ReadDesc& r, unsigned ws_at, int tid, bool odd) {
@@ -2168,9 +2167,9 @@ __device__ bool walk_segment(const uint8_t* trace, int trace_band0, int bands_en
 
 // Recomputes the trace of segment seg (bands [seg*kCkBands, (seg+1)*kCkBands)) of
 // a checkpointed read into `mem` (kCkBands * kSlots bytes).  The whole warp calls it.
-__device__ __noinline__ void recompute_segment(const CoreArgs& ca, const ReadDesc& r, unsigned rg_at, int lane, int seg,
-                                               uint8_t* mem) {
-    Rings& rg = smem_ref<Rings>(rg_at);
+// Inlined at its three calls (as a function: the recompute of 1 kb reads 6-10% slower).
+__device__ __forceinline__ void recompute_segment(const CoreArgs& ca, const ReadDesc& r, Rings& rg, int lane, int seg,
+                                                  uint8_t* mem) {
     FillSpan sp;
     sp.b_begin = max(2, seg * kCkBands);
     sp.b_end = min((seg + 1) * kCkBands, r.n_bands);
@@ -2269,7 +2268,7 @@ __device__ void post_read_warp(const CoreArgs& ca, const PostArgs& a, int ri, ui
             // the trace was not kept: recompute it kCkBands bands at a time from
             // the checkpoints, top segment first, and walk each
             for (int seg = (w.k + w.e + 2) / kCkBands; seg >= 0; --seg) {
-                recompute_segment(ca, r, smem_u32(&rg), lane, seg, ck_seg);
+                recompute_segment(ca, r, rg, lane, seg, ck_seg);
                 if (walk_segment<kWalkPairs, kRing>(ck_seg, seg * kCkBands, min((seg + 1) * kCkBands, n_bands),
                                                seg * kCkBands, ring, lane, w, out, cap, a, r))
                     break;
@@ -2364,7 +2363,7 @@ __device__ void post_tail(const CoreArgs& ca, const PostArgs& a, int ri, const R
             // recompute and walk again, summing the emissions in walk order
             Walk w{n_kmers - 1, best_e, 0, 0, 0, n_kmers - 1, 0, 0.0};
             for (int seg = (w.k + w.e + 2) / kCkBands; seg >= 0; --seg) {
-                recompute_segment(ca, r, smem_u32(&rg), lane, seg, ck_seg);
+                recompute_segment(ca, r, rg, lane, seg, ck_seg);
                 if (walk_segment<kWalkSum, kRing>(ck_seg, seg * kCkBands, min((seg + 1) * kCkBands, n_bands),
                                               seg * kCkBands, ring, lane, w, out, cap, a, r))
                     break;
@@ -2742,7 +2741,7 @@ __device__ void post_ck_block(const CoreArgs& ca, const PostArgs& a, int ri, uin
     if (best > -INFINITY) {
         for (int top = (w.k + w.e + 2) / kCkBands; top >= 0; top -= kWideThreads / 32) {
             if (top - warp >= 0)
-                recompute_segment(ca, r, smem_u32(&rings[warp]), lane, top - warp, mem + (int64_t)warp * kSegBytes);
+                recompute_segment(ca, r, rings[warp], lane, top - warp, mem + (int64_t)warp * kSegBytes);
             if (t == 0) ended = 0;
             __syncthreads();  // the segments are in memory
             if (warp == 0) {
@@ -2889,7 +2888,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(const __g
         __syncwarp();  // the read's parameters are in memory for the warp
         if (!r.skip) {
             if (r.ck)
-                fill_warp_ck<kScores>(a, r, smem_u32(&sm.warp_rings[warp]), lane);
+                fill_warp<kScores, true>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
             else
                 fill_warp<kScores, false>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
         }
@@ -2951,7 +2950,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
         const ReadDesc& r = a.reads[ri];
         if (!r.skip) {
             if (r.ck)
-                fill_warp_ck<kScores>(a, r, smem_u32(&sm.warp_rings[warp]), lane);
+                fill_warp<kScores, true>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
             else
                 fill_warp<kScores, false>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
         }
