@@ -100,6 +100,10 @@ struct abea_batch {
     // sizes
     int64_t seq_bytes = 0, n_events_total = 0, ev_pad_total = 0, km_pad_total = 0,
             band_pad_total = 0, pair_cap = 0, band_cells = 0;
+    // what the backward pass chooses its launch by: events of the longest read and of all, and
+    // the reads with short paths (adj_short) and their events
+    int32_t adj_longest = 0, adj_short_n = 0;
+    int64_t adj_events = 0, adj_short_events = 0;
     int64_t trace_pad_total = 0;  // bands of kept traces
     int64_t ck_floats = 0;        // checkpoint records
     int32_t n_ck = 0;             // checkpointed reads (recompute scratch slots)
@@ -426,8 +430,18 @@ static abea_status_t plan(abea_batch* b, const HostInputs& in, int var_aware, in
     b->ck_floats = ckf;
     b->n_ck = n_ck;
     int32_t n_spec = 0;
-    for (const ReadDesc& r : b->reads)
-        if (!r.skip && r.n_bands >= kSpecMinBands) ++n_spec;
+    b->adj_longest = b->adj_short_n = 0;
+    b->adj_events = b->adj_short_events = 0;
+    for (const ReadDesc& r : b->reads) {
+        if (r.skip) continue;
+        if (r.n_bands >= kSpecMinBands) ++n_spec;
+        b->adj_longest = std::max(b->adj_longest, r.n_events);
+        b->adj_events += r.n_events;
+        if (adj_short(r)) {
+            ++b->adj_short_n;
+            b->adj_short_events += r.n_events;
+        }
+    }
     // one scratch slot per block that starts on a wide read (a block walks one wide read
     // at a time and keeps its slot; the first picks take the longest reads, so at most
     // one slot per qualifying read)
@@ -1143,16 +1157,18 @@ extern "C" abea_status_t abea_batch_read_bands(abea_ctx_t* c, abea_batch_t* b, i
 static abea_status_t queue_backward(abea_ctx* c, abea_batch* b, bool model_grad) {
     if (model_grad)
         CUDA_TRY(cudaMemsetAsync(b->d_grad_model, 0, sizeof(double) * 2 * ABEA_NUM_KMER, c->stream));
-    // One block per read takes as long as the longest read or the SMs' share of all of
-    // them, whichever is more: where the longest read decides, a cluster per read.
-    int64_t longest = 0, all = 0;
-    for (const ReadDesc& r : b->reads) {
-        longest = std::max<int64_t>(longest, r.n_events);
-        all += r.n_events;
-    }
+    // Where short paths are most of the work, in more reads than blocks fit the SMs (8 each),
+    // they go to a warp each (the other reads then wait for them: a launch of their own).
+    // One block per read takes as long as the longest read or the SMs' share of all of them,
+    // whichever is more: where the longest read decides, and its path may have more than one
+    // part, a cluster per read (152 reads of 600 bases, one part each: the call 0.18 ms with
+    // clusters, 0.08 without).
+    const bool warps = b->adj_short_n > 8 * c->sm_count && 2 * b->adj_short_events > b->adj_events;
+    const bool split = !warps && 2 * (int64_t)b->adj_longest >= kAdjPart &&
+                       (int64_t)b->adj_longest * c->sm_count > b->adj_events;
     AdjArgs a{b->d_reads, b->n_reads, b->var_aware, b->d_seq, b->d_model, b->d_ev_mean, b->d_pairs,
               b->d_path_len, b->d_path_flags, b->d_grad_sc, b->d_gn, b->d_path_em,
-              model_grad ? b->d_grad_model : nullptr, b->d_adj_status, longest * c->sm_count > all};
+              model_grad ? b->d_grad_model : nullptr, b->d_adj_status, split, warps ? b->adj_short_n : 0};
     cudaError_t e = launch_adjoint(a, c->stream);
     if (e != cudaSuccess) return fail(ABEA_ERR_CUDA, "adjoint launch failed: %s", cudaGetErrorString(e));
     return ABEA_OK;

@@ -3237,7 +3237,70 @@ extern "C" abea_status_t abea_align_noalloc(abea_aligned_pair_t* pairs, int32_t*
 namespace abea {
 
 constexpr int kAdjThreads = 256, kAdjSums = 9;
-constexpr int kAdjPart = 4096;  // least cells of a part
+
+// A read's path as the backward pass walks it.
+struct AdjPath {
+    const AdjArgs& a;
+    const ReadDesc r;
+    int len, flags, st, cells;
+    __device__ __forceinline__ AdjPath(const AdjArgs& args, int ri) : a(args), r(args.reads[ri]) {
+        len = r.skip ? 0 : a.path_len[ri];
+        flags = r.skip ? 0 : a.path_flags[ri];
+        st = 0;
+        if (len > 0 && (flags & (kPathTruncated | kPathNoEnd | kPathError)))
+            st = (flags & kPathTruncated) ? ABEA_ERR_CAPACITY : ABEA_ERR_UNDEFINED;
+        cells = st == 0 ? max(len, 0) : 0;
+    }
+    // adds path position j's terms: shift, scale, var, j11, j12, j22, t1, t2, em
+    __device__ __forceinline__ void add(int j, double (&acc)[kAdjSums]) const {
+        const abea_aligned_pair_t* out = a.pairs + r.out_off;
+        const bool rev = (flags & kPathReversed) != 0;
+        const int w = rev ? len - 1 - j : j;  // walk position, 0 = best end
+        const abea_aligned_pair_t c = out[j];
+        bool counted;
+        if (w < len - 1) {
+            const abea_aligned_pair_t nx = rev ? out[j - 1] : out[j + 1];
+            counted = nx.read_pos == c.read_pos - 1;  // D or U: the next walked cell is one event back
+        } else {
+            counted = flags >> 8 != (int)ABEA_FROM_L;
+        }
+        if (!counted) return;
+        const char* s = a.seq + r.seq_off;
+        uint32_t rank = 0;
+#pragma unroll
+        for (int q = 0; q < ABEA_KMER_SIZE; ++q) rank = (rank << 2) | base_rank(s[c.ref_pos + q]);
+        const abea_model_t m = a.model[rank];
+        const double scale = r.scale, shift = r.shift, var = r.var, log_var = r.log_var;
+        const double mu = m.level_mean, sig = m.level_stdv;
+        const double sd = a.var_aware ? sig * var : sig;
+        const double lsd = a.var_aware ? (double)m.level_log_stdv + log_var : (double)m.level_log_stdv;
+        const double x = a.ev_mean[r.ev_off + c.read_pos];
+        const double isd = 1.0 / sd;
+        const double av = (x - (scale * mu + shift)) * isd;
+        acc[0] += av * isd;
+        acc[1] += av * mu * isd;
+        if (a.var_aware) acc[2] += (av * av - 1.0) / var;
+        acc[3] += isd * isd;
+        acc[4] += mu * isd * isd;
+        acc[5] += mu * mu * isd * isd;
+        acc[6] -= av * isd;
+        acc[7] -= av * mu * isd;
+        acc[8] += -0.91893853320467274 - lsd - 0.5 * av * av;
+        if (a.grad_model) {
+            atomicAdd(&a.grad_model[2 * rank], av * scale * isd);
+            atomicAdd(&a.grad_model[2 * rank + 1], (av * av - 1.0) / sig);
+        }
+    }
+};
+// Sum i of read ri.
+__device__ __forceinline__ void adj_write(const AdjArgs& a, int ri, int i, double v) {
+    if (i < 3)
+        a.grad_scalings[3 * ri + i] = v;
+    else if (i < 8)
+        a.gn[5 * ri + i - 3] = v;
+    else
+        a.path_em[ri] = v;
+}
 
 template <int kBlocks>
 __global__ void __cluster_dims__(kBlocks, 1, 1) __launch_bounds__(kAdjThreads) abea_adjoint_kernel(AdjArgs a) {
@@ -3247,77 +3310,48 @@ __global__ void __cluster_dims__(kBlocks, 1, 1) __launch_bounds__(kAdjThreads) a
     const int ri = blockIdx.x / kBlocks, rank = blockIdx.x % kBlocks;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     if (kBlocks > 1) cg::this_cluster().sync();  // every block of the cluster runs before its memory is written
-    const ReadDesc r = a.reads[ri];
-    const int len = r.skip ? 0 : a.path_len[ri];
-    const int flags = r.skip ? 0 : a.path_flags[ri];
-    int st = 0;
-    if (len > 0 && (flags & (kPathTruncated | kPathNoEnd | kPathError)))
-        st = (flags & kPathTruncated) ? ABEA_ERR_CAPACITY : ABEA_ERR_UNDEFINED;
-    const int cells = st == 0 ? max(len, 0) : 0;
+    const AdjPath p(a, ri);
+    if (kBlocks == 1 && a.n_warp && adj_short(p.r)) return;  // abea_adjoint_warp_kernel's
+    const int cells = p.cells;
     const int parts = min(kAdjSplit, 1 + cells / kAdjPart), per_part = (cells + parts - 1) / parts;
-    const abea_aligned_pair_t* out = a.pairs + r.out_off;
-    const bool rev = (flags & kPathReversed) != 0;
-    const int last_from = flags >> 8;
-    const char* s = a.seq + r.seq_off;
-    const double scale = r.scale, shift = r.shift, var = r.var, log_var = r.log_var;
+    // A short path's cells 256 at a time (a thread's one cell each), their terms added lane by
+    // lane over the rows; a longer one's parts whole, each thread's sum first.
+    const int step = cells <= kAdjShort ? kAdjThreads : per_part;
     for (int part = rank; part < parts; part += kBlocks) {
-        double acc[kAdjSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // shift, scale, var, j11, j12, j22, t1, t2, em
-        const int end = min(cells, (part + 1) * per_part);
-        for (int j = part * per_part + t; j < end; j += kAdjThreads) {
-            const int w = rev ? len - 1 - j : j;  // walk position, 0 = best end
-            const abea_aligned_pair_t c = out[j];
-            bool counted;
-            if (w < len - 1) {
-                const abea_aligned_pair_t nx = rev ? out[j - 1] : out[j + 1];
-                counted = nx.read_pos == c.read_pos - 1;  // D or U: the next walked cell is one event back
-            } else {
-                counted = last_from != (int)ABEA_FROM_L;
-            }
-            if (!counted) continue;
-            uint32_t rank_k = 0;
+        const int first = part * per_part, end = min(cells, first + per_part);
+        double v[2] = {0.0, 0.0};  // this warp's one or two sums
+        for (int at = first; at < end || at == first; at += step) {
+            double acc[kAdjSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+            for (int j = at + t; j < min(end, at + step); j += kAdjThreads) p.add(j, acc);
+            // A warp per sum: 3,700 additions, a third of butterflies over every warp (which
+            // were a fifth of the FP64 work of a 600-base read).
 #pragma unroll
-            for (int q = 0; q < ABEA_KMER_SIZE; ++q) rank_k = (rank_k << 2) | base_rank(s[c.ref_pos + q]);
-            const abea_model_t m = a.model[rank_k];
-            const double mu = m.level_mean, sig = m.level_stdv;
-            const double sd = a.var_aware ? sig * var : sig;
-            const double lsd = a.var_aware ? (double)m.level_log_stdv + log_var : (double)m.level_log_stdv;
-            const double x = a.ev_mean[r.ev_off + c.read_pos];
-            const double isd = 1.0 / sd;
-            const double av = (x - (scale * mu + shift)) * isd;
-            acc[0] += av * isd;
-            acc[1] += av * mu * isd;
-            if (a.var_aware) acc[2] += (av * av - 1.0) / var;
-            acc[3] += isd * isd;
-            acc[4] += mu * isd * isd;
-            acc[5] += mu * mu * isd * isd;
-            acc[6] -= av * isd;
-            acc[7] -= av * mu * isd;
-            acc[8] += -0.91893853320467274 - lsd - 0.5 * av * av;
-            if (a.grad_model) {
-                atomicAdd(&a.grad_model[2 * rank_k], av * scale * isd);
-                atomicAdd(&a.grad_model[2 * rank_k + 1], (av * av - 1.0) / sig);
+            for (int i = 0; i < kAdjSums; ++i) sums[i][t] = acc[i];
+            __syncthreads();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = warp + h * (kAdjThreads / 32);
+                if (i < kAdjSums)
+#pragma unroll
+                    for (int q = 0; q < kAdjThreads; q += 32) v[h] += sums[i][q + lane];
             }
+            __syncthreads();  // the sums may be written again
         }
-        // A warp per sum: 3,700 additions, a third of butterflies over every warp (which were
-        // a fifth of the FP64 work of a 600-base read).
 #pragma unroll
-        for (int i = 0; i < kAdjSums; ++i) sums[i][t] = acc[i];
-        __syncthreads();
-        for (int i = warp; i < kAdjSums; i += kAdjThreads / 32) {
-            double v = sums[i][lane];
+        for (int h = 0; h < 2; ++h) {
+            const int i = warp + h * (kAdjThreads / 32);
+            if (i >= kAdjSums) continue;
 #pragma unroll
-            for (int q = 32; q < kAdjThreads; q += 32) v += sums[i][q + lane];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFull, v, off);
+            for (int off = 16; off > 0; off >>= 1) v[h] += __shfl_xor_sync(kFull, v[h], off);
             if (lane == 0) {
                 if (kBlocks > 1)
-                    *cg::this_cluster().map_shared_rank(&part_sums[part][i], 0) = v;
+                    *cg::this_cluster().map_shared_rank(&part_sums[part][i], 0) = v[h];
                 else
-                    part_sums[part][i] = v;
+                    part_sums[part][i] = v[h];
             }
         }
-        __syncthreads();  // the sums may be written again; part_sums is
     }
+    __syncthreads();
     if (kBlocks > 1) {
         cg::this_cluster().sync();  // the other blocks' sums are in the first block's memory
         if (rank != 0) return;
@@ -3325,14 +3359,29 @@ __global__ void __cluster_dims__(kBlocks, 1, 1) __launch_bounds__(kAdjThreads) a
     if (t < kAdjSums) {
         double v = 0.0;
         for (int i = 0; i < parts; ++i) v += part_sums[i][t];
-        if (t < 3)
-            a.grad_scalings[3 * ri + t] = v;
-        else if (t < 8)
-            a.gn[5 * ri + t - 3] = v;
-        else
-            a.path_em[ri] = v;
+        adj_write(a, ri, t, v);
     }
-    if (t == 0) a.adj_status[ri] = st;
+    if (t == 0) a.adj_status[ri] = p.st;
+}
+
+// Many short reads: a warp per read.  A block per read leaves eight reads on an SM, and the
+// latency of a read's loads and of its reduction is then the bound (20,000 reads of 50-120
+// bases 0.60 ms a call, as warps 0.46).
+__global__ void __launch_bounds__(32) abea_adjoint_warp_kernel(AdjArgs a) {
+    const int ri = blockIdx.x, lane = threadIdx.x;
+    const AdjPath p(a, ri);
+    if (!adj_short(p.r)) return;
+    double v[kAdjSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (int j = lane; j < p.cells; j += 32) p.add(j, v);
+#pragma unroll
+    for (int i = 0; i < kAdjSums; ++i)
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v[i] += __shfl_xor_sync(kFull, v[i], off);
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < kAdjSums; ++i) adj_write(a, ri, i, v[i]);
+        a.adj_status[ri] = p.st;
+    }
 }
 
 // One warp per read took as long as the longest read: 1.7 ms of 512 reads of 1-10 kb, now
@@ -3341,8 +3390,9 @@ cudaError_t launch_adjoint(const AdjArgs& a, cudaStream_t stream) {
     if (a.n_reads <= 0) return cudaSuccess;
     if (a.split)
         abea_adjoint_kernel<kAdjSplit><<<a.n_reads * kAdjSplit, kAdjThreads, 0, stream>>>(a);
-    else
+    else if (a.n_warp < a.n_reads)
         abea_adjoint_kernel<1><<<a.n_reads, kAdjThreads, 0, stream>>>(a);
+    if (a.n_warp > 0) abea_adjoint_warp_kernel<<<a.n_reads, 32, 0, stream>>>(a);
     return cudaGetLastError();
 }
 

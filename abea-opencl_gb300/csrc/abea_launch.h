@@ -112,8 +112,14 @@ struct AdjArgs {
     double* grad_model;     // [4096][2]: d/d level_mean, level_stdv, summed over reads
     int32_t* adj_status;    // [n]: 0, or why the read has no gradient
     int split;              // a cluster of kAdjSplit blocks per read instead of one block
+    int n_warp;             // reads (adj_short) that a warp each takes; 0: none, the other kernel takes all
 };
 constexpr int kAdjSplit = 8;
+// Paths of at most kAdjShort cells are summed lane by lane: cells l, l + 32, l + 64, ... in turn.
+constexpr int kAdjShort = 1024;
+// A read whose path is surely one of those: each move steps back an event, a k-mer or both.
+__host__ __device__ inline bool adj_short(const ReadDesc& r) { return r.n_events + (int64_t)r.n_kmers <= kAdjShort; }
+constexpr int kAdjPart = 4096;  // a path is cut into one part more for each so many cells
 
 // Backward pass over the stored paths of a finished forward run.
 cudaError_t launch_adjoint(const AdjArgs& a, cudaStream_t stream);

@@ -280,3 +280,25 @@ def test_gpu_adjoint_in_parts(oracle_mod, length):
     out = dev.backward()
     for key in ("grad_scalings", "path_emission"):
         assert np.array_equal(out[key], np.repeat(one[key][:1], 153, axis=0)), key
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length", [8, 25, 100, 140, 160, 330, 360, 375, 390])
+def test_gpu_adjoint_of_many_short_reads(length):
+    """More short reads than resident blocks, each by one warp: the same
+    bits as alone, one block per read, for paths around 32 and 256 cells, and around the limit
+    of 1,024 events and k-mers."""
+    from abea_gb300 import synth
+    b = synth.make_batch("adjoint", seed=32, lengths=[length])
+    ctx = abea.Context(0, abea.MODE_BATCHED)
+    dev = ctx.upload(b)
+    dev.run()
+    one = dev.backward()
+    seq, ev = read_of(b, 0)
+    many = abea.from_reads([seq] * 1300, [ev] * 1300, np.repeat(b.scalings[:1], 1300), b.model)
+    dev = ctx.upload(many)
+    dev.run()
+    out = dev.backward()
+    for key in ("grad_scalings", "path_emission", "status"):
+        assert np.array_equal(out[key], np.repeat(one[key][:1], 1300, axis=0)), key
+    assert np.allclose(out["grad_model"], 1300 * one["grad_model"], rtol=1e-9, atol=1e-9)
