@@ -1422,7 +1422,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
         pend = false;
         char* const sc = reinterpret_cast<char*>(&ws.sc[0][0]);
         constexpr int kRow = 4 * kSlots, kRows = kScoreRing * kRow;
-        int rw = (kWideChunk * j * kRow) & (kRows - 1);  // byte offset of the chunk's first score row
+        int rw = (int)((unsigned)(kWideChunk * kRow) * (unsigned)j & (kRows - 1));  // byte offset of the chunk's first score row
         int row0 = (rw - kRow) & (kRows - 1);            // and of the row before it
         while (true) {
             kb_cur = kb;
