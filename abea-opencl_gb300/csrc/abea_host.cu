@@ -152,7 +152,7 @@ struct abea_ctx {
     int64_t store_scores = 0;
     int64_t use_graph = 1;
     int64_t long_read_bands = 0;
-    int64_t mid_read_bands = 0;  // a second wide-shape threshold (ABEA_OPT_MEDIUM_READ_BANDS; 0 = the autotuned value, else none)
+    int64_t mid_read_bands = 0;  // a second wide-shape threshold (ABEA_OPT_MEDIUM_READ_BANDS; 0 = none)
     int64_t spin_limit = 1 << 22;
     int64_t var_aware = 0;
     int64_t trace_budget = 0;  // bytes of trace a read may keep (0 = every trace)
@@ -172,7 +172,6 @@ struct abea_ctx {
     char* h_aux = nullptr;  // pinned: abea_align_batch's mirrors, then its counters and statuses
     size_t h_aux_bytes = 0;
     std::map<uint64_t, int64_t> tuned;      // autotuned wide-shape threshold per workload signature
-    std::map<uint64_t, int64_t> tuned_mid;  // second wide threshold per workload signature, from a cache file
 };
 
 // ---------------------------------------------------------------- context
@@ -757,21 +756,17 @@ static abea_status_t queue_work(abea_ctx* c, abea_batch* b, int* launches, bool 
 
 // The batched form's order: wide reads (threshold from the option, else the
 // autotuned value of this workload signature, else the heuristic; and a second one from
-// the option, else from a cache file, else none), then the rest.
+// the option, if set), then the rest.
 static void prepare_order(abea_ctx* c, abea_batch* b) {
     b->n_wide = 0;
     if (c->mode != ABEA_MODE_BATCHED) return;
     const uint64_t sig = workload_signature(b);
-    int64_t thr = c->long_read_bands, mid = c->mid_read_bands;
+    int64_t thr = c->long_read_bands;
     if (thr == 0) {
         auto it = c->tuned.find(sig);
         if (it != c->tuned.end()) thr = it->second;
     }
-    if (mid == 0) {
-        auto it = c->tuned_mid.find(sig);
-        if (it != c->tuned_mid.end()) mid = it->second;
-    }
-    choose_shape_reads(b, c->sm_count, thr, mid, b->scores_kept, c->wide_cluster != 0);
+    choose_shape_reads(b, c->sm_count, thr, c->mid_read_bands, b->scores_kept, c->wide_cluster != 0);
 }
 
 static abea_status_t run_batch(abea_ctx* c, abea_batch* b) {
@@ -853,8 +848,7 @@ extern "C" abea_status_t abea_autotune(abea_ctx_t* c, abea_batch_t* b, int64_t* 
     const abea_mode_t mode0 = c->mode;
     const int64_t thr0 = c->long_read_bands, mid0 = c->mid_read_bands;
     c->mode = ABEA_MODE_BATCHED;
-    // without a second threshold: neither the option's nor one from a cache file may
-    // shape the timings
+    // without a second threshold: the option's may not shape the timings
     c->mid_read_bands = INT64_MAX;
     const int blocks = batched_blocks_per_sm(b->scores_kept) * c->sm_count;
     int64_t longest = 0;
@@ -899,25 +893,22 @@ extern "C" abea_status_t abea_autotune(abea_ctx_t* c, abea_batch_t* b, int64_t* 
     c->mid_read_bands = mid0;
     if (st) return st;
     c->tuned[workload_signature(b)] = best;
-    c->tuned_mid.erase(workload_signature(b));  // of an older cache file
     if (best_threshold) *best_threshold = best;
     if (best_ms) *best_ms = best_t;
     return ABEA_OK;
 }
 
 // Autotuner cache: "abea-autotune 2 sm_count <n>" then "<signature> <wide threshold>
-// <second threshold>" lines (INT64_MAX = none).  Version 1 files (no second
-// threshold) are read too.
+// INT64_MAX" lines.  The third field was the threshold of a medium shape (two reads per
+// block): a line that has one was tuned with it and is left to the heuristic, as one wide
+// read per block is what no one tuned its reads for.  Version 1 files have no third field.
 extern "C" abea_status_t abea_autotune_save(abea_ctx_t* c, const char* path, int32_t* n_entries) {
     if (!c || !path) return fail(ABEA_ERR_INVALID_ARG, "abea_autotune_save: null argument");
     FILE* f = fopen(path, "w");
     if (!f) return fail(ABEA_ERR_INVALID_ARG, "abea_autotune_save: cannot open %s", path);
     fprintf(f, "abea-autotune 2 sm_count %d\n", c->sm_count);
-    for (const auto& kv : c->tuned) {
-        auto m = c->tuned_mid.find(kv.first);
-        fprintf(f, "%llu %lld %lld\n", (unsigned long long)kv.first, (long long)kv.second,
-                (long long)(m == c->tuned_mid.end() ? INT64_MAX : m->second));
-    }
+    for (const auto& kv : c->tuned)
+        fprintf(f, "%llu %lld %lld\n", (unsigned long long)kv.first, (long long)kv.second, (long long)INT64_MAX);
     const bool ok = fclose(f) == 0;
     if (!ok) return fail(ABEA_ERR_INVALID_ARG, "abea_autotune_save: write to %s failed", path);
     if (n_entries) *n_entries = (int32_t)c->tuned.size();
@@ -955,8 +946,10 @@ extern "C" abea_status_t abea_autotune_load(abea_ctx_t* c, const char* path, int
     fclose(f);
     if (!at_end) return fail(ABEA_ERR_INVALID_ARG, "abea_autotune_load: malformed line in %s", path);
     for (const auto& kv : got) {
-        c->tuned[kv.first] = kv.second.first;
-        c->tuned_mid[kv.first] = kv.second.second;
+        if (kv.second.second == INT64_MAX)
+            c->tuned[kv.first] = kv.second.first;
+        else
+            c->tuned.erase(kv.first);
     }
     if (n_entries) *n_entries = (int32_t)got.size();
     return ABEA_OK;

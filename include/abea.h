@@ -140,7 +140,7 @@ typedef enum {
                                    memory); 0 = one block per wide read */
     ABEA_OPT_MEDIUM_READ_BANDS = 8 /* BATCHED: a second threshold: reads with at least this many bands
                                    run on the wide shape too (it once chose a medium shape of two
-                                   reads per block); 0 = that of a loaded cache file, else none */
+                                   reads per block); 0 = none */
 } abea_option_t;
 
 typedef struct abea_ctx abea_ctx_t;

@@ -446,3 +446,32 @@ def test_more_wide_reads_than_blocks(lib, workload):
     pp, pc = pdev.results()
     assert_same_alignments(batch, gp, gc, pp, pc)
     assert np.array_equal(gb.view(np.uint32), pdev.best_scores().view(np.uint32))
+
+
+def test_cache_lines_tuned_with_the_medium_shape_are_left_to_the_heuristic(lib, tmp_path):
+    """A cache line's third field was the threshold of a shape with two reads per block: such a
+    line loads, and its workload runs as an untuned one does."""
+    from abea_gb300 import synth
+    batch = synth.make_batch("small", seed=9)
+    ctx = abea.Context(0, abea.MODE_BATCHED)
+    ctx.upload(batch).autotune()
+    path = str(tmp_path / "tuned.txt")
+    assert ctx.autotune_save(path) == 1
+    head, line = open(path).read().split("\n")[:2]
+    sig = line.split()[0]
+    (tmp_path / "medium.txt").write_text(f"{head}\n{sig} {1 << 40} 1\n")
+
+    def warp_reads_slow(c):  # what tells the shapes apart: the cells that take FP64
+        dev = c.upload(batch)
+        dev.run()
+        dev.results()
+        return dev._counters()["fp64"]
+
+    fresh = abea.Context(0, abea.MODE_BATCHED)
+    untuned = warp_reads_slow(fresh)
+    for name, tuned in (("medium.txt", False), ("none.txt", True)):
+        (tmp_path / "none.txt").write_text(f"{head}\n{sig} {1 << 40} {2**63 - 1}\n")
+        other = abea.Context(0, abea.MODE_BATCHED)
+        assert other.autotune_load(str(tmp_path / name)) == 1
+        assert (warp_reads_slow(other) != untuned) == tuned
+        assert other.autotune_save(path) == (1 if tuned else 0)
