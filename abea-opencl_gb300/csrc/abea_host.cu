@@ -2085,10 +2085,9 @@ extern "C" const char* abea_internal_set_error(const char* msg) {
 // The batched form's heuristic wide-shape threshold for a batch of reads with
 // these band counts on `blocks` resident blocks (no device needed): for tests
 // and for callers who size batches.  INT64_MAX = no wide read; -1 = bad input.
-// The heuristic on band counts alone (host code, for tests); ck (optional) marks
-// checkpointed reads, which stay on the warp shape (as with the cluster pair).
-extern "C" int64_t abea_internal_wide_threshold_ck(const int64_t* n_bands, const int32_t* ck, int32_t n_reads,
-                                                   int32_t blocks) {
+// ck (optional) marks checkpointed reads: with `pair` they stay on the warp shape, as they
+// do on the cluster pair; without, they may be wide, as everywhere else.
+static int64_t threshold_of(const int64_t* n_bands, const int32_t* ck, int32_t n_reads, int32_t blocks, bool pair) {
     if (n_reads < 0 || blocks < 1 || (n_reads > 0 && !n_bands)) return -1;
     abea_batch b;
     b.n_reads = n_reads;
@@ -2103,7 +2102,17 @@ extern "C" int64_t abea_internal_wide_threshold_ck(const int64_t* n_bands, const
     std::stable_sort(b.order.begin(), b.order.end(), [&](int32_t x, int32_t y) {
         return b.reads[(size_t)x].n_bands > b.reads[(size_t)y].n_bands;
     });
-    return heuristic_threshold(&b, blocks, false);
+    return heuristic_threshold(&b, blocks, !pair);
+}
+
+extern "C" int64_t abea_internal_wide_threshold_ck(const int64_t* n_bands, const int32_t* ck, int32_t n_reads,
+                                                   int32_t blocks) {
+    return threshold_of(n_bands, ck, n_reads, blocks, true);
+}
+
+extern "C" int64_t abea_internal_wide_threshold_any(const int64_t* n_bands, const int32_t* ck, int32_t n_reads,
+                                                    int32_t blocks) {
+    return threshold_of(n_bands, ck, n_reads, blocks, false);
 }
 
 extern "C" int64_t abea_internal_wide_threshold(const int64_t* n_bands, int32_t n_reads, int32_t blocks) {

@@ -100,3 +100,35 @@ def test_checkpointed_reads_keep_the_split():
     thr = f(nb.ctypes.data, ck.ctypes.data, len(nb), 152)
     k = int(np.sum((nb >= thr) & (ck == 0)))
     assert thr > 1 and 0 < k < 152, (thr, k)
+
+
+def threshold_any(nb, ck, blocks=152):
+    if not os.path.exists(abea.LIB_PATH):
+        abea.build()
+    f = abea.lib().abea_internal_wide_threshold_any
+    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32]
+    f.restype = C.c_int64
+    nb = np.ascontiguousarray(nb, dtype=np.int64)
+    ck = np.ascontiguousarray(ck, dtype=np.int32)
+    return f(nb.ctypes.data, ck.ctypes.data, len(nb), blocks)
+
+
+def test_checkpointed_reads_may_be_wide():
+    """The rule without the cluster pair: a long checkpointed read, and every read of a
+    latency-bound batch with or without them, go wide (one read of 9 kb checkpointed 5.3 ms
+    wide, 31 on a warp); many short checkpointed reads per SM stay on the warp shape (2,400 of
+    1 kb: 13.0 ms against 18.7)."""
+    from abea_gb300 import synth
+    assert threshold_any([24928], [1]) == 1
+    nb = synth.make_batch("f5c_batch", seed=1).n_bands()
+    none = np.zeros(len(nb), dtype=np.int32)
+    assert threshold_any(nb, none) == 1 == threshold_any(nb, none + 1)
+    some = none.copy()
+    some[np.argsort(-nb)[:10]] = 1  # the ten longest
+    assert threshold_any(nb, some) == 1
+    # one long checkpointed read among many short ones: it alone where the short ones would
+    # then be the longer part, every read where it bounds the batch
+    ck = np.array([1] + [0] * 2432, dtype=np.int32)
+    assert 1759 < threshold_any([24928] + [1759] * 2432, ck) <= 24928
+    assert threshold_any([54000] + [1759] * 2432, ck) == 1
+    assert threshold_any([3413] * 2400, [1] * 2400) >= 2**62
