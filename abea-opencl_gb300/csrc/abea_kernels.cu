@@ -101,11 +101,13 @@ __device__ __forceinline__ CellConsts make_consts(const ReadDesc& r, const Globa
 // to host memory are in flight at once: a warp-shape read's pre stage is latency-
 // bound on them (a k-mer's six bases share the cache lines of its neighbours').
 constexpr int kPreUnroll = 4, kEvUnroll = 16;
-// Returns whether some k-mer of this thread's is none for a grid (grid_kmer_ok).
+// kWide: the read's parameters side by side too (km4), for the wide shape; returns whether
+// some k-mer of this thread's is none for a grid (grid_kmer_ok).
+template <bool kWide>
 __device__ __forceinline__ bool pre_read(const PreArgs& a, int i, int t, int nt) {
     const ReadDesc r = a.reads[i];
     if (r.skip) return false;
-    const float k1_max = grid_k1_max(r.step_h, r.stay_h);
+    const float k1_max = kWide ? grid_k1_max(r.step_h, r.stay_h) : 0.0f;
     bool odd = false;
     const InMirror* m = r.in_hbm ? nullptr : a.inm;
     const char* seq = a.seq;
@@ -146,13 +148,13 @@ __device__ __forceinline__ bool pre_read(const PreArgs& a, int i, int t, int nt)
                 }
                 rsd = __frcp_rn(sd);
                 k1 = __fsub_rn(kLogInvSqrt2Pi, lsd);
-                odd |= !grid_kmer_ok(sd, k1, k1_max);
+                if (kWide) odd |= !grid_kmer_ok(sd, k1, k1_max);
             }
             a.km_gm[r.km_off + k] = gm;
             a.km_sd[r.km_off + k] = sd;
             a.km_rsd[r.km_off + k] = rsd;
             a.km_k1[r.km_off + k] = k1;
-            if (a.km4) a.km4[r.km_off + k] = make_float4(gm, sd, rsd, k1);
+            if (kWide) a.km4[r.km_off + k] = make_float4(gm, sd, rsd, k1);
         }
     }
     const int ne = r.n_events, ne_pad = round_up_dev(ne);
@@ -175,7 +177,7 @@ __device__ __forceinline__ bool pre_read(const PreArgs& a, int i, int t, int nt)
 __global__ void __launch_bounds__(128) abea_pre_kernel(PreArgs a) {
     const int i = blockIdx.x;
     if (i >= a.n_reads) return;
-    pre_read(a, i, threadIdx.x, blockDim.x);
+    pre_read<false>(a, i, threadIdx.x, blockDim.x);
 }
 
 // ---------------------------------------------------------------- prefetch rings
@@ -2836,7 +2838,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(const __g
     const int free_rank = sm.free_rank, wide_slot = sm.wide_slot;
     while (wide_read >= 0) {
         const ReadDesc& r = a.reads[wide_read];
-        const bool odd = __syncthreads_or(pre_read(pa, wide_read, t, kWideThreads));  // the read's parameters are in memory for the whole block
+        const bool odd = __syncthreads_or(pre_read<true>(pa, wide_read, t, kWideThreads));  // and its parameters are in memory
         bool filled = true;
         if (!r.skip) {
             if (r.ck)
@@ -2884,7 +2886,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(const __g
         }
         const int ri = a.order[a.n_wide + q];
         const ReadDesc& r = a.reads[ri];
-        pre_read(pa, ri, lane, 32);
+        pre_read<false>(pa, ri, lane, 32);
         __syncwarp();  // the read's parameters are in memory for the warp
         if (!r.skip) {
             if (r.ck)

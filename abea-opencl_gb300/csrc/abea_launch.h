@@ -32,7 +32,7 @@ struct PreArgs {
     float* km_k1;
     float* last_col;
     const InMirror* inm;  // nullptr, or a device copy of the input mirror
-    float4* km4;          // the four k-mer parameters side by side, for the wide shape (nullptr: not wanted)
+    float4* km4;          // the four k-mer parameters side by side, written for a wide read only
 };
 
 // What a run counts: band cells computed again because the band loop's FP32 proof did not

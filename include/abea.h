@@ -133,7 +133,9 @@ typedef enum {
                                    reference ignores var, GPU/align_cuda.cl:509); taken at batch creation */
     ABEA_OPT_TRACE_BUDGET = 6,  /* bytes of backpointers a read may keep in HBM (128 per band); a read
                                    needing more keeps band-score checkpoints every 256 bands (4 bytes per
-                                   band) and its traceback recomputes the trace 256 bands at a time.
+                                   band) and its traceback recomputes the trace 256 bands at a time (32 KB of
+                                   scratch per such read; the batched form also takes 512 KB for each of
+                                   512 bands or more, at most one per SM, to recompute 16 times 256 at once).
                                    0 (default) = keep every trace.  Taken at batch creation. */
     ABEA_OPT_WIDE_CLUSTER = 7,  /* BATCHED: 1 = the longest reads run on a cluster of two blocks (the
                                    second SM computes the emissions ahead into the first one's shared
