@@ -909,11 +909,6 @@ struct WideRead {
         rec[2 * kSlots] = __int_as_float(k0);
         rec[2 * kSlots + 1] = __int_as_float(kWideChunk * j + 1 - k0);  // the event of band 4j + 3
     }
-    // whether k-mer k may be on a grid
-    __device__ __forceinline__ bool grid_kmer(int k) const {
-        const float4 km = a.km4[r.km_off + k];
-        return grid_kmer_ok(km.y, km.w, grid_k1_max(cc.step_h, cc.stay_h));
-    }
     // the end cells of band b-1 (its row of the ring) and the left neighbour of a slot
     __device__ __forceinline__ void ends(int row, int k0, float& ll, float& ur) const {
         ll = ws.sc[row][k0 & (kSlots - 1)];
@@ -1597,8 +1592,11 @@ __device__ __noinline__ bool fill_chain(const CoreArgs& a, const ReadDesc& r, un
         if (odd) {
             // up to the next k-mer that is none for a grid, looked for among the next 4,096
             const int k_from = max(kp, 0), k_stop = min(w.n_kmers, k_from + 8 * kWideThreads);
+            const float4* km4 = a.km4 + r.km_off;
+            const float k1_max = grid_k1_max(r.step_h, r.stay_h);
+#pragma unroll 1
             for (int k = k_from + tid; k < k_stop; k += kWideThreads)
-                if (!w.grid_kmer(k)) atomicMin(&ws.k_odd, k);
+                if (!grid_kmer_ok(km4[k].y, km4[k].w, k1_max)) atomicMin(&ws.k_odd, k);
             __syncthreads();
             k_end = min(k_stop, ws.k_odd);
         }
