@@ -604,6 +604,10 @@ static int64_t d2h_bytes(const abea_batch* b) {
 // longest read, or all of them over the blocks.  That wins when it is within 2% of
 // the first and either the longest read bounds it or there are at most 8 reads per
 // block, unless there are reads that may not be wide: those would start last.
+// Between the two, every checkpointed read (a batch's longest) on the wide shape: on the
+// warp shape each runs its bands twice beside fifteen others (4,096 reads of 1-10 kb, 894 of
+// them checkpointed: 55 ms; with none wide 55, with scalings off by some percent, whose bands
+// leave the grids, 75).
 // Calibrated on GB300 (ms, every read wide / none): 1,024 reads of 1-10 kb 11.8 / 14.3,
 // 608 reads of 3 kb 4.90 / 5.74, 1,216 of 3 kb 9.30 / 6.78, 2,432 of 3 kb 18.9 / 9.7
 // (sixteen warps on an SM take 131 cycles per band together, one wide read 200-290),
@@ -642,8 +646,17 @@ static int64_t heuristic_threshold(const abea_batch* b, int blocks, bool ck_wide
     const size_t n = b->order.size();
     std::vector<const ReadDesc*> wide_ok;  // the reads that may be wide, longest first
     double rest_bands = 0, rest_start = 0, all_wide = 0;
+    double ck_cycles = 0, kept_bands = 0, kept_start = 0;  // the checkpointed reads wide, the others on warps
+    size_t n_ck = 0;
     for (int32_t i : b->order) {
         const ReadDesc& r = b->reads[(size_t)i];
+        if (r.ck) {
+            ++n_ck;
+            ck_cycles += wide_cycles(r);
+        } else {
+            kept_bands += warp_bands(r);
+            kept_start += warp_start(r);
+        }
         rest_bands += warp_bands(r);
         rest_start += warp_start(r);
         all_wide += wide_cycles(r);
@@ -672,6 +685,17 @@ static int64_t heuristic_threshold(const abea_batch* b, int blocks, bool ck_wide
         if (k == 0 || t < best_t * 0.98) {  // a wide read must buy at least 2%
             best_t = t;
             best_n = k;
+        }
+    }
+    // Every checkpointed read wide where they are more than one per block: the blocks take
+    // those in turn, then all their warps the others.
+    if (ck_wide && n_ck > (size_t)max_wide && n_ck < n) {
+        const double t = ck_cycles / std::max(blocks, 1) +
+                         std::max(warp_cycles(warp_bands(*wide_ok[n_ck]), warp_start(*wide_ok[n_ck]), 16),
+                                  warp_cycles(kept_bands, kept_start, 16) / (16.0 * std::max(blocks, 1)));
+        if (t < best_t * 0.98) {
+            best_t = t;
+            best_n = (int)n_ck;
         }
     }
     if (all_ok && !wide_ok.empty()) {
@@ -1981,8 +2005,8 @@ extern "C" int32_t abea_align_cap(abea_aligned_pair_t* out_2, int32_t out_capaci
         (n_events > 0 && !events))
         return fail(ABEA_ERR_INVALID_ARG, "abea_align: invalid argument");
     if (!t_ctx.ctx) {
-        // The batched form puts a lone read on the wide shape (about 380 cycles per
-        // band, against 1,150 for one warp); every call has its own layout, so
+        // The batched form puts a lone read on the wide shape (a read of 20 kb: 183 cycles
+        // per band, on one warp some 500); every call has its own layout, so
         // there is no graph to replay.
         int dev = 0;
         cudaGetDevice(&dev);

@@ -753,13 +753,15 @@ __device__ __forceinline__ T& smem_ref(unsigned at) {
 //   exact (chain_exact): any band.  B, warps 0-3, one k-mer slot per thread, runs the
 //     band-to-band chain with the exact sums and their proofs (abea_cell.cuh), E, warps
 //     4-11, the emissions and their splits up to 16 bands ahead.  Bound by the chain's own
-//     dependent instructions, ~330 cycles per band.
+//     dependent instructions: 390 cycles per band, 440 where a proof fails in most bands.
 //   grid (chain_grid): bands inside the read whose scores are all below -2^11.  A
 //     candidate is then one add of a part that E makes and proves ahead ("candidates on
 //     a grid"), the chain's bound its exchange through shared memory (94 cycles per band on
-//     a bare one), and E does the backpointers.  Measured ~150 cycles per band, E's issue
-//     slots the bound now: align() of a 20 kb read 8.10 -> 5.21 ms, the 1.3 Mbase batch of
-//     f5c's lengths 7.97 -> 5.14 ms, 1,024 reads of 1-10 kb 17.3 -> 12.7 ms.
+//     a bare one), and E does the backpointers.  Some 155 cycles per band, bound by the
+//     chain's own latency (E waits for it half of its time).  With the exact engine
+//     throughout, in an earlier form of 290 cycles per band, align() of a 20 kb read took
+//     8.10 ms, now 5.0, the 1.3 Mbase batch of f5c's lengths 7.97, now 5.2, 1,024 reads of
+//     1-10 kb 17.3, now 12.1.
 //
 // A band's cells lie on one anti-diagonal (event + k-mer = band - 2) and each band moves
 // k0 by at most one, so the placement of band p gives a window [k0, k0 + 128) that holds
@@ -779,8 +781,8 @@ static_assert(kExactRing % kExactGroups == 0, "each ring slot, and its two barri
 
 // Grid engine.  B = warps 0 and 1, two slots per thread, E = four groups of two warps:
 // the warps w with w & 2.  A warp runs on scheduler (w & 3) of the SM, so B has its two to
-// itself; with a fifth group there (warps 4 and 5) a read of 20 kb took 5.2-5.4 ms, now
-// 5.0.  Measured on a bare chain, cycles per band: 87
+// itself; with a fifth group there (warps 4 and 5) a read of 20 kb took 5-8% longer.
+// Measured on a bare chain, cycles per band: 87
 // with four B warps alone and 134 with E's load on every scheduler; 94 with two, whatever
 // runs on the other two schedulers; 141 with one warp of four slots per lane.
 //   Named barriers: 1 = B's per-band barrier, 2 + g = E group g's own, 6 + s = EMPTY[s]: B
@@ -791,8 +793,8 @@ static_assert(kExactRing % kExactGroups == 0, "each ring slot, and its two barri
 // and a flag word next to nothing.  B's polls of a header are bounded by the spin limit:
 // when it runs out the run reports a timeout and the read is given up (`dead`), B going on
 // with a fixed bound until it can leave in step with E, whose turn by then waits for nothing
-// but its own work.  (E polling a word for the released chunks in place of EMPTY costs 8% of
-// a long read: its turns bound the chain.)
+// but its own work.  (E polling a word for the released chunks in place of EMPTY, which would
+// bound its waits too, took 8% of a long read.)
 constexpr int kGridRing = 7;        // chunks in the ring
 constexpr int kGridGroups = 4;
 constexpr int kPerLane = 2;         // slots per thread of B and of E
@@ -1055,7 +1057,9 @@ __device__ __forceinline__ void chain_exact(const WideRead<kCk>& w, int tid, int
                 // A proof failed in some lane: in a read's first bands, three of four, where
                 // an emission far below its score was added to it (Fast2Sum's condition).
                 // TwoSum proves those; with FP64 for them all, the first 800 bands of a read
-                // took 710 cycles each and a read of 1 kb 760 us, now 620.
+                // took 710 cycles each and a read of 1 kb 760 us, now 570.  (No vote per band,
+                // a failed proof redoing its chunk: 325 cycles per band where all hold, but the
+                // tests for it cost the bands with votes 5%.)
                 const bool redo = bad && !here;
                 bool okd2, oku2;
                 const float d2 = exact_from_split<true>(lp, EmSplit{ep.x, ep.z}, mm.x, okd2);
@@ -1149,7 +1153,7 @@ __device__ __forceinline__ void grid_chunk(WideSmem& ws, const float4* km4, cons
 // read whose scalings are off follows the trim cells (k-mer -1, the cheapest way through
 // the events) to the last event, then the first invalid event (n_events, its lower left
 // cell) through the k-mers.
-// Such bands took 437 cycles each on the exact engine, now 160-185 (20,000 bands).
+// Such bands take 440 cycles each on the exact engine, here 160-185 (20,000 bands).
 //   The trim cell is the up candidate of the one before it: their difference is a float
 // (two neighbours' within a factor of two), and so is their sum; its other two candidates
 // come from -inf.  A cell past the last event gets parts of -inf: its score is -inf, its
@@ -1527,7 +1531,7 @@ __device__ __forceinline__ void chain_grid(const WideRead<kCk>& w, int tid, int 
         }
     }
     // Every chunk before j is released; each E group ends up waiting for one of chunks j ..
-    // j + 4, and once chunk j + g is made no group waits for an older chunk of its slot.
+    // j + 3, and once chunk j + g is made no group waits for an older chunk of its slot.
     if (t == 0) {
         ws.exit = j;
         ws.failing = pen > 32 ? 1 : 0;
@@ -1639,8 +1643,8 @@ __device__ __noinline__ bool fill_chain(const CoreArgs& a, const ReadDesc& r, un
 // once per band they cost ~400 cycles per band).  E reads its inputs straight
 // from the pre stage's arrays (L2), one band ahead.  Every wait is bounded by
 // spin_limit polls; a wait that runs out is counted and goes on (the
-// batch then reports a timeout).  Measured: 1,030 cycles per band against 600
-// for the single-block wide shape, so the option is off by default.
+// batch then reports a timeout).  Measured (64 reads of 1-6 kb): 1,080 cycles per band of
+// the longest read against 190 on the single-block wide shape, so the option is off by default.
 constexpr int kClRing = 16;    // bands of emissions in flight (<= 28: the k-mer window above)
 constexpr int kClPublish = 8;  // block 0 publishes its progress every kClPublish bands (< kClRing)
 

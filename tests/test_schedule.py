@@ -132,3 +132,15 @@ def test_checkpointed_reads_may_be_wide():
     assert 1759 < threshold_any([24928] + [1759] * 2432, ck) <= 24928
     assert threshold_any([54000] + [1759] * 2432, ck) == 1
     assert threshold_any([3413] * 2400, [1] * 2400) >= 2**62
+
+
+def test_checkpointed_part_of_a_large_batch_is_wide():
+    """4,096 reads of 1-10 kb, those over 8 kb checkpointed (six per SM): all of these wide, none
+    of the others; without checkpoints none."""
+    rng = np.random.default_rng(1)
+    lens = rng.integers(1000, 10001, 4096)
+    nb = lens - 5 + (lens * 1.71).astype(np.int64) + 2
+    ck = (lens > 8000).astype(np.int32)
+    thr = threshold_any(nb, ck)
+    assert nb[ck == 0].max() < thr <= nb[ck == 1].min()
+    assert threshold_any(nb, 0 * ck) >= 2**62
