@@ -97,6 +97,7 @@ struct abea_batch {
     std::vector<int32_t> dev_order;       // the batched form's order: wide reads, then the rest longest first
     std::vector<int32_t> dev_order_sent;  // the order last copied to the device
     int32_t n_wide = 0;          // leading reads of `order` run on the wide shape
+    int one_fill = 0;            // the warp-shape reads share one copy of the fill
     // sizes
     int64_t seq_bytes = 0, n_events_total = 0, ev_pad_total = 0, km_pad_total = 0,
             band_pad_total = 0, pair_cap = 0, band_cells = 0;
@@ -620,6 +621,14 @@ static int64_t d2h_bytes(const abea_batch* b) {
 // are shared from 8 on).  A checkpointed one twice: its traceback recomputes it on the same
 // warp.
 constexpr double kWarpBase = 950, kWarpMore = 68;
+// Checkpointed and other reads in more than one wave of warps: a block's warps then run the
+// forward pass of either and the recompute at once, whose copies of the fill do not fit the
+// instruction cache together (4.9 warps stalled on it per issued instruction; 0.8 before the
+// grids).  One copy for all, a call, is 10% slower by itself and faster there (4,096 reads of
+// 1-10 kb, over 4 kb checkpointed: 82 -> 68 ms; over 6 kb, scalings off: 97 -> 65; 2,000 of 0.5-6
+// kb, less than a wave: 17.8 against 19.8).
+static bool one_fill(size_t n_warp, int blocks) { return n_warp > (size_t)blocks * 16; }
+constexpr double kOneFill = 1.1;
 static double warp_bands(const ReadDesc& r) { return (r.ck ? 2.0 : 1.0) * (double)r.n_bands; }
 static double warp_start(const ReadDesc& r) {
     const double nb = (double)r.n_bands;
@@ -662,7 +671,7 @@ static int64_t heuristic_threshold(const abea_batch* b, int blocks, bool ck_wide
         all_wide += wide_cycles(r);
         if (ck_wide || !r.ck) wide_ok.push_back(&r);
     }
-    const bool all_ok = wide_ok.size() == n;
+    const bool all_ok = wide_ok.size() == n, mixed = n_ck > 0 && n_ck < n;
     const int max_wide = (int)std::min<size_t>(wide_ok.size(), (size_t)std::max(0, blocks - 1));
     double best_t = 0;
     int best_n = 0;
@@ -681,7 +690,8 @@ static int64_t heuristic_threshold(const abea_batch* b, int blocks, bool ck_wide
         const ReadDesc* longest = j < n ? &b->reads[(size_t)b->order[j]] : nullptr;
         const double t_warp = longest ? warp_cycles(warp_bands(*longest), warp_start(*longest), warps) : 0.0;
         const double t_wide = k > 0 ? wide_cycles(*wide_ok[0]) : 0.0;
-        const double t = std::max(t_wide, std::max(t_warp, warp_cycles(rest_bands, rest_start, warps) / (warps * free_blocks)));
+        const double t = std::max(t_wide, (mixed && one_fill(n - (size_t)k, blocks) ? kOneFill : 1.0) *
+                                              std::max(t_warp, warp_cycles(rest_bands, rest_start, warps) / (warps * free_blocks)));
         if (k == 0 || t < best_t * 0.98) {  // a wide read must buy at least 2%
             best_t = t;
             best_n = k;
@@ -730,6 +740,9 @@ static void choose_shape_reads(abea_batch* b, int sm_count, int64_t threshold, i
     b->dev_order = wide;
     b->dev_order.insert(b->dev_order.end(), rest.begin(), rest.end());
     b->n_wide = (int32_t)wide.size();
+    bool ck = false, kept = false;
+    for (int32_t i : rest) (b->reads[(size_t)i].ck ? ck : kept) = true;
+    b->one_fill = ck && kept && one_fill(rest.size(), blocks) ? 1 : 0;
 }
 
 // Queues pre, core and post for a batch on the context's stream.
@@ -742,7 +755,7 @@ static abea_status_t launch_all(abea_ctx* c, abea_batch* b, int* launches, bool 
                        b->d_last_col, b->d_trace, b->scores_kept ? b->d_scores : nullptr, b->d_band_k0,
                        b->d_slow, b->d_order, b->d_queue, b->n_wide, b->d_ck, b->d_ck_scratch, b->d_spec,
                        b->n_spec,
-                       (long long)c->spin_limit, b->d_km4};
+                       (long long)c->spin_limit, b->one_fill, b->d_km4};
     la.post = PostArgs{b->d_reads, b->n_reads, g, b->d_ev_mean, b->d_km_gm, b->d_km_sd, b->d_km_k1, b->d_km_rsd,
                        b->d_last_col, b->d_trace, b->d_band_k0, b->d_pairs, b->d_n_pairs, b->d_best,
                        b->d_status, b->d_path_len, b->d_path_flags, b->d_best_event,
@@ -820,6 +833,7 @@ static abea_status_t run_batch(abea_ctx* c, abea_batch* b) {
         key.push_back((uint64_t)b->n_reads);
         key.push_back((uint64_t)b->n_wide);
         key.push_back((uint64_t)c->spin_limit);
+        key.push_back((uint64_t)b->one_fill);
         key.push_back((uint64_t)(b->scores_kept ? 1 : 0) | ((uint64_t)b->var_aware << 1) |
                       ((uint64_t)(c->wide_cluster != 0) << 2));
         if (!b->graph || key != b->graph_key) {

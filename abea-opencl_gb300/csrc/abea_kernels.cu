@@ -746,6 +746,12 @@ __device__ __forceinline__ T& smem_ref(unsigned at) {
     return *reinterpret_cast<T*>(__cvta_shared_to_generic(at));
 }
 
+// The one copy of the fill that all warps share when a.one_fill asks for it.
+template <bool kScores>
+__device__ __noinline__ void fill_span(const CoreArgs& a, const ReadDesc& r, unsigned rg_at, int lane, FillSpan sp) {
+    fill_warp<kScores, true>(a, r, smem_ref<Rings>(rg_at), lane, sp);
+}
+
 // ---------------------------------------------------------------- wide shape
 // A read's fill by one block of 16 warps, in chunks of four bands (a tile of
 // backpointers), by two engines over one ring of band scores in shared memory:
@@ -2169,9 +2175,14 @@ __device__ bool walk_segment(const uint8_t* trace, int trace_band0, int bands_en
     return ended;
 }
 
+constexpr int kPostRingDeep = 8;  // trace chunks of a traceback with shared memory to spare (16 KB)
+constexpr int kPostRingMany = 4;  // of each of a block's sixteen warps'
+
 // Recomputes the trace of segment seg (bands [seg*kCkBands, (seg+1)*kCkBands)) of
 // a checkpointed read into `mem` (kCkBands * kSlots bytes).  The whole warp calls it.
-// Inlined at its three calls (as a function: the recompute of 1 kb reads 6-10% slower).
+// Inlined at its three calls (as a function: the recompute of 1 kb reads 6-10% slower) but
+// for ca.one_fill (kMany: where many warps may run it).
+template <bool kMany>
 __device__ __forceinline__ void recompute_segment(const CoreArgs& ca, const ReadDesc& r, Rings& rg, int lane, int seg,
                                                   uint8_t* mem) {
     FillSpan sp;
@@ -2183,7 +2194,10 @@ __device__ __forceinline__ void recompute_segment(const CoreArgs& ca, const Read
     sp.trace_band0 = seg * kCkBands;
     sp.trace_tiles = kCkBands / 4;
     sp.side = false;
-    fill_warp<false, true>(ca, r, rg, lane, sp);
+    if (kMany && ca.one_fill)
+        fill_span<false>(ca, r, smem_u32(&rg), lane, sp);
+    else
+        fill_warp<false, true>(ca, r, rg, lane, sp);
     __syncwarp();
     __threadfence_block();
 }
@@ -2272,7 +2286,7 @@ __device__ void post_read_warp(const CoreArgs& ca, const PostArgs& a, int ri, ui
             // the trace was not kept: recompute it kCkBands bands at a time from
             // the checkpoints, top segment first, and walk each
             for (int seg = (w.k + w.e + 2) / kCkBands; seg >= 0; --seg) {
-                recompute_segment(ca, r, rg, lane, seg, ck_seg);
+                recompute_segment<kRing == kPostRingMany>(ca, r, rg, lane, seg, ck_seg);
                 if (walk_segment<kWalkPairs, kRing>(ck_seg, seg * kCkBands, min((seg + 1) * kCkBands, n_bands),
                                                seg * kCkBands, ring, lane, w, out, cap, a, r))
                     break;
@@ -2367,7 +2381,7 @@ __device__ void post_tail(const CoreArgs& ca, const PostArgs& a, int ri, const R
             // recompute and walk again, summing the emissions in walk order
             Walk w{n_kmers - 1, best_e, 0, 0, 0, n_kmers - 1, 0, 0.0};
             for (int seg = (w.k + w.e + 2) / kCkBands; seg >= 0; --seg) {
-                recompute_segment(ca, r, rg, lane, seg, ck_seg);
+                recompute_segment<kRing == kPostRingMany>(ca, r, rg, lane, seg, ck_seg);
                 if (walk_segment<kWalkSum, kRing>(ck_seg, seg * kCkBands, min((seg + 1) * kCkBands, n_bands),
                                               seg * kCkBands, ring, lane, w, out, cap, a, r))
                     break;
@@ -2433,7 +2447,6 @@ __device__ __forceinline__ void post_write(const PostArgs& a, int ri, int result
 // last cell and the QC follow from the written pairs.
 constexpr int kSpecMargin = 64;
 constexpr int kSpecWarps = kWideThreads / 32;
-constexpr int kPostRingDeep = 8;  // trace chunks of a traceback with shared memory to spare (16 KB)
 
 struct WidePostSmem {  // overlays the wide fill's shared memory once the fill is done
     float best;
@@ -2745,7 +2758,7 @@ __device__ void post_ck_block(const CoreArgs& ca, const PostArgs& a, int ri, uin
     if (best > -INFINITY) {
         for (int top = (w.k + w.e + 2) / kCkBands; top >= 0; top -= kWideThreads / 32) {
             if (top - warp >= 0)
-                recompute_segment(ca, r, rings[warp], lane, top - warp, mem + (int64_t)warp * kSegBytes);
+                recompute_segment<false>(ca, r, rings[warp], lane, top - warp, mem + (int64_t)warp * kSegBytes);
             if (t == 0) ended = 0;
             __syncthreads();  // the segments are in memory
             if (warp == 0) {
@@ -2891,14 +2904,16 @@ __global__ void __launch_bounds__(kWideThreads, 1) abea_batched_kernel(const __g
         pre_read<false>(pa, ri, lane, 32);
         __syncwarp();  // the read's parameters are in memory for the warp
         if (!r.skip) {
-            if (r.ck)
+            if (a.one_fill)
+                fill_span<kScores>(a, r, smem_u32(&sm.warp_rings[warp]), lane, forward_span(a, r));
+            else if (r.ck)
                 fill_warp<kScores, true>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
             else
                 fill_warp<kScores, false>(a, r, sm.warp_rings[warp], lane, forward_span(a, r));
         }
         __syncwarp();
         __threadfence_block();
-        post_read_warp<4>(a, p, ri, sm.post[warp].tr, sm.warp_rings[warp], lane);
+        post_read_warp<kPostRingMany>(a, p, ri, sm.post[warp].tr, sm.warp_rings[warp], lane);
     }
 }
 
@@ -2941,7 +2956,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
         // block reuses the fill's shared memory
         cluster.sync();
         __threadfence_block();
-        if (rank == 0 && warp == 0) post_read_warp<4>(a, p, wide_read, sm.post[0].tr, sm.warp_rings[0], lane);
+        if (rank == 0 && warp == 0) post_read_warp<kPostRingMany>(a, p, wide_read, sm.post[0].tr, sm.warp_rings[0], lane);
     }
     // phase 2: every warp pulls reads longest-first
     const int n_rest = a.n_reads - a.n_wide;
@@ -2960,7 +2975,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
         }
         __syncwarp();
         __threadfence_block();
-        post_read_warp<4>(a, p, ri, sm.post[warp].tr, sm.warp_rings[warp], lane);
+        post_read_warp<kPostRingMany>(a, p, ri, sm.post[warp].tr, sm.warp_rings[warp], lane);
     }
     cluster.sync();  // neither block leaves while the other may still write its shared memory
 }

@@ -62,6 +62,7 @@ struct CoreArgs {
     int32_t* spec;                 // traceback cell maps: kSpecRound * kSpecBands int32 per slot
     int32_t n_spec;                // slots (queue[2] hands them out)
     long long spin_limit;          // polls before a device-side wait gives up (kCountTimeouts counts those)
+    int one_fill;                  // every warp-shape fill through one copy of the code (fill_span)
     const float4* km4;             // {km_gm, km_sd, km_rsd, km_k1} of each k-mer position (wide shape)
 };
 
