@@ -127,3 +127,25 @@ def test_more_checkpointed_reads_than_blocks(oracle_mod):
     op, oc, obest = oracle_mod.align_batch(batch)
     same_alignments(batch, gp, gc, op, oc)
     assert np.array_equal(dev.best_scores().view(np.uint32), obest.view(np.uint32))
+
+
+@pytest.mark.parametrize("scores", [False, True])
+@pytest.mark.parametrize("n", [2432, 2433, 3000])
+def test_checkpointed_and_other_reads_in_more_than_a_wave(oracle_mod, n, scores):
+    """Up to 16 warp-shape reads per SM of a GB300's 152, and more (their fills then share one
+    copy of the code), every third read checkpointed, over one and over two segments."""
+    from abea_gb300 import synth
+    lengths = np.tile([40, 100, 230], 1000)[:n]
+    batch = synth.make_batch("small", seed=7, lengths=lengths)
+    budget = (int(np.sort(batch.n_bands())[-(n // 3)]) + 3) // 4 * 4 * BYTES_PER_BAND - 1
+    ck = (batch.n_bands() + 3) // 4 * 4 * BYTES_PER_BAND > budget
+    assert 0 < ck.sum() < n and (batch.n_bands()[ck] > 512).any()
+    ctx = abea.Context(0, abea.MODE_BATCHED, store_scores=scores)
+    ctx.set_option(abea.OPT_TRACE_BUDGET, budget)
+    ctx.set_option(abea.OPT_LONG_READ_BANDS, 1 << 40)
+    dev = ctx.upload(batch)
+    dev.run()
+    pairs, counts = dev.results()
+    op, oc, obest = oracle_mod.align_batch(batch, threads=8)
+    same_alignments(batch, pairs, counts, op, oc)
+    assert np.array_equal(dev.best_scores().view(np.uint32), obest.view(np.uint32))
